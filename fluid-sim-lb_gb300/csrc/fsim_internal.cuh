@@ -243,6 +243,9 @@ struct fsim_sim {
   uint2* d_leaf_range = nullptr; // pleaf
   int n_pleaf = 0, n_gleaf = 0;
   bool have_topology = false;
+  // d_cell_range indexes the current particles (a rollout's restored
+  // topologies and checkpoints leave them apart until the next sort)
+  bool ranges_match = false;
 
   // grid fields (per slot)
   float* vel = nullptr;     // slot*1536
@@ -390,6 +393,7 @@ int launch_g2p(fsim_sim* s);
 // divergence (the solution is then read from x64: FP64 / MIXED precision)
 int pcg_solve(fsim_sim* s, const fsim_pcg_params* prm, fsim_pcg_stats* st,
               const double* b64 = nullptr);
+int ensure_dense(fsim_sim* s, size_t bytes);  // dense_tmp of at least bytes
 int download_dense(fsim_sim* s, int field, float* out, uint8_t* active);
 int download_marker(fsim_sim* s, int32_t* out, uint8_t* active);
 int seed_fluid(fsim_sim* s, const fsim_seed_pass* passes, int npasses, uint64_t seed);

@@ -747,6 +747,7 @@ int load_state(fsim_rollout* r, const Checkpoint& c) {
   RB_CK(d2d(s->keys[0], c.keys.p, size_t(n), s->stream));
   s->n_total = s->n_live = n;
   s->have_topology = true;
+  s->ranges_match = false;
   return FSIM_OK;
 }
 
@@ -757,6 +758,7 @@ int restore_topo(fsim_rollout* r, const TopoRec& t) {
   if (rc) return rc;
   s->n_pleaf = t.n_pleaf;
   s->n_gleaf = t.n_gleaf;
+  s->ranges_match = false;
   RB_CK(d2d(s->d_slot, t.slot.p, size_t(s->lm.dense), s->stream));
   RB_CK(d2d(s->d_leaf_id, t.leaf_id.p, size_t(t.n_gleaf), s->stream));
   RB_CK(d2d(s->d_nbr, t.nbr.p, size_t(t.n_gleaf) * 27, s->stream));

@@ -932,7 +932,7 @@ int launch_cfl(fsim_sim* s) {
   return FSIM_OK;
 }
 
-static int ensure_dense(fsim_sim* s, size_t bytes) {
+int ensure_dense(fsim_sim* s, size_t bytes) {
   if (s->dense_tmp.bytes >= bytes) return FSIM_OK;
   if (s->dense_tmp.p) cudaFree(s->dense_tmp.p);
   s->dense_tmp.p = nullptr;

@@ -13,7 +13,7 @@
 // caller downloads (same layout as fsim_download_field).
 #include <algorithm>
 #include <cmath>
-#include <vector>
+#include <cstring>
 
 #include "fsim_internal.cuh"
 
@@ -38,7 +38,113 @@ struct LsArgs {
   unsigned* phi;   // ordered bits, dense
 };
 
-// one thread per particle: every voxel point within R + w of it
+// Level set of the particle leaves' neighbourhood, one CTA per grid leaf, a
+// thread per voxel point.  The field is min over particles of
+// sqrt(d2) - radius, and rounding is monotone, so it is taken from the
+// smallest d2: each voxel looks at the cells around it ring by ring (ring r:
+// cells whose box is r away on some axis) and stops when the next ring cannot
+// hold a nearer particle.  d2 of a particle is never below its cell's box
+// distance, in rounded arithmetic too (boxes are integers), so the pruning
+// changes no bit.  Inside the fluid the eight cells at the voxel decide;
+// outside it the search runs over occupancy bits, a word per z row.  A
+// splat from the particles instead (k_ls_splat) writes the 905 voxels in
+// reach of every particle with an atomic each, 2,600 atomics per fluid
+// voxel, nearly all of them lost to a nearer particle: 15.9 ms at 128^3
+// (3.65 M particles) against 0.42 ms here, bound by the issue of the distance
+// and bit-search instructions.
+struct LsGatherArgs {
+  const float* part;
+  int64_t cap;
+  const uint32_t* keys;
+  const int32_t* leaf_id;
+  const int32_t* nbr;
+  const uint2* cell_range;
+  const uint32_t* occ;  // [particle leaf][16]: a bit per cell that holds particles
+  LeafMap lm;
+  int n_pleaf, check_dead, rings;
+  float radius, half_width, lim2;  // lim2: no d2 above it reaches the band
+  float* phi;
+};
+
+__global__ void __launch_bounds__(512) k_ls_occupancy(const uint2* __restrict__ cell_range,
+                                                      uint32_t* __restrict__ occ) {
+  const uint2 rg = cell_range[int64_t(blockIdx.x) * 512 + threadIdx.x];
+  const unsigned b = __ballot_sync(0xffffffffu, rg.y > rg.x);
+  if ((threadIdx.x & 31) == 0) occ[int64_t(blockIdx.x) * 16 + (threadIdx.x >> 5)] = b;
+}
+
+constexpr int kLsRings = 8;  // cells of the 27 leaves around a voxel: rings 0 .. 7
+
+__global__ void __launch_bounds__(512) k_ls_gather(const __grid_constant__ LsGatherArgs a) {
+  __shared__ int nb[27];
+  __shared__ uint32_t rows[24 * 24];  // bit z + 8 of row (x + 8, y + 8): cell (x, y, z)
+  const int s = blockIdx.x, tid = threadIdx.x;
+  if (tid < 27) {
+    const int ns = a.nbr[int64_t(s) * 27 + tid];
+    nb[tid] = ns < a.n_pleaf ? ns : -1;
+  }
+  int lx, ly, lz;
+  leaf_coords(a.lm, uint32_t(a.leaf_id[s]), lx, ly, lz);
+  __syncthreads();
+  for (int r = tid; r < 24 * 24; r += 512) {
+    const int x = r / 24, y = r % 24;
+    uint32_t m = 0;
+#pragma unroll
+    for (int dz = 0; dz < 3; ++dz) {
+      const int ns = nb[(x >> 3) * 9 + (y >> 3) * 3 + dz];
+      const int bit = ((x & 7) << 6) | ((y & 7) << 3);
+      if (ns >= 0)
+        m |= ((a.occ[int64_t(ns) * 16 + (bit >> 5)] >> (bit & 31)) & 255u) << (8 * dz);
+    }
+    rows[r] = m;
+  }
+  __syncthreads();
+  const int vx = tid >> 6, vy = (tid >> 3) & 7, vz = tid & 7;
+  const int g[3] = {lx * 8 + vx, ly * 8 + vy, lz * 8 + vz};
+  const int* n = a.lm.n;
+  if (g[0] > n[0] || g[1] > n[1] || g[2] > n[2] || g[0] < -1 || g[1] < -1 || g[2] < -1) return;
+  const float fx = float(g[0]), fy = float(g[1]), fz = float(g[2]);
+  float best = a.lim2;
+  for (int r = 0; r < a.rings; ++r) {
+    if (float(r * r) >= best) break;
+    for (int X = vx - 1 - r; X <= vx + r; ++X) {
+      const int ax = X >= vx ? X - vx : vx - 1 - X;
+      if (float(ax * ax) >= best) continue;
+      for (int Y = vy - 1 - r; Y <= vy + r; ++Y) {
+        const int ay = Y >= vy ? Y - vy : vy - 1 - Y;
+        const int axy2 = ax * ax + ay * ay;
+        uint32_t m = rows[(X + 8) * 24 + Y + 8];
+        // the ring's cells of this row: all of it, or its two ends
+        const uint32_t lo = 1u << (vz + 7 - r), hi = 1u << (vz + 8 + r);
+        m &= (ax == r || ay == r) ? (hi | (hi - lo)) : (lo | hi);
+        while (m != 0u && float(axy2) < best) {
+          const int Z = __ffs(int(m)) - 9;
+          m &= m - 1u;
+          const int az = Z >= vz ? Z - vz : vz - 1 - Z;
+          if (float(axy2 + az * az) >= best) continue;
+          const int ns = nb[((X + 8) >> 3) * 9 + ((Y + 8) >> 3) * 3 + ((Z + 8) >> 3)];
+          const uint2 rg =
+              a.cell_range[int64_t(ns) * 512 + (((X & 7) << 6) | ((Y & 7) << 3) | (Z & 7))];
+          for (uint32_t q = rg.x; q < rg.y; ++q) {
+            if (a.check_dead && a.keys[q] == kDeadKey) continue;
+            const float dx = __fsub_rn(fx, a.part[q]), dy = __fsub_rn(fy, a.part[a.cap + q]),
+                        dz = __fsub_rn(fz, a.part[2 * a.cap + q]);
+            best = fminf(best, __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)),
+                                         __fmul_rn(dz, dz)));
+          }
+        }
+      }
+    }
+  }
+  // past lim2 the value lies outside the band: half_width, as below
+  const float v = best < a.lim2 ? __fsub_rn(__fsqrt_rn(best), a.radius) : a.half_width;
+  const int64_t o = (int64_t(g[0] + 1) * (n[1] + 2) + (g[1] + 1)) * (n[2] + 2) + (g[2] + 1);
+  a.phi[o] = fminf(fmaxf(v, -a.half_width), a.half_width);
+}
+
+// The splat, for bands wider than the leaf neighbourhood reaches and for
+// particles that are not binned (appended by sources since the last sort):
+// one thread per particle, every voxel point within R + w of it.
 __global__ void k_ls_splat(const __grid_constant__ LsArgs a) {
   const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= a.n || a.keys[i] == kDeadKey) return;
@@ -100,36 +206,86 @@ __global__ void k_ls_mean(const float* __restrict__ in, float* __restrict__ out,
   out[o] = fminf(fmaxf(__fdiv_rn(s, 27.0f), -w), w);
 }
 
+// band mask: |phi| < w
+__global__ void k_ls_active(const float* __restrict__ phi, uint8_t* __restrict__ act, int64_t n,
+                            float w) {
+  const int64_t o = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (o < n) act[o] = fabsf(phi[o]) < w;
+}
+
 __global__ void k_fill_u32(unsigned* __restrict__ p, int64_t n, unsigned v) {
   const int64_t o = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (o < n) p[o] = v;
 }
 
-int level_set(fsim_t* s, float radius, float half_width, int mean_iterations, unsigned* bits,
-              float* f[2], int64_t tot, float* phi) {
+// Rings of cells that can hold a particle within reach of a voxel, or 0 when
+// they do not fit in the leaf neighbourhood.
+int gather_rings(const fsim_t* s, float radius, float half_width) {
+  if (s->composite_sort || !s->ranges_match) return 0;
+  const float reach = std::ceil(radius + half_width);
+  return reach <= float(kLsRings) ? int(reach) : 0;
+}
+
+int level_set(fsim_t* s, float radius, float half_width, int mean_iterations, float* f[2],
+              uint8_t* act, int64_t tot, float* phi, uint8_t* active) {
   const int n0 = s->lm.n[0] + 2, n1 = s->lm.n[1] + 2, n2 = s->lm.n[2] + 2;
   const unsigned g = unsigned((tot + 255) / 256);
-  // every voxel starts outside the band: the ordered bits of +inf
-  FSIM_LAUNCH(s, "levelset_fill", k_fill_u32, g, 256, 0, bits, tot, 0xFF800000u);
-  LsArgs a;
-  a.part = s->part[s->cur];
-  a.cap = s->cap_p;
-  a.n = s->n_live;
-  a.keys = s->keys[0];
-  a.n0 = n0;
-  a.n1 = n1;
-  a.n2 = n2;
-  a.radius = radius;
-  a.half_width = half_width;
-  a.phi = bits;
-  FSIM_LAUNCH(s, "levelset_splat", k_ls_splat, unsigned(std::max<int64_t>((a.n + 255) / 256, 1)),
-              256, 0, a);
-  FSIM_LAUNCH(s, "levelset_finish", k_ls_finish, g, 256, 0, bits, f[0], tot, half_width);
+  const int rings = gather_rings(s, radius, half_width);
+  if (rings > 0 && s->n_pleaf > 0) {
+    // voxels outside the grid leaves lie outside the band
+    uint32_t w;
+    std::memcpy(&w, &half_width, 4);
+    FSIM_LAUNCH(s, "levelset_fill", k_fill_u32, g, 256, 0, reinterpret_cast<unsigned*>(f[0]), tot,
+                w);
+    uint32_t* occ = reinterpret_cast<uint32_t*>(f[1]);  // read before the mean writes f[1]
+    FSIM_LAUNCH(s, "levelset_occupancy", k_ls_occupancy, unsigned(s->n_pleaf), 512, 0,
+                s->d_cell_range, occ);
+    LsGatherArgs a;
+    a.part = s->part[s->cur];
+    a.cap = s->cap_p;
+    a.keys = s->keys[0];
+    a.leaf_id = s->d_leaf_id;
+    a.nbr = s->d_nbr;
+    a.cell_range = s->d_cell_range;
+    a.occ = occ;
+    a.lm = s->lm;
+    a.n_pleaf = s->n_pleaf;
+    a.check_dead = s->deleted_outside ? 1 : 0;
+    a.rings = rings;
+    a.radius = radius;
+    a.half_width = half_width;
+    const float reach = radius + half_width;
+    a.lim2 = reach * reach * 1.00001f;
+    a.phi = f[0];
+    FSIM_LAUNCH(s, "levelset_gather", k_ls_gather, unsigned(s->n_gleaf), 512, 0, a);
+  } else {
+    unsigned* bits = reinterpret_cast<unsigned*>(f[1]);
+    // every voxel starts outside the band: the ordered bits of +inf
+    FSIM_LAUNCH(s, "levelset_fill", k_fill_u32, g, 256, 0, bits, tot, 0xFF800000u);
+    LsArgs a;
+    a.part = s->part[s->cur];
+    a.cap = s->cap_p;
+    a.n = s->n_live;
+    a.keys = s->keys[0];
+    a.n0 = n0;
+    a.n1 = n1;
+    a.n2 = n2;
+    a.radius = radius;
+    a.half_width = half_width;
+    a.phi = bits;
+    FSIM_LAUNCH(s, "levelset_splat", k_ls_splat,
+                unsigned(std::max<int64_t>((a.n + 255) / 256, 1)), 256, 0, a);
+    FSIM_LAUNCH(s, "levelset_finish", k_ls_finish, g, 256, 0, bits, f[0], tot, half_width);
+  }
   for (int it = 0; it < mean_iterations; ++it) {
     FSIM_LAUNCH(s, "levelset_mean", k_ls_mean, g, 256, 0, f[0], f[1], n0, n1, n2, half_width);
     std::swap(f[0], f[1]);
   }
   FSIM_CK(s, cudaMemcpyAsync(phi, f[0], size_t(tot) * 4, cudaMemcpyDeviceToHost, s->stream));
+  if (active) {
+    FSIM_LAUNCH(s, "levelset_active", k_ls_active, g, 256, 0, f[0], act, tot, half_width);
+    FSIM_CK(s, cudaMemcpyAsync(active, act, size_t(tot), cudaMemcpyDeviceToHost, s->stream));
+  }
   FSIM_CK(s, cudaStreamSynchronize(s->stream));
   return FSIM_OK;
 }
@@ -146,19 +302,14 @@ extern "C" int fsim_particles_to_level_set(fsim_t* s, float radius, float half_w
   cudaSetDevice(s->dev);
   if (!s->have_topology) return fail(s, FSIM_ERR_STATE, "no particles uploaded or seeded");
   const int64_t tot = int64_t(s->lm.n[0] + 2) * (s->lm.n[1] + 2) * (s->lm.n[2] + 2);
-  unsigned* bits = nullptr;
-  float* f[2] = {nullptr, nullptr};
-  cudaError_t e = cudaMalloc(&bits, size_t(tot) * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&f[0], size_t(tot) * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&f[1], size_t(tot) * 4);
-  int rc = e == cudaSuccess ? level_set(s, radius, half_width, mean_iterations, bits, f, tot, phi)
-                            : cuda_fail(s, e, "level set buffers");
-  cudaStreamSynchronize(s->stream);
-  if (bits) cudaFree(bits);
-  if (f[0]) cudaFree(f[0]);
-  if (f[1]) cudaFree(f[1]);
+  // two fields and the band mask, in the handle's staging for dense downloads;
+  // the occupancy words (64 B per particle leaf) may need more than a field
+  const size_t field =
+      (std::max(size_t(tot) * 4, size_t(s->n_pleaf) * 64) + 255) / 256 * 256;
+  int rc = ensure_dense(s, 2 * field + size_t(tot));
   if (rc) return rc;
-  if (active)
-    for (int64_t o = 0; o < tot; ++o) active[o] = std::fabs(phi[o]) < half_width ? 1 : 0;
-  return FSIM_OK;
+  char* base = static_cast<char*>(s->dense_tmp.p);
+  float* f[2] = {reinterpret_cast<float*>(base), reinterpret_cast<float*>(base + field)};
+  return level_set(s, radius, half_width, mean_iterations, f,
+                   reinterpret_cast<uint8_t*>(base + 2 * field), tot, phi, active);
 }

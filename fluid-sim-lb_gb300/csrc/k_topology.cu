@@ -663,6 +663,7 @@ int rebuild_after_sort(fsim_sim* s, bool gather) {
   FSIM_LAUNCH(s, "cell_ranges", k_ranges, nblk(s->n_live, 256 * kKeysPerThread), 256, 0, s->keys[0], s->d_cnt,
               s->d_slot, s->d_cell_range, s->d_leaf_range);
   s->have_topology = true;
+  s->ranges_match = true;
   s->deleted_outside = false;
   return FSIM_OK;
 }
