@@ -323,6 +323,9 @@ struct fsim_sim {
   // and the flags on chip): -1 by system size, 0 never, 1 wherever it fits
   // (FSIM_PCG_RES)
   int pcg_res = -1;
+  // small FP32 and MIXED solves by one thread-block cluster (where pcg_res is
+  // by size); false once a cluster launch has been refused
+  bool pcg_cluster = true;
 
   // water sources and the time they see
   std::vector<fsim_source> sources;

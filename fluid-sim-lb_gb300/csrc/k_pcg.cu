@@ -2748,6 +2748,19 @@ struct LoopTimer {
   }
 };
 
+#include "pcg_cluster.cuh"
+
+// The cluster loop takes FP32 and MIXED solves of at most kClLeaves particle
+// leaves (what its shared memory and registers hold), unless another loop is
+// asked for by its switch: it is the fastest loop at every such size
+// (pcg_cluster.cuh; at 232 leaves 5.1 us per iteration against the resident
+// loop's 6.4 and the pair's 6.7).  FP64 is bound by the FP64 pipe, which 16
+// SMs hold too little of.
+bool use_cluster(const fsim_sim* s, int precision) {
+  return precision != FSIM_PREC_FP64 && s->pcg_res < 0 && s->pcg_cluster && s->n_pleaf > 0 &&
+         s->n_pleaf <= kClLeaves && !(precision == FSIM_PREC_FP32 && s->pcg_cg1 == 1);
+}
+
 // One inner solve: setup, then the iterations.  The iterations run as a CUDA
 // graph whose conditional WHILE node repeats {spmv, update}; the kernel head
 // that sets the stop flag clears the condition, so the whole loop runs
@@ -2761,6 +2774,13 @@ int run_inner(fsim_sim* s, PcgArgs& a, int grid, const char* nm_setup, const cha
               const char* nm_upd, bool setup = true, int par0 = 0) {
   a.cond = 0;
   if (setup) FSIM_LAUNCH(s, nm_setup, (k_pcg_setup<T, DM>), grid, kThreads, 0, a);
+  if constexpr (DM < 2) {
+    if (use_cluster(s, DM == 0 ? FSIM_PREC_FP32 : FSIM_PREC_MIXED)) {
+      const int rc = run_cluster<DM>(s, a);
+      if (rc != FSIM_ERR_CUDA) return rc;
+      s->pcg_cluster = false;  // refused: the pair, for the rest of this handle's life
+    }
+  }
   const int wpb = kHotThreads / 32;
   int occ_a = 1, occ_b = 1;
   const bool zd = use_zdirect<T>(s, a.n_pleaf);
@@ -3032,7 +3052,9 @@ int pcg_solve(fsim_sim* s, const fsim_pcg_params* prm, fsim_pcg_stats* st, const
     *s->h_sc = h;
     FSIM_CK(s, cudaMemcpyAsync(s->d_sc, s->h_sc, sizeof(PcgScalars), cudaMemcpyHostToDevice,
                                s->stream));
-    if (use_resident(s, prm->precision)) {
+    if (use_cluster(s, prm->precision)) {
+      rc = run_inner<float, 0>(s, a, grid, "pcg_setup", "pcg_spmv", "pcg_update");
+    } else if (use_resident(s, prm->precision)) {
       rc = run_resident(s, a, grid);
       if (rc == FSIM_ERR_CUDA) {  // cooperative launch refused: the pair
         cudaGetLastError();
