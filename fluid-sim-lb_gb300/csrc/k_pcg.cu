@@ -1892,586 +1892,6 @@ __global__ void __launch_bounds__(kHotThreads, 4) k_pcg_cg1_s(const __grid_const
   }
 }
 
-// ---- on-chip resident loop: one persistent CTA per SM ---------------------------
-// fp32 solves whose particle leaves fit on chip (by default 2 to kResLeaves
-// particle leaves per SM; FSIM_PCG_RES=1 / 0 forces it on / off): one
-// cooperative launch runs every iteration.  CTA c owns the contiguous slots
-// [c * per, c * per + nl), per = ceil(n_pleaf / G) <= kResLeaves, and keeps
-// every vector of the iteration on chip: p and the flags in shared memory,
-// r and A p in tensor memory, x in tensor and shared memory (each warp owns
-// up to kResHL half leaves, a lane one z-column of each).  Per iteration,
-// as the reference's ComputeLocal1-3 (common/solver.cc:297-366):
-//   S: p = z + beta p on the own columns (into shared memory, and the
-//      columns other CTAs read into a global mirror), then A p (kept) and
-//      the p.Ap partials;
-//   grid barrier: every CTA sums the G partials in CTA order -> alpha;
-//   U: x += alpha p, r -= alpha A p, z = M r (of the columns other CTAs read
-//      also into a global mirror), the r.r and r.z partials;
-//   grid barrier -> r.r, r.z, beta and the loop test.
-// (One more grid barrier before the first iteration publishes the first z.)
-// Stencil neighbours in the CTA's own leaves come from shared memory; those
-// in other CTAs' leaves are formed as z + beta p from the mirrors of z and
-// the previous p, read through L2 (the owner's operations, so the owner's
-// bits; p alternates between two mirror buffers by iteration parity), by all
-// 32 lanes of the warp together and handed out by warp shuffles.  A p is summed in the
-// reference's column order.  The dot products are summed per thread, per
-// CTA and over CTAs in fixed orders: the solve is deterministic (its
-// per-thread order differs from the pair's, so the bits do too).  Thread 0
-// alone runs the scalar steps (alpha, beta, the loop test) in fp64.  x and r
-// are written back whole at the end.  Barrier waits are bounded (kResPolls);
-// a CTA that gives up sets bar_err and every CTA leaves the loop
-// (FSIM_ERR_TIMEOUT), freeing its tensor memory.
-constexpr int kResWarps = 28;
-constexpr int kResThreads = kResWarps * 32;
-constexpr int kResHL = 4;                             // half leaves per warp
-constexpr int kResLeaves = kResWarps * kResHL / 2;    // leaves per CTA
-// dynamic shared memory: p and the flags of the CTA's leaves, and x of every
-// warp's half leaves 1 .. kResHL - 1 (half leaf 0's x is in tensor memory)
-constexpr size_t kResSmemX = size_t(kResHL - 1) * kResWarps * 256 * sizeof(float);
-constexpr size_t kResSmem = size_t(kResLeaves) * 512 * (sizeof(float) + 1) + kResSmemX;
-constexpr unsigned kResPolls = 1u << 22;  // about 2-4 s of L2 round trips
-
-__device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-// Grid barrier of round `round` with the CTA's NV partials: publish, arrive
-// (a GPU-scope release add on one counter, after the CTA barrier that orders
-// the CTA's mirror stores first), wait with acquire loads until all G CTAs
-// of the round have arrived, then sum the G partials in CTA order (every CTA
-// the same totals), and thread 0 runs fin(totals) before the closing CTA
-// barrier.  Rows row0.. of the float partials; each phase type has
-// its own rows, which a CTA can only rewrite after every CTA has passed the
-// next barrier, and so has read them.  Waits are bounded: a CTA that gives
-// up sets bar_err, which the others also poll.  With PcgArgs::res_withhold
-// (tests) CTA 0 does not arrive at the first barrier and the limit is 256
-// polls, so every CTA's wait gives up.  (Publishing each partial
-// beside the round number in one 64-bit word, polled by every CTA, measured
-// slower: 33.2 against 30.1 us per iteration at 256^3, and again with
-// relaxed words and no fence on the p.Ap barrier, 21.8 against 16.8: the
-// polling of 152 slots by every CTA costs more than the counter's second
-// round trip.)
-template <int NV, typename F>
-__device__ __forceinline__ bool res_sync(const PcgArgs& a, float (&v)[NV], int row0,
-                                         unsigned round, int* s_ok, F&& fin) {
-  block_sum_p<float, NV, kResThreads>(v);  // its CTA barrier orders the CTA's stores first
-  if (threadIdx.x < 32) {
-    // warp 0: lane 0 publishes, arrives and waits; the warp then sums
-    const int lane = threadIdx.x, G = int(gridDim.x);
-    int ok = 1;
-    if (lane == 0) {
-#pragma unroll
-      for (int k = 0; k < NV; ++k) a.partf[(row0 + k) * a.maxb + blockIdx.x] = v[k];
-      if (!(a.res_withhold && blockIdx.x == 0 && round == 1))
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;\n" ::"l"(&a.sc->bar_count) : "memory");
-      const unsigned target = round * gridDim.x;
-      const unsigned limit = a.res_withhold ? 256u : kResPolls;
-      unsigned polls = 0;
-      while (ld_acquire_gpu(&a.sc->bar_count) < target) {
-        if ((++polls & 255u) == 0u &&
-            (polls > limit || ld_acquire_gpu(&a.sc->bar_err) != 0u)) {
-          ok = 0;
-          break;
-        }
-      }
-      if (!ok) atomicExch(&a.sc->bar_err, 1u);
-      *s_ok = ok;
-    }
-    ok = __shfl_sync(0xffffffffu, ok, 0);
-    __syncwarp();  // orders lane 0's acquire before the other lanes' loads
-    if (ok) {
-      // lane adds partials lane, lane + 32, ... in that order; each batch's
-      // loads are all issued before its adds (a zero pad adds exactly nothing)
-      float x[NV];
-#pragma unroll
-      for (int k = 0; k < NV; ++k) x[k] = 0.f;
-      for (int i0 = lane; i0 < G; i0 += 32 * 8) {
-        float t[NV][8];
-#pragma unroll
-        for (int k = 0; k < NV; ++k)
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const int i = i0 + 32 * u;
-            t[k][u] = i < G ? __ldcg(a.partf + (row0 + k) * a.maxb + i) : 0.f;
-          }
-#pragma unroll
-        for (int k = 0; k < NV; ++k)
-#pragma unroll
-          for (int u = 0; u < 8; ++u) x[k] = __fadd_rn(x[k], t[k][u]);
-      }
-      double tot[NV];
-#pragma unroll
-      for (int k = 0; k < NV; ++k) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x[k] = __fadd_rn(x[k], __shfl_down_sync(0xffffffffu, x[k], o));
-        tot[k] = double(x[k]);
-      }
-      if (lane == 0) fin(tot);
-    }
-  }
-  __syncthreads();
-  return *s_ok != 0;
-}
-
-// Shared p of the CTA's leaves in 16-byte chunk planes: float4 element
-// ((leaf * 2 + chunk) * 8 + x) * 8 + y holds the cells z = 4 chunk ..
-// 4 chunk + 3 of column (x, y), so the lanes of a quarter warp (consecutive
-// y) touch consecutive 16-byte words.  ps_col4 is the float4 index of chunk 0
-// of a column; chunk 1 is 64 further, and the in-leaf neighbour columns are
-// -8 / +8 (x) and -1 / +1 (y) away, constant offsets from the own column.
-__device__ __forceinline__ int ps_col4(int leaf, int x, int y) { return (leaf * 16 + x) * 8 + y; }
-__device__ __forceinline__ void ps_ld4(const float* ps, int i, Col<float>& c) {
-  const float4* q = reinterpret_cast<const float4*>(ps);
-  const float4 u = q[i], w = q[i + 64];
-  c.v[0] = u.x; c.v[1] = u.y; c.v[2] = u.z; c.v[3] = u.w;
-  c.v[4] = w.x; c.v[5] = w.y; c.v[6] = w.z; c.v[7] = w.w;
-}
-__device__ __forceinline__ void ps_st4(float* ps, int i, const Col<float>& c) {
-  float4* q = reinterpret_cast<float4*>(ps);
-  q[i] = make_float4(c.v[0], c.v[1], c.v[2], c.v[3]);
-  q[i + 64] = make_float4(c.v[4], c.v[5], c.v[6], c.v[7]);
-}
-
-// The resident loop's scalar state, kept by thread 0.
-struct ResScalars {
-  double rr, rz, rz_old, alpha, beta, pAp;
-  int status, max_iter;
-  PcgRule rule;
-};
-
-// Where a neighbour of the CTA's cells lives.
-struct ResFrame {
-  const float* ps;       // shared p of the CTA's leaves
-  const uint8_t* fsm;    // shared flags
-  int L0, nl, n_pleaf;
-};
-__device__ __forceinline__ bool res_local(const ResFrame& fr, int slot) {
-  return slot >= fr.L0 && slot < fr.L0 + fr.nl;
-}
-
-// p (current iteration) of cell (x, y, z) of leaf `slot`: from shared memory
-// for the CTA's leaves, else formed from the mirrors of z and the previous p.
-__device__ __forceinline__ float res_pcell(const ResFrame& fr, const PcgArgs& a,
-                                           const float* pm_old, const DiagInv<float>* tab,
-                                           float beta, int slot, int x, int y, int z) {
-  if (res_local(fr, slot)) return fr.ps[(ps_col4(slot - fr.L0, x, y) + (z >> 2) * 64) * 4 + (z & 3)];
-  const unsigned o = slot_or_null(slot, fr.n_pleaf) * 512u + unsigned(x * 64 + y * 8 + z);
-  // the mirror holds z = M r (the owner's product): pnew_of's operations
-  return tadd(__ldcg(static_cast<const float*>(a.r) + o), tmul(beta, __ldcg(pm_old + o)));
-}
-
-// The half leaf's faces in other CTAs' leaves (its outward x face and both
-// y faces: 16 columns of 8 cells), formed by all 32 lanes in step: lane L
-// forms cells 4 (L & 1) .. + 3 of face column t = L >> 1 (t < 8: the x face
-// at y = t; 8 .. 11: the -y face at x = xb + t - 8; 12 .. 15: the +y face)
-// from the mirrors of z and the previous p, with the owner's operations.
-// Faces in the CTA's own leaves are left to shared memory (v stays 0).
-__device__ __forceinline__ void res_faces(const ResFrame& fr, const PcgArgs& a, const float* pm_old,
-                                          const DiagInv<float>* tab, float beta, int xb,
-                                          const int fs[6], int lane, float (&v)[4]) {
-  const int t = lane >> 1;
-  int slot, off;
-  if (t < 8) {
-    slot = xb == 0 ? fs[0] : fs[1];
-    off = (xb == 0 ? 7 : 0) * 64 + t * 8;
-  } else if (t < 12) {
-    slot = fs[2];
-    off = (xb + t - 8) * 64 + 56;
-  } else {
-    slot = fs[3];
-    off = (xb + t - 12) * 64;
-  }
-  off += 4 * (lane & 1);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) v[j] = 0.f;
-  if (!res_local(fr, slot)) {
-    const unsigned o = slot_or_null(slot, fr.n_pleaf) * 512u + unsigned(off);
-    // the mirror holds z = M r (the owner's product): pnew_of's operations
-    const float4 zm = __ldcg(reinterpret_cast<const float4*>(static_cast<const float*>(a.r) + o));
-    const float4 po = __ldcg(reinterpret_cast<const float4*>(pm_old + o));
-    v[0] = tadd(zm.x, tmul(beta, po.x));
-    v[1] = tadd(zm.y, tmul(beta, po.y));
-    v[2] = tadd(zm.z, tmul(beta, po.z));
-    v[3] = tadd(zm.w, tmul(beta, po.w));
-  }
-}
-// column c of the faces formed by res_faces (lanes 2 c and 2 c + 1)
-__device__ __forceinline__ void res_face_col(const float (&v)[4], int c, Col<float>& out) {
-#pragma unroll
-  for (int z = 0; z < 8; ++z) out.v[z] = __shfl_sync(0xffffffffu, v[z & 3], 2 * c + (z >> 2));
-}
-
-// A p on the lane's column (xb + lx, y) of leaf s (own values P), in the
-// reference's column order; 0 off-fluid.  Called by all 32 lanes of the
-// warp together (res_faces, res_face_col).
-__device__ __forceinline__ void res_ap(const ResFrame& fr, const PcgArgs& a, const float* pm_old,
-                                       const DiagInv<float>* tab, float beta, int s, int xb, int lx,
-                                       int y, int lane, const int fs[6], const Col<float>& P,
-                                       uint2 f, Col<float>& ap) {
-  const int x = xb + lx;
-  const int own = ps_col4(s - fr.L0, x, y);
-  float fv[4];
-  res_faces(fr, a, pm_old, tab, beta, xb, fs, lane, fv);
-  // one neighbour column at a time, in the reference's order: -x, -y, -z,
-  // diag, +z, +y, +x
-  Col<float> nc;
-#pragma unroll
-  for (int z = 0; z < 8; ++z) ap.v[z] = 0.f;
-  if (xb == 0) res_face_col(fv, y, nc);  // warp-uniform: the outward face is -x
-  if (x > 0)
-    ps_ld4(fr.ps, own - 8, nc);
-  else if (res_local(fr, fs[0]))
-    ps_ld4(fr.ps, ps_col4(fs[0] - fr.L0, 7, y), nc);
-#pragma unroll
-  for (int z = 0; z < 8; ++z) ap.v[z] = tsub(ap.v[z], nc.v[z]);
-  Col<float> gy;  // the -y face column for lanes at y = 0, the +y one at y = 7
-  res_face_col(fv, (y == 0 ? 8 : 12) + lx, gy);
-  if (y > 0)
-    ps_ld4(fr.ps, own - 1, nc);
-  else if (res_local(fr, fs[2]))
-    ps_ld4(fr.ps, ps_col4(fs[2] - fr.L0, x, 7), nc);
-  else
-    nc = gy;
-#pragma unroll
-  for (int z = 0; z < 8; ++z) ap.v[z] = tsub(ap.v[z], nc.v[z]);
-  const float zm = res_pcell(fr, a, pm_old, tab, beta, fs[4], x, y, 7);
-  const float zp = res_pcell(fr, a, pm_old, tab, beta, fs[5], x, y, 0);
-#pragma unroll
-  for (int z = 0; z < 8; ++z) {
-    const uint8_t g = fbyte(f, z);
-    const float vzm = z == 0 ? zm : P.v[(z + 7) & 7], vzp = z == 7 ? zp : P.v[(z + 1) & 7];
-    ap.v[z] = tsub(ap.v[z], vzm);
-    ap.v[z] = tadd(ap.v[z], tmul(tab[g & 15].d, P.v[z]));
-    ap.v[z] = tsub(ap.v[z], vzp);
-  }
-  if (y < 7)
-    ps_ld4(fr.ps, own + 1, nc);
-  else if (res_local(fr, fs[3]))
-    ps_ld4(fr.ps, ps_col4(fs[3] - fr.L0, x, 0), nc);
-  else
-    nc = gy;
-#pragma unroll
-  for (int z = 0; z < 8; ++z) ap.v[z] = tsub(ap.v[z], nc.v[z]);
-  if (xb != 0) res_face_col(fv, y, nc);  // the outward face is +x
-  if (x < 7)
-    ps_ld4(fr.ps, own + 8, nc);
-  else if (res_local(fr, fs[1]))
-    ps_ld4(fr.ps, ps_col4(fs[1] - fr.L0, 0, y), nc);
-#pragma unroll
-  for (int z = 0; z < 8; ++z) {
-    ap.v[z] = tsub(ap.v[z], nc.v[z]);
-    if (!(fbyte(f, z) & 1)) ap.v[z] = 0.f;
-  }
-}
-
-// r and A p of the CTA's cells live in tensor memory (TMEM): all 512
-// columns, allocated by warp 0; warp w uses TMEM lanes 32 (w % 4) .. + 31
-// (the quarter it may access), and for its half leaf k columns (w / 4) * 32
-// + 8 k .. + 7 for r and the same + kResTmemAp for A p (lane L holds its
-// column's 8 cells).  That leaves the registers to 28 warps, and A p, formed
-// once per iteration for p.Ap, is kept for the update of r; from then to the
-// next S its columns hold z = M r, formed once for r.z and p = z + beta p.  x of half leaf
-// 0 takes columns kResTmemX + (w / 4) * 8 .. + 7; x of half leaves 1 .. 3
-// is in shared memory.  So every vector of the iteration stays on chip, and
-// x is read and written in global memory once per solve.
-constexpr unsigned kResTmemCols = 512;
-constexpr unsigned kResTmemVec = (kResWarps + 3) / 4 * kResHL * 8;  // columns of r or A p
-constexpr unsigned kResTmemAp = kResTmemVec;
-constexpr unsigned kResTmemX = 2 * kResTmemVec;
-static_assert(kResTmemX + (kResWarps + 3) / 4 * 8 <= kResTmemCols, "TMEM columns");
-
-// x of the warp's half leaf k >= 1 in shared memory: two 16-byte chunks per
-// lane (cells z = 0..3 and 4..7), consecutive lanes in consecutive words
-__device__ __forceinline__ void xs_ld(const float4* xs, int k, int warp, int lane, float (&v)[8]) {
-  const float4 u = xs[(((k - 1) * kResWarps + warp) * 2 + 0) * 32 + lane];
-  const float4 w = xs[(((k - 1) * kResWarps + warp) * 2 + 1) * 32 + lane];
-  v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
-  v[4] = w.x; v[5] = w.y; v[6] = w.z; v[7] = w.w;
-}
-__device__ __forceinline__ void xs_st(float4* xs, int k, int warp, int lane, const float (&v)[8]) {
-  xs[(((k - 1) * kResWarps + warp) * 2 + 0) * 32 + lane] = make_float4(v[0], v[1], v[2], v[3]);
-  xs[(((k - 1) * kResWarps + warp) * 2 + 1) * 32 + lane] = make_float4(v[4], v[5], v[6], v[7]);
-}
-__device__ __forceinline__ void tmem_ld8(unsigned t, float (&v)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
-               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]),
-                 "=f"(v[6]), "=f"(v[7])
-               : "r"(t)
-               : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-}
-__device__ __forceinline__ void tmem_st8(unsigned t, const float (&v)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"r"(t),
-               "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]),
-               "f"(v[7])
-               : "memory");
-}
-__device__ __forceinline__ void tmem_wait_st() {
-  asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
-}
-
-__global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(const __grid_constant__ PcgArgs a) {
-  extern __shared__ __align__(16) unsigned char res_smem[];
-  float* ps = reinterpret_cast<float*>(res_smem);
-  uint8_t* fsm = res_smem + size_t(kResLeaves) * 512 * sizeof(float);
-  float4* xs = reinterpret_cast<float4*>(res_smem + size_t(kResLeaves) * 512 * (sizeof(float) + 1));
-  __shared__ DiagInv<float> tab[16];
-  __shared__ int s_ok, s_done;
-  __shared__ float s_fa, s_fbeta;
-  __shared__ ResScalars q;  // thread 0's
-  __shared__ unsigned s_taddr;
-  PcgScalars* sc = a.sc;
-  const int G = int(gridDim.x);
-  const int per = (a.n_pleaf + G - 1) / G;  // the host checks per <= kResLeaves
-  ResFrame fr;
-  fr.ps = ps;
-  fr.fsm = fsm;
-  fr.L0 = int(blockIdx.x) * per;
-  fr.nl = max(0, min(per, a.n_pleaf - fr.L0));
-  fr.n_pleaf = a.n_pleaf;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  fill_diag_table<float>(tab);
-  for (int i = threadIdx.x; i < fr.nl * 512; i += kResThreads) {
-    fsm[i] = a.flags[int64_t(fr.L0) * 512 + i];
-    ps[i] = 0.f;  // p of iteration -1
-  }
-  if (warp == 0) {
-    const unsigned sa = static_cast<unsigned>(__cvta_generic_to_shared(&s_taddr));
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(sa),
-                 "r"(kResTmemCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-  const unsigned tbase = s_taddr + ((32u * unsigned(warp & 3)) << 16) + unsigned(warp >> 2) * 32u;
-  const unsigned txb = s_taddr + ((32u * unsigned(warp & 3)) << 16) + kResTmemX + unsigned(warp >> 2) * 8u;
-  // the warp's half leaves: r and x on chip, the face slots, and which of
-  // the lane's columns other CTAs read (bit k of mir: the column is on a face
-  // whose neighbour leaf is in another CTA, or the leaf's -z or +z neighbour
-  // is, which reads a cell of every column); only those go to the mirrors
-  int nbl[kResHL];
-  unsigned mir = 0;
-#pragma unroll
-  for (int k = 0; k < kResHL; ++k) {
-    const int hl = warp + k * kResWarps;
-    nbl[k] = -1;
-    if (hl < 2 * fr.nl) {
-      const HalfLeaf h = half_pos(2 * fr.L0 + hl, lane);
-      const unsigned og = unsigned(h.s) * 512u + unsigned(h.c);
-      Col<float> r0;
-      ldcol(static_cast<const float*>(a.r), og, r0);
-      tmem_st8(tbase + 8u * k, r0.v);
-      Col<float> z0;
-      {
-        const uint2 f = *reinterpret_cast<const uint2*>(fsm + (hl >> 1) * 512 + h.c);
-#pragma unroll
-        for (int z = 0; z < 8; ++z) z0.v[z] = tmul(tab[fbyte(f, z) & 15].inv, r0.v[z]);
-        tmem_st8(tbase + kResTmemAp + 8u * k, z0.v);
-      }
-      ldcol(static_cast<const float*>(a.x), og, r0);
-      if (k == 0)
-        tmem_st8(txb, r0.v);
-      else
-        xs_st(xs, k, warp, lane, r0.v);
-      nbl[k] = face_slot_lane(a.nbr, h.s, lane);
-      int fs[6];
-      face_slots(nbl[k], fs);
-      const bool xo = h.xb == 0 ? (h.lx == 0 && !res_local(fr, fs[0]))
-                                : (h.lx == 3 && !res_local(fr, fs[1]));
-      const bool yo = (h.cy == 0 && !res_local(fr, fs[2])) || (h.cy == 7 && !res_local(fr, fs[3]));
-      const bool zo = !res_local(fr, fs[4]) || !res_local(fr, fs[5]);
-      if (xo || yo || zo) {
-        mir |= 1u << k;
-        stcol(static_cast<float*>(a.r), og, z0);  // the mirror of z for the first iteration
-      }
-    }
-  }
-  tmem_wait_st();
-  // Thread 0 keeps the scalar state in fp64 and runs the loop test and the
-  // alpha / beta steps (GB300's FP64 pipe is narrow, and the solve's
-  // settings are read once: after the barriers' acquire loads every read of
-  // the scalar block is an L2 round trip); the other threads take the stop
-  // flag and the fp32 alpha and beta from shared memory.
-  int it = sc->iter;
-  if (threadIdx.x == 0) {
-    q = ResScalars{sc->rr, sc->rz, sc->rz_old, 0.0, 0.0, 0.0, sc->status, sc->max_iter, pcg_rule(sc)};
-    s_done = sc->done || it >= q.max_iter || converged(q.rule, q.rr);  // PCGDriver::Solve's loop test
-    s_fbeta = 0.f;
-  }
-  __syncthreads();
-  unsigned round = 0;
-  bool ok = true;
-  float* x = static_cast<float*>(a.x);
-  float* rmir = static_cast<float*>(a.r);  // during the loop: the mirror of z = M r
-  {
-    // every CTA's z mirror is written before any CTA's first stencil reads it
-    float v[1] = {0.f};
-    ok = res_sync<1>(a, v, 0, ++round, &s_ok, [](const double (&)[1]) {});
-  }
-  while (ok && !s_done) {
-    float* pm_new = static_cast<float*>((it & 1) ? a.p1 : a.p0);
-    const float* pm_old = static_cast<const float*>((it & 1) ? a.p0 : a.p1);
-    const float fbeta = s_fbeta;
-    // S: p = z + beta p on the own columns
-#pragma unroll
-    for (int k = 0; k < kResHL; ++k) {
-      const int hl = warp + k * kResWarps;
-      if (hl < 2 * fr.nl) {
-        const HalfLeaf h = half_pos(2 * fr.L0 + hl, lane);
-        Col<float> P;
-        const int own = ps_col4(hl >> 1, h.xb + h.lx, h.cy);
-        ps_ld4(ps, own, P);
-        float zk[8];  // z = M r, left in the A p columns by U (or the set-up)
-        tmem_ld8(tbase + kResTmemAp + 8u * k, zk);
-#pragma unroll
-        for (int z = 0; z < 8; ++z) P.v[z] = tadd(zk[z], tmul(fbeta, P.v[z]));  // pnew_of's operations
-        ps_st4(ps, own, P);
-        if ((mir >> k) & 1u) stcol(pm_new, unsigned(h.s) * 512u + unsigned(h.c), P);
-      }
-    }
-    __syncthreads();
-    Dot<0> dp;
-#pragma unroll
-    for (int k = 0; k < kResHL; ++k) {
-      const int hl = warp + k * kResWarps;
-      int fs[6];
-      face_slots(nbl[k], fs);
-      if (hl < 2 * fr.nl) {
-        const HalfLeaf h = half_pos(2 * fr.L0 + hl, lane);
-        const int ol = (hl >> 1) * 512 + h.c;
-        Col<float> P, ap;
-        ps_ld4(ps, ps_col4(hl >> 1, h.xb + h.lx, h.cy), P);
-        const uint2 f = *reinterpret_cast<const uint2*>(fsm + ol);
-        res_ap(fr, a, pm_old, tab, fbeta, h.s, h.xb, h.lx, h.cy, lane, fs, P, f, ap);
-#pragma unroll
-        for (int z = 0; z < 8; ++z) dp.add(P.v[z], ap.v[z]);
-        tmem_st8(tbase + kResTmemAp + 8u * k, ap.v);
-      }
-    }
-    tmem_wait_st();
-    {
-      float v[1] = {dp.pvalue()};
-      ok = res_sync<1>(a, v, 0, ++round, &s_ok, [&](const double (&tot)[1]) {
-        q.pAp = round_t(q.rule, tot[0]);
-        q.alpha = q.rule.fp32 ? double(__fdiv_rn(float(q.rz), float(q.pAp))) : q.rz / q.pAp;
-        s_fa = float(q.alpha);
-        if (!(q.alpha <= 1e5)) {  // CHECK_LE(alpha, LARGE_FLOAT)
-          q.status = FSIM_ERR_BREAKDOWN;
-          s_done = 1;
-        }
-      });
-      if (!ok || s_done) break;
-    }
-    // U: x += alpha p, r -= alpha A p
-    const float fa = s_fa, fna = -fa;
-    Dot<0> drr, drz;
-#pragma unroll
-    for (int k = 0; k < kResHL; ++k) {
-      const int hl = warp + k * kResWarps;
-      if (hl < 2 * fr.nl) {
-        const HalfLeaf h = half_pos(2 * fr.L0 + hl, lane);
-        const int ol = (hl >> 1) * 512 + h.c;
-        const unsigned og = unsigned(h.s) * 512u + unsigned(h.c);
-        Col<float> P, X, R;
-        if (k == 0)
-          tmem_ld8(txb, X.v);
-        else
-          xs_ld(xs, k, warp, lane, X.v);
-        ps_ld4(ps, ps_col4(hl >> 1, h.xb + h.lx, h.cy), P);
-        const uint2 f = *reinterpret_cast<const uint2*>(fsm + ol);
-#pragma unroll
-        for (int z = 0; z < 8; ++z) X.v[z] = tadd(tmul(fa, P.v[z]), X.v[z]);
-        if (k == 0)
-          tmem_st8(txb, X.v);
-        else
-          xs_st(xs, k, warp, lane, X.v);
-        float ap[8];
-        tmem_ld8(tbase + 8u * k, R.v);
-        tmem_ld8(tbase + kResTmemAp + 8u * k, ap);
-#pragma unroll
-        for (int z = 0; z < 8; ++z) {
-          const uint8_t g = fbyte(f, z);
-          R.v[z] = tadd(tmul(fna, ap[z]), R.v[z]);
-          drr.add(R.v[z], R.v[z]);
-          ap[z] = tmul(tab[g & 15].inv, R.v[z]);  // z = M r, for r.z and the next S
-          drz.add(R.v[z], ap[z]);
-        }
-        tmem_st8(tbase + 8u * k, R.v);
-        tmem_st8(tbase + kResTmemAp + 8u * k, ap);
-        if ((mir >> k) & 1u) {
-          Col<float> Z;
-#pragma unroll
-          for (int z = 0; z < 8; ++z) Z.v[z] = ap[z];
-          stcol(rmir, og, Z);
-        }
-      }
-    }
-    tmem_wait_st();
-    {
-      float v[2] = {drr.pvalue(), drz.pvalue()};
-      ok = res_sync<2>(a, v, 1, ++round, &s_ok, [&](const double (&tot)[2]) {
-        q.rr = round_t(q.rule, tot[0]);
-        const double rzn = round_t(q.rule, tot[1]);
-        q.beta = q.rule.fp32 ? double(__fdiv_rn(float(rzn), float(q.rz))) : rzn / q.rz;
-        q.rz_old = q.rz;
-        q.rz = rzn;
-        s_fbeta = float(q.beta);
-        if (!(q.beta <= 1e5)) {  // CHECK_LE(beta, LARGE_FLOAT)
-          q.status = FSIM_ERR_BREAKDOWN;
-          s_done = 1;
-        } else {
-          s_done = (it + 1 >= q.max_iter) || converged(q.rule, q.rr);  // the next loop test
-        }
-      });
-      if (!ok) break;
-      ++it;
-    }
-  }
-  if (!ok && threadIdx.x == 0) q.status = FSIM_ERR_TIMEOUT;
-  // x and r back to global memory; every warp is then done with TMEM, and
-  // warp 0 frees it
-  tmem_wait_st();
-#pragma unroll
-  for (int k = 0; k < kResHL; ++k) {
-    const int hl = warp + k * kResWarps;
-    if (hl < 2 * fr.nl) {
-      const HalfLeaf h = half_pos(2 * fr.L0 + hl, lane);
-      const unsigned og = unsigned(h.s) * 512u + unsigned(h.c);
-      Col<float> X;
-      if (k == 0)
-        tmem_ld8(txb, X.v);
-      else
-        xs_ld(xs, k, warp, lane, X.v);
-      stcol(x, og, X);
-      tmem_ld8(tbase + 8u * k, X.v);
-      stcol(rmir, og, X);
-    }
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-  __syncthreads();
-  if (warp == 0) {
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(s_taddr),
-                 "r"(kResTmemCols)
-                 : "memory");
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    sc->iter = it;
-    sc->done = 1;
-    sc->status = q.status;
-    sc->rr = q.rr;
-    sc->rz = q.rz;
-    sc->rz_old = q.rz_old;
-    sc->alpha = q.alpha;
-    sc->beta = q.beta;
-    sc->pAp = q.pAp;
-  }
-}
-
 // MIXED: x64 += d (inner solution); d is the fp32 x of the inner solve.
 __global__ void k_accumulate_x64(const __grid_constant__ PcgArgs a) {
   const int64_t n = int64_t(a.n_pleaf) * 512;
@@ -2750,15 +2170,31 @@ struct LoopTimer {
 
 #include "pcg_cluster.cuh"
 
-// The cluster loop takes FP32 and MIXED solves of at most kClLeaves particle
-// leaves (what its shared memory and registers hold), unless another loop is
-// asked for by its switch: it is the fastest loop at every such size
-// (pcg_cluster.cuh; at 232 leaves 5.1 us per iteration against the resident
-// loop's 6.4 and the pair's 6.7).  FP64 is bound by the FP64 pipe, which 16
-// SMs hold too little of.
+// The cluster loop takes small FP32 and MIXED solves, unless another loop is
+// asked for by its switch: up to two leaves per warp of 8 for FP32 (at 216 to
+// 236 leaves 5.0 - 5.2 us per iteration against the resident loop's 5.5) and
+// one leaf per warp of 12 for MIXED (with two it takes 8.3 us at 232 leaves,
+// the resident loop 7.4; with one, 5.0 against 7.5 at 189).  FP64 is bound by
+// the FP64 pipe, which 16 SMs hold too little of.
 bool use_cluster(const fsim_sim* s, int precision) {
+  const int most = precision == FSIM_PREC_FP32 ? kClLeaves : kClLeavesMixed;
   return precision != FSIM_PREC_FP64 && s->pcg_res < 0 && s->pcg_cluster && s->n_pleaf > 0 &&
-         s->n_pleaf <= kClLeaves && !(precision == FSIM_PREC_FP32 && s->pcg_cg1 == 1);
+         s->n_pleaf <= most && !(precision == FSIM_PREC_FP32 && s->pcg_cg1 == 1);
+}
+
+#include "pcg_resident.cuh"
+
+// The resident loop takes every other solve that fits on chip (56 particle
+// leaves per SM, 13 for FP64): it beats the pair at all such sizes (tables in
+// pcg_resident.cuh; at one leaf per SM 5.5 against 6.5 us per iteration for
+// FP32, 7.5 / 9.2 for MIXED, 9.5 / 19.7 for FP64).  FSIM_PCG_RES=0 / 1 turns
+// it off / on ahead of the cluster loop.  FSIM_PCG_CG1=1 keeps the sizes at
+// which its loop was ever chosen, below two leaves per SM.
+bool use_resident(const fsim_sim* s, int precision) {
+  const int64_t most = precision == FSIM_PREC_FP64 ? kR64Leaves : kResLeaves;
+  if (precision == FSIM_PREC_FP32 && s->pcg_cg1 == 1 && s->pcg_res < 0 && s->n_pleaf < 2 * s->num_sms)
+    return false;
+  return s->pcg_res != 0 && s->n_pleaf > 0 && s->n_pleaf <= most * s->num_sms;
 }
 
 // One inner solve: setup, then the iterations.  The iterations run as a CUDA
@@ -2774,12 +2210,18 @@ int run_inner(fsim_sim* s, PcgArgs& a, int grid, const char* nm_setup, const cha
               const char* nm_upd, bool setup = true, int par0 = 0) {
   a.cond = 0;
   if (setup) FSIM_LAUNCH(s, nm_setup, (k_pcg_setup<T, DM>), grid, kThreads, 0, a);
+  constexpr int prec = DM == 0 ? FSIM_PREC_FP32 : (DM == 1 ? FSIM_PREC_MIXED : FSIM_PREC_FP64);
   if constexpr (DM < 2) {
-    if (use_cluster(s, DM == 0 ? FSIM_PREC_FP32 : FSIM_PREC_MIXED)) {
+    if (use_cluster(s, prec)) {
       const int rc = run_cluster<DM>(s, a);
       if (rc != FSIM_ERR_CUDA) return rc;
-      s->pcg_cluster = false;  // refused: the pair, for the rest of this handle's life
+      s->pcg_cluster = false;  // refused: another loop, for the rest of this handle's life
     }
+  }
+  if (use_resident(s, prec)) {
+    const int rc = run_resident<DM>(s, a);
+    if (rc != FSIM_ERR_CUDA) return rc;
+    s->pcg_res = 0;  // a refused cooperative launch: the pair
   }
   const int wpb = kHotThreads / 32;
   int occ_a = 1, occ_b = 1;
@@ -2911,52 +2353,6 @@ int run_cg1(fsim_sim* s, PcgArgs& a, int grid) {
   return FSIM_OK;
 }
 
-// One fp32 solve by the resident loop: setup, then one cooperative launch of
-// one CTA per SM that runs every iteration.  FSIM_ERR_CUDA when the launch is
-// refused (the caller then runs the pair).
-int run_resident(fsim_sim* s, PcgArgs& a, int grid) {
-  void* const fn = reinterpret_cast<void*>(k_pcg_resident);
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kResSmem)) !=
-      cudaSuccess) {
-    cudaGetLastError();
-    return FSIM_ERR_CUDA;
-  }
-  int occ = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kResThreads, kResSmem);
-  if (occ < 1) return FSIM_ERR_CUDA;
-  a.cond = 0;
-  FSIM_LAUNCH(s, "pcg_setup", (k_pcg_setup<float, 0>), grid, kThreads, 0, a);
-  LoopTimer lt(s);
-  {
-    fsim::ProfScope ps(s, "pcg_resident");
-    void* args[] = {&a};
-    const cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(unsigned(s->num_sms)),
-                                                      dim3(unsigned(kResThreads)), args, kResSmem,
-                                                      s->stream);
-    s->launches++;
-    if (e != cudaSuccess) return cuda_fail(s, e, "pcg_resident");
-  }
-  lt.stop();
-  FSIM_CK(s, cudaMemcpyAsync(s->h_sc, a.sc, sizeof(PcgScalars), cudaMemcpyDeviceToHost, s->stream));
-  FSIM_CK(s, cudaStreamSynchronize(s->stream));
-  if (s->h_sc->bar_err) return fail(s, FSIM_ERR_TIMEOUT, "PCG: a resident-loop barrier gave up");
-  return FSIM_OK;
-}
-// The resident loop takes fp32 solves whose particle leaves fit (at most
-// kResLeaves per SM) and are many enough to amortise its fixed cost per
-// iteration (two grid barriers, about 7.6 us in all): from kResMinLeaves per
-// SM.  Measured per iteration against the pair: 20.95 against 32.1 us at
-// 256^3 (55 leaves per SM), 9.0 against 12.45 at 128^3 (7.6), 7.9 against
-// 6.5-7.0 at 64^3 (about one leaf per SM); the two meet near two leaves per
-// SM.  FSIM_PCG_RES=0 / 1 turns it off / on wherever it fits.
-constexpr int kResMinLeaves = 2;
-bool use_resident(const fsim_sim* s, int precision) {
-  if (precision != FSIM_PREC_FP32 || s->pcg_res == 0) return false;
-  const int64_t n = s->n_pleaf, sms = s->num_sms;
-  if (n > int64_t(kResLeaves) * sms) return false;
-  return s->pcg_res > 0 || n >= int64_t(kResMinLeaves) * sms;
-}
-
 // fp32 solves take the single-reduction iteration on request (FSIM_PCG_CG1=1).
 // It saves one launch's fixed cost per iteration (5.1 against 7.0 us per
 // iteration at 64^3, 9.9 against 12.5 at 128^3) but moves 41 B per unknown
@@ -3052,19 +2448,7 @@ int pcg_solve(fsim_sim* s, const fsim_pcg_params* prm, fsim_pcg_stats* st, const
     *s->h_sc = h;
     FSIM_CK(s, cudaMemcpyAsync(s->d_sc, s->h_sc, sizeof(PcgScalars), cudaMemcpyHostToDevice,
                                s->stream));
-    if (use_cluster(s, prm->precision)) {
-      rc = run_inner<float, 0>(s, a, grid, "pcg_setup", "pcg_spmv", "pcg_update");
-    } else if (use_resident(s, prm->precision)) {
-      rc = run_resident(s, a, grid);
-      if (rc == FSIM_ERR_CUDA) {  // cooperative launch refused: the pair
-        cudaGetLastError();
-        s->pcg_res = 0;
-        *s->h_sc = h;
-        FSIM_CK(s, cudaMemcpyAsync(s->d_sc, s->h_sc, sizeof(PcgScalars), cudaMemcpyHostToDevice,
-                                   s->stream));
-        rc = run_inner<float, 0>(s, a, grid, "pcg_setup", "pcg_spmv", "pcg_update");
-      }
-    } else if (use_cg1(s, prm->precision)) {
+    if (use_cg1(s, prm->precision) && !use_resident(s, prm->precision)) {
       for (int b = 0; b < 2; ++b) {
         a.w[b] = s->cgw[b];
         a.sv[b] = s->cgs[b];

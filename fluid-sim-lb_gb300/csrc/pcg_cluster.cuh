@@ -31,8 +31,8 @@
 // Measured us per iteration, against the pair (sphere drop; particle leaves):
 //   leaves        24          84          156         189         232
 //   FP32     2.15 / 6.57  2.65 / 6.42  3.21 / 6.51  3.43 / 6.48  5.10 / 6.66
-//   MIXED    3.58 / 10.1  4.17 / 9.32  4.88 / 9.17  5.04 / 9.51  8.28 / 9.90
-// (the resident loop: 5.9 to 6.6).  At 24 leaves it is latency (two one-way
+//   MIXED    3.58 / 10.1  4.17 / 9.32  4.88 / 9.17  5.04 / 9.51  (8.28 / 9.90)
+// (the resident loop: 5.0 to 5.5 for FP32, 7.4 to 7.7 for MIXED).  At 24 leaves it is latency (two one-way
 // pushes, four CTA barriers, six warp reductions); from about 100 on also the
 // bandwidth of shared memory.
 //
@@ -41,9 +41,29 @@
 // barrier, so no CTA's shared memory goes while another may still reach it.
 constexpr int kClCtas = 16;                       // CTAs of the cluster (one per SM)
 constexpr int kClWarps = 12;                      // warps per CTA, at most (168 registers)
-constexpr int kClPerWarp = 2;                     // leaves per warp, at most
-constexpr int kClLeaves = kClCtas * kClWarps * kClPerWarp;  // 384 particle leaves
+constexpr int kClPerWarp = 2;                     // leaves per warp, at most (FP32)
+constexpr int kClLeaves = 256;                    // particle leaves: FP32
+constexpr int kClLeavesMixed = kClCtas * kClWarps;  // 192: MIXED, one per warp
 constexpr unsigned kClPolls = 1u << 22;
+
+// p of a CTA's leaves in shared memory (here and in the resident loop), in 16-byte chunk planes: float4 element
+// ((leaf * 2 + chunk) * 8 + x) * 8 + y holds the cells z = 4 chunk ..
+// 4 chunk + 3 of column (x, y), so the lanes of a quarter warp (consecutive
+// y) touch consecutive 16-byte words.  ps_col4 is the float4 index of chunk 0
+// of a column; chunk 1 is 64 further, and the in-leaf neighbour columns are
+// -8 / +8 (x) and -1 / +1 (y) away, constant offsets from the own column.
+__device__ __forceinline__ int ps_col4(int leaf, int x, int y) { return (leaf * 16 + x) * 8 + y; }
+__device__ __forceinline__ void ps_ld4(const float* ps, int i, Col<float>& c) {
+  const float4* q = reinterpret_cast<const float4*>(ps);
+  const float4 u = q[i], w = q[i + 64];
+  c.v[0] = u.x; c.v[1] = u.y; c.v[2] = u.z; c.v[3] = u.w;
+  c.v[4] = w.x; c.v[5] = w.y; c.v[6] = w.z; c.v[7] = w.w;
+}
+__device__ __forceinline__ void ps_st4(float* ps, int i, const Col<float>& c) {
+  float4* q = reinterpret_cast<float4*>(ps);
+  q[i] = make_float4(c.v[0], c.v[1], c.v[2], c.v[3]);
+  q[i + 64] = make_float4(c.v[4], c.v[5], c.v[6], c.v[7]);
+}
 
 __device__ __forceinline__ unsigned cl_rank() {
   unsigned r;
@@ -87,6 +107,10 @@ __device__ __forceinline__ float cl_ldcell(unsigned addr) {
 
 template <typename P>
 __device__ __forceinline__ P pshfl_xor(P v, int o);
+template <>
+__device__ __forceinline__ double pshfl_xor<double>(double v, int o) {
+  return __shfl_xor_sync(0xffffffffu, v, o);
+}
 template <>
 __device__ __forceinline__ float pshfl_xor<float>(float v, int o) {
   return __shfl_xor_sync(0xffffffffu, v, o);
@@ -203,6 +227,7 @@ __device__ __forceinline__ float cl_div(float2 a, float2 b) {
   const float s = __fadd_rn(q, d);
   return s == s ? s : q;  // inf and NaN quotients stay what the leading term says
 }
+__device__ __forceinline__ void cl_split(double v, double& o) { o = v; }
 __device__ __forceinline__ void cl_split(double v, float& o) { o = float(v); }
 __device__ __forceinline__ void cl_split(double v, float2& o) {
   o.x = float(v);
@@ -223,6 +248,20 @@ struct ClStop {
   P thr;
   bool fixed, strict;
 };
+template <typename P>
+__device__ __forceinline__ ClStop<P> cl_stop_of(const PcgScalars* sc) {
+  ClStop<P> q;
+  q.fixed = sc->mode == FSIM_PCG_FIXED;
+  q.strict = sc->mode == FSIM_PCG_ABSOLUTE;
+  if constexpr (std::is_same<P, float>::value)
+    q.thr = q.strict ? float(sc->thr) : __double2float_rd(sc->thr);
+  else
+    cl_split(sc->thr, q.thr);
+  return q;
+}
+__device__ __forceinline__ bool cl_stop(const ClStop<double>& q, double rr) {
+  return !q.fixed && (q.strict ? rr < q.thr : rr <= q.thr);
+}
 __device__ __forceinline__ bool cl_stop(const ClStop<float>& q, float rr) {
   return !q.fixed && (q.strict ? rr < q.thr : rr <= q.thr);
 }
@@ -442,13 +481,7 @@ __global__ void __launch_bounds__(kClWarps * 32, 1)
   float alpha = 0.f, beta = float(sc->beta);
   int it = sc->iter, status = sc->status;
   const int max_it = sc->max_iter;
-  ClStop<P> stop;
-  stop.fixed = sc->mode == FSIM_PCG_FIXED;
-  stop.strict = sc->mode == FSIM_PCG_ABSOLUTE;
-  if constexpr (DM == 0)
-    stop.thr = stop.strict ? float(sc->thr) : __double2float_rd(sc->thr);
-  else
-    cl_split(sc->thr, stop.thr);
+  const ClStop<P> stop = cl_stop_of<P>(sc);
   const int it0 = it;
   unsigned tag = 0;
   bool bad = false;
@@ -636,8 +669,10 @@ int run_cluster(fsim_sim* s, PcgArgs& a) {
   const int per = (a.n_pleaf + kClCtas - 1) / kClCtas;
   const int KH = per <= kClWarps ? 1 : kClPerWarp;
   const int W = (per + KH - 1) / KH;
-  const void* fn = KH == 1 ? reinterpret_cast<const void*>(k_pcg_cluster<DM, 1>)
-                           : reinterpret_cast<const void*>(k_pcg_cluster<DM, kClPerWarp>);
+  const void* fn = reinterpret_cast<const void*>(k_pcg_cluster<DM, 1>);
+  if constexpr (DM == 0) {
+    if (KH > 1) fn = reinterpret_cast<const void*>(k_pcg_cluster<DM, kClPerWarp>);
+  }
   const int most = int(cl_layout(kClWarps, KH).bytes);
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e == cudaSuccess)
