@@ -200,6 +200,8 @@ struct fsim_sim {
   // around the PCG iteration loops (fsim_pcg_stats::loop_ms)
   cudaEvent_t ev_loop[2] = {nullptr, nullptr};
   double pcg_loop_ms = 0.0;
+  bool pcg_defer = false;    // the solve in progress may stay in flight
+  bool pcg_pending = false;  // it does: pcg_collect reads its results
   float* io_stage = nullptr;   // AoS staging of the early position download
   int64_t io_stage_cap = 0;
   bool io_vel_pending = false; // vel upload in flight on io_stream (ev_io)
@@ -382,6 +384,10 @@ int rebin_uploaded(fsim_sim* s, int64_t* invalid);
 
 // kernel entry points implemented in the .cu files
 int launch_keys_from_positions(fsim_sim* s, int mode, float dt);
+// fsim_step_host: keys of the n_total uploaded rows after the move, for
+// rebuild_topology; *invalid: positions outside [0, N] (then nothing is set up)
+int launch_host_keys(fsim_sim* s, const float* pos, const float* gvel, float dt, bool keep_gvel,
+                     int64_t* invalid);
 int launch_p2g(fsim_sim* s, bool fused, float dt);
 int launch_apply_bc(fsim_sim* s);
 int launch_save_velocities(fsim_sim* s);
@@ -394,8 +400,12 @@ int launch_cfl(fsim_sim* s);
 int launch_g2p(fsim_sim* s);
 // b64: an fp64 right-hand side on the particle-leaf cells instead of the
 // divergence (the solution is then read from x64: FP64 / MIXED precision)
+// defer: where the iterations are one launch (the cluster and resident loops
+// of FP32 and FP64), return with the solve in flight; after the stream's next
+// synchronisation pcg_collect fills st (and reports a timeout)
 int pcg_solve(fsim_sim* s, const fsim_pcg_params* prm, fsim_pcg_stats* st,
-              const double* b64 = nullptr);
+              const double* b64 = nullptr, bool defer = false);
+int pcg_collect(fsim_sim* s, const fsim_pcg_params* prm, fsim_pcg_stats* st);
 int ensure_dense(fsim_sim* s, size_t bytes);  // dense_tmp of at least bytes
 int download_dense(fsim_sim* s, int field, float* out, uint8_t* active);
 int download_marker(fsim_sim* s, int32_t* out, uint8_t* active);

@@ -2157,6 +2157,15 @@ struct LoopTimer {
     on = s->ev_loop[0] && s->ev_loop[1] &&
          cudaEventRecord(s->ev_loop[0], s->stream) == cudaSuccess;
   }
+  void mark() { on = on && cudaEventRecord(s->ev_loop[1], s->stream) == cudaSuccess; }
+  // the time between the marks, once the second one has been reached
+  static void collect(fsim_sim* s) {
+    float ms = 0.f;
+    if (s->ev_loop[1] && cudaEventElapsedTime(&ms, s->ev_loop[0], s->ev_loop[1]) == cudaSuccess)
+      s->pcg_loop_ms += double(ms);
+    else
+      cudaGetLastError();
+  }
   void stop() {
     if (on && cudaEventRecord(s->ev_loop[1], s->stream) == cudaSuccess) {
       cudaEventSynchronize(s->ev_loop[1]);
@@ -2167,6 +2176,21 @@ struct LoopTimer {
     on = false;
   }
 };
+
+// The end of a loop that is one launch: its scalars to the host, and, unless
+// the solve may stay in flight, the wait for them.
+int end_one_launch(fsim_sim* s, const PcgArgs& a, LoopTimer& lt) {
+  lt.mark();
+  FSIM_CK(s, cudaMemcpyAsync(s->h_sc, a.sc, sizeof(PcgScalars), cudaMemcpyDeviceToHost, s->stream));
+  if (s->pcg_defer) {
+    s->pcg_pending = true;
+    return FSIM_OK;
+  }
+  FSIM_CK(s, cudaStreamSynchronize(s->stream));
+  LoopTimer::collect(s);
+  if (s->h_sc->bar_err) return fail(s, FSIM_ERR_TIMEOUT, "PCG: an on-chip loop's wait gave up");
+  return FSIM_OK;
+}
 
 #include "pcg_cluster.cuh"
 
@@ -2386,7 +2410,31 @@ int ensure_pcg_vectors(fsim_sim* s, int precision) {
 
 }  // namespace
 
-int pcg_solve(fsim_sim* s, const fsim_pcg_params* prm, fsim_pcg_stats* st, const double* b64) {
+// Results of the FP32 and FP64 solves, from the scalars on the host
+static void one_solve_stats(fsim_sim* s, const fsim_pcg_params* prm, fsim_pcg_stats* st) {
+  int status = s->h_sc->status;
+  if (status == FSIM_OK && prm->mode == FSIM_PCG_RELATIVE && !(s->h_sc->rr <= s->h_sc->thr))
+    status = FSIM_ERR_NOT_CONVERGED;
+  st->iterations = s->h_sc->iter;
+  st->refinements = 1;
+  st->n_rows = int32_t(s->h_sc->n_rows);
+  st->status = status;
+  st->rr = s->h_sc->rr;
+  st->bb = s->h_sc->bb;
+  st->loop_ms = s->pcg_loop_ms;
+}
+
+int pcg_collect(fsim_sim* s, const fsim_pcg_params* prm, fsim_pcg_stats* st) {
+  if (!s->pcg_pending) return FSIM_OK;  // the solve has reported already
+  s->pcg_pending = false;
+  LoopTimer::collect(s);
+  if (s->h_sc->bar_err) return fail(s, FSIM_ERR_TIMEOUT, "PCG: an on-chip loop's wait gave up");
+  one_solve_stats(s, prm, st);
+  return FSIM_OK;
+}
+
+int pcg_solve(fsim_sim* s, const fsim_pcg_params* prm, fsim_pcg_stats* st, const double* b64,
+              bool defer) {
   if (!prm) return fail(s, FSIM_ERR_INVALID, "pcg params missing");
   if (prm->mode < 0 || prm->mode > 2 || prm->precision < 0 || prm->precision > 2)
     return fail(s, FSIM_ERR_INVALID, "bad pcg mode/precision");
@@ -2397,6 +2445,8 @@ int pcg_solve(fsim_sim* s, const fsim_pcg_params* prm, fsim_pcg_stats* st, const
   if (rc) return rc;
   s->pcg_loop_ms = 0.0;
   s->pcg_seg_max = 0;
+  s->pcg_pending = false;
+  s->pcg_defer = defer && prm->precision != FSIM_PREC_MIXED && !s->profiling;
   const int grid = std::max(1, std::min(s->n_pleaf, s->max_blocks));
   PcgArgs a;
   memset(&a, 0, sizeof(a));
@@ -2459,17 +2509,13 @@ int pcg_solve(fsim_sim* s, const fsim_pcg_params* prm, fsim_pcg_stats* st, const
     else
       rc = run_inner<double, 2>(s, a, grid, "pcg_setup_f64", "pcg_spmv_f64", "pcg_update_f64");
     if (rc) return rc;
-    total_it = s->h_sc->iter;
-    n_rows = int64_t(s->h_sc->n_rows);
-    final_rr = s->h_sc->rr;
-    bb = s->h_sc->bb;
-    status = s->h_sc->status;
-    if (status == FSIM_OK && prm->mode == FSIM_PCG_RELATIVE && !(final_rr <= s->h_sc->thr))
-      status = FSIM_ERR_NOT_CONVERGED;
     if (prm->precision == FSIM_PREC_FP64)
       FSIM_LAUNCH(s, "pcg_to_pressure", k_to_pressure<double>,
                   unsigned(std::min<int64_t>((nvec + 255) / 256, 4096)), 256, 0, s->x64, s->pres,
                   nvec);
+    if (s->pcg_seg_max > 0) s->pcg_last_iters = s->pcg_seg_max;
+    if (st && !s->pcg_pending) one_solve_stats(s, prm, st);
+    return FSIM_OK;
   } else {
     // MIXED: fp32 Jacobi-PCG with exact dots, and fp64 residual replacement
     // (reliable updates): each time the recursive residual has dropped by

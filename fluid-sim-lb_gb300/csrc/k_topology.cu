@@ -125,6 +125,72 @@ __global__ void k_keys(float* __restrict__ part, int64_t cap, const uint32_t* __
   }
 }
 
+// The keys of a step on a host-resident state (fsim_step_host), one pass over
+// the uploaded rows: validity and cell key of the uploaded position (kold),
+// then mode 1's advection, clamping, deletion in solids and key (knew), with
+// the advected position stored (and gvel, for a gather that moves it).  Counts
+// positions outside [0, N] and neighbouring rows out of cell order.  The rows
+// need no rebinning of their own first: by (new key, old key, row) they are in
+// the order that rebinning them, moving them and rebinning again gives.
+__global__ void __launch_bounds__(256)
+    k_host_keys(const float* __restrict__ pos, const float* __restrict__ gvel,
+                float* __restrict__ part, int64_t cap, uint32_t* __restrict__ kold,
+                uint32_t* __restrict__ knew, uint32_t* __restrict__ vout, int64_t n, LeafMap lm,
+                SolidDesc sd, float dt, int keep_gvel, unsigned long long* __restrict__ invalid,
+                unsigned long long* __restrict__ unsorted) {
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  auto old_key = [&](int64_t r, float (&p)[3]) {
+    bool ok = true;
+    int id[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      p[d] = pos[3 * r + d];
+      ok &= (p[d] >= 0.f) && (p[d] <= float(lm.n[d]));
+      id[d] = int(floorf(p[d]));
+    }
+    return ok ? cell_key(lm, id[0], id[1], id[2]) : kDeadKey;
+  };
+  float p[3] = {0.f, 0.f, 0.f}, q[3];
+  const uint32_t old = i < n ? old_key(i, p) : kDeadKey;
+  uint32_t next = __shfl_down_sync(0xffffffffu, old, 1);
+  if ((threadIdx.x & 31) == 31) next = i + 1 < n ? old_key(i + 1, q) : kDeadKey;
+  const unsigned desc = __ballot_sync(0xffffffffu, i + 1 < n && old > next);
+  const unsigned bad = __ballot_sync(0xffffffffu, i < n && old == kDeadKey);
+  if ((threadIdx.x & 31) == 0) {
+    if (desc) atomicAdd(unsorted, static_cast<unsigned long long>(__popc(desc)));
+    if (bad) atomicAdd(invalid, static_cast<unsigned long long>(__popc(bad)));
+  }
+  if (i >= n) return;
+  int id[3];
+  float g[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    g[d] = gvel[3 * i + d];
+    p[d] = fadd(p[d], fmul(g[d], dt));
+    id[d] = int(floorf(p[d]));
+  }
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+    if (id[d] < 0) { id[d] = 0; p[d] = 0.f; }
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+    if (id[d] >= lm.n[d]) { id[d] = lm.n[d]; p[d] = float(lm.n[d]); }
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    part[d * cap + i] = p[d];
+    if (keep_gvel) part[(6 + d) * cap + i] = g[d];
+  }
+  kold[i] = old;
+  knew[i] = is_solid(sd, id[0], id[1], id[2]) ? kDeadKey : cell_key(lm, id[0], id[1], id[2]);
+  vout[i] = uint32_t(i);
+}
+
+__global__ void k_permute_keys(const uint32_t* __restrict__ in, const uint32_t* __restrict__ perm,
+                               uint32_t* __restrict__ out, int64_t n) {
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = in[perm[i]];
+}
+
 // Live particles = index of the first dead key: the keys are sorted and the
 // dead key is the largest value.  One block narrows [lo, hi] (which holds
 // that index; hi = n when no key is dead) by probing blockDim.x evenly spaced
@@ -531,6 +597,69 @@ SourceRegions regions_at(const fsim_sim* s, float t) {
 
 }  // namespace
 
+// stable radix sort of (key, value) pairs by cell key
+static int sort_pairs(fsim_sim* s, const uint32_t* kin, uint32_t* kout, const uint32_t* vin,
+                      uint32_t* vout, int64_t n) {
+  const int bits = key_bits(s->lm);
+  size_t need = 0;
+  FSIM_CK(s, cub::DeviceRadixSort::SortPairs(nullptr, need, kin, kout, vin, vout, n, 0, bits,
+                                             s->stream));
+  if (need > s->sort_tmp_bytes) {
+    if (s->sort_tmp) cudaFree(s->sort_tmp);
+    s->sort_tmp = nullptr;
+    s->sort_tmp_bytes = 0;
+    FSIM_CK(s, cudaMalloc(&s->sort_tmp, need));
+    s->sort_tmp_bytes = need;
+  }
+  if (n > 0) {
+    fsim::ProfScope ps(s, "radix_sort(cub)");
+    FSIM_CK(s, cub::DeviceRadixSort::SortPairs(s->sort_tmp, need, kin, kout, vin, vout, n, 0, bits,
+                                               s->stream));
+  }
+  return FSIM_OK;
+}
+
+static int ensure_keys64(fsim_sim* s, int64_t n) {
+  if (n <= s->cap64) return FSIM_OK;
+  s->cap64 = 0;
+  for (int b = 0; b < 2; ++b) {
+    if (s->keys64[b]) cudaFree(s->keys64[b]);
+    s->keys64[b] = nullptr;
+    FSIM_CK(s, cudaMalloc(&s->keys64[b], size_t(std::max<int64_t>(n, 1)) * 8));
+  }
+  s->cap64 = n;
+  return FSIM_OK;
+}
+
+int launch_host_keys(fsim_sim* s, const float* pos, const float* gvel, float dt, bool keep_gvel,
+                     int64_t* invalid) {
+  const int64_t n = s->n_total;
+  unsigned long long* cnt = reinterpret_cast<unsigned long long*>(s->d_cnt);
+  FSIM_CK(s, cudaMemsetAsync(s->d_cnt + 3, 0, 5 * sizeof(int64_t), s->stream));
+  FSIM_LAUNCH(s, "advect_keys", k_host_keys, nblk(n, 256), 256, 0, pos, gvel, s->part[s->cur],
+              s->cap_p, s->keys[0], s->keys[1], s->vals[1], n, s->lm, s->solid, dt,
+              keep_gvel ? 1 : 0, cnt + 3, cnt + 7);
+  FSIM_CK(s, cudaMemcpyAsync(s->h_cnt + 3, s->d_cnt + 3, 5 * sizeof(int64_t),
+                             cudaMemcpyDeviceToHost, s->stream));
+  FSIM_CK(s, cudaStreamSynchronize(s->stream));
+  *invalid = s->h_cnt[3];
+  s->composite_sort = false;
+  if (*invalid || s->h_cnt[7] == 0) return FSIM_OK;
+  // rows out of cell order: their old cells decide the order within a new cell,
+  // so they are sorted by old key first and by new key after (stable; one sort
+  // of (new, old) as 64-bit keys takes 2.8 ms at 32 M rows, these two 1.7)
+  int rc = ensure_keys64(s, (n + 1) / 2);
+  if (rc) return rc;
+  if ((rc = sort_pairs(s, s->keys[0], reinterpret_cast<uint32_t*>(s->keys64[0]), s->vals[1],
+                       s->vals[0], n)))
+    return rc;
+  FSIM_LAUNCH(s, "permute_keys", k_permute_keys, nblk(n, 256), 256, 0, s->keys[1], s->vals[0],
+              s->keys[0], n);
+  std::swap(s->keys[0], s->keys[1]);
+  std::swap(s->vals[0], s->vals[1]);
+  return FSIM_OK;
+}
+
 int launch_keys_from_positions(fsim_sim* s, int mode, float dt) {
   const int64_t n = s->n_total;
   FSIM_CK(s, cudaMemsetAsync(s->d_cnt + 3, 0, sizeof(int64_t), s->stream));
@@ -539,14 +668,8 @@ int launch_keys_from_positions(fsim_sim* s, int mode, float dt) {
   if (mode == 1 && s->delete_in_sources) reg = regions_at(s, s->src_time);
   unsigned long long* k64 = nullptr;
   if (mode == 1 && s->composite_sort) {
-    if (n > s->cap64) {
-      for (int b = 0; b < 2; ++b) {
-        if (s->keys64[b]) cudaFree(s->keys64[b]);
-        s->keys64[b] = nullptr;
-        FSIM_CK(s, cudaMalloc(&s->keys64[b], size_t(std::max<int64_t>(n, 1)) * 8));
-      }
-      s->cap64 = n;
-    }
+    const int rc = ensure_keys64(s, n);
+    if (rc) return rc;
     k64 = reinterpret_cast<unsigned long long*>(s->keys64[1]);
   }
   FSIM_LAUNCH(s, "advect_keys", k_keys, nblk(n, 256), 256, 0, s->part[s->cur], s->cap_p,
@@ -583,21 +706,8 @@ int rebuild_topology(fsim_sim* s) {
     s->composite_sort = false;
     return rebuild_after_sort(s);
   }
-  // radix sort (stable)
-  size_t need = 0;
-  FSIM_CK(s, cub::DeviceRadixSort::SortPairs(nullptr, need, s->keys[1], s->keys[0], s->vals[1],
-                                             s->vals[0], n, 0, bits, s->stream));
-  if (need > s->sort_tmp_bytes) {
-    if (s->sort_tmp) cudaFree(s->sort_tmp);
-    s->sort_tmp = nullptr;
-    FSIM_CK(s, cudaMalloc(&s->sort_tmp, need));
-    s->sort_tmp_bytes = need;
-  }
-  if (n > 0) {
-    fsim::ProfScope ps(s, "radix_sort(cub)");
-    FSIM_CK(s, cub::DeviceRadixSort::SortPairs(s->sort_tmp, need, s->keys[1], s->keys[0],
-                                               s->vals[1], s->vals[0], n, 0, bits, s->stream));
-  }
+  const int rc = sort_pairs(s, s->keys[1], s->keys[0], s->vals[1], s->vals[0], n);
+  if (rc) return rc;
   return rebuild_after_sort(s);
 }
 

@@ -700,9 +700,5 @@ int run_cluster(fsim_sim* s, PcgArgs& a) {
     return FSIM_ERR_CUDA;
   }
   s->launches++;
-  FSIM_CK(s, cudaMemcpyAsync(s->h_sc, a.sc, sizeof(PcgScalars), cudaMemcpyDeviceToHost, s->stream));
-  lt.stop();
-  FSIM_CK(s, cudaStreamSynchronize(s->stream));
-  if (s->h_sc->bar_err) return fail(s, FSIM_ERR_TIMEOUT, "PCG: a cluster-loop wait gave up");
-  return FSIM_OK;
+  return end_one_launch(s, a, lt);
 }

@@ -1214,9 +1214,5 @@ int run_resident(fsim_sim* s, PcgArgs& a) {
     }
   }
   s->launches++;
-  FSIM_CK(s, cudaMemcpyAsync(s->h_sc, a.sc, sizeof(PcgScalars), cudaMemcpyDeviceToHost, s->stream));
-  lt.stop();
-  FSIM_CK(s, cudaStreamSynchronize(s->stream));
-  if (s->h_sc->bar_err) return fail(s, FSIM_ERR_TIMEOUT, "PCG: a resident-loop barrier gave up");
-  return FSIM_OK;
+  return end_one_launch(s, a, lt);
 }
