@@ -18,6 +18,7 @@
 // All arithmetic that the reference does in float is done with explicit
 // round-to-nearest intrinsics so that nvcc cannot contract it into FMAs.
 #include <cstring>
+#include <type_traits>
 
 #include "fsim_internal.cuh"
 
@@ -124,122 +125,198 @@ __host__ __device__ constexpr unsigned box_axis_mask(int D, int ax, unsigned m) 
   return r;
 }
 
-__global__ void __launch_bounds__(256) k_p2g_cells(const __grid_constant__ GridArgs a) {
-  __shared__ unsigned long long sv[3][kNodeBlock];
-  __shared__ unsigned long long sw[3][kNodeBlock];
-  __shared__ uint8_t touched[1024];
-  const int s = blockIdx.x;  // particle leaf
-  const int tid = threadIdx.x;
-  for (int v = tid; v < kNodeBlock; v += 256) {
-    sv[0][v] = 0ull; sv[1][v] = 0ull; sv[2][v] = 0ull;
-    sw[0][v] = 0ull; sw[1][v] = 0ull; sw[2][v] = 0ull;
-  }
-  for (int v = tid; v < 1024; v += 256) touched[v] = 0;
-  __syncthreads();
-  int org[3];
-  origin_of(a, s, org);
+// A term x of a node sum as two 32-bit integers, hi 2^27 + lo = round(x 2^32)
+// (the same integer as to_fix(x), ties included): hi = round(x 2^5) from the
+// low mantissa bits of x + 1.5 2^18, the rest of x exactly, lo = round(rest
+// 2^32).  |x| < kPieceMax; 18 terms of a node then keep both sums below 2^31.
+constexpr float kPieceMax = 65536.0f;
+__device__ __forceinline__ void to_pieces(float x, int& hi, int& lo) {
+  constexpr float kMagic = 393216.0f;  // 1.5 * 2^18: its last bit is 2^-5
+  const float t = __fadd_rn(x, kMagic);
+  hi = __float_as_int(t) - __float_as_int(kMagic);
+  lo = __float2int_rn(__fmul_rn(__fsub_rn(x, __fsub_rn(t, kMagic)), kFixScale));
+}
+
+// Node sums of one component of the CTA's cells, added into shared memory.
+// WIDE: 64-bit atomics (any |x| < 2^31); otherwise the two pieces of a term
+// are added by one 32-bit atomic each, which shared memory has in hardware
+// (its 64-bit addition is not one; with it the 256^3 dam break's pass took
+// 1,065 us, 707 with the pieces, 164 and 111 at 128^3, the same bits; what
+// bounds it now is issue, the 18 node sums of each particle first of all).
+// Returns whether a term was too large for the pieces.
+template <int D, bool WIDE>
+__device__ __forceinline__ bool splat_cell(const GridArgs& a, const uint2 rg, const int cl[3],
+                                           const int g[3], unsigned long long* sv,
+                                           unsigned long long* sw, uint8_t* touched) {
   const float* px = a.part;
   const int64_t cap = a.cap;
-  for (int c = tid; c < 512; c += 256) {
+  // box extents: 3 on the tangential axes, 2 on the normal axis D
+  constexpr int e0 = D == 0 ? 2 : 3, e1 = D == 1 ? 2 : 3, e2 = D == 2 ? 2 : 3;
+  float am[18], aw[18];
+#pragma unroll
+  for (int t = 0; t < 18; ++t) { am[t] = 0.f; aw[t] = 0.f; }
+  unsigned reach = 0u;  // box nodes some particle's 8-node stencil includes
+  for (uint32_t q = rg.x; q < rg.y; ++q) {
+    if (a.check_dead && a.keys[q] == kDeadKey) continue;
+    const float uD = px[(3 + D) * cap + q];
+    float w1[3][3];   // per-axis weights over the box positions
+    unsigned m1[3];   // per-axis reached positions
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) {
+      const float pa = px[ax * cap + q];
+      const float ga = float(g[ax]);
+      if (ax == D) {
+        const float x = __fsub_rn(pa, ga);
+        w1[ax][0] = __fsub_rn(1.0f, x); w1[ax][1] = x; w1[ax][2] = 0.f;
+        m1[ax] = 3u;
+      } else {
+        const float lo = __fadd_rn(ga, 0.5f);
+        if (pa < lo) {  // stencil starts one below the cell
+          const float f = __fsub_rn(pa, __fsub_rn(lo, 1.0f));
+          w1[ax][0] = __fsub_rn(1.0f, f); w1[ax][1] = f; w1[ax][2] = 0.f;
+          m1[ax] = 3u;
+        } else {
+          const float f = __fsub_rn(pa, lo);
+          w1[ax][0] = 0.f; w1[ax][1] = __fsub_rn(1.0f, f); w1[ax][2] = f;
+          m1[ax] = 6u;
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < e0; ++i) {
+#pragma unroll
+      for (int j = 0; j < e1; ++j) {
+        const float wij = __fmul_rn(w1[0][i], w1[1][j]);
+#pragma unroll
+        for (int k = 0; k < e2; ++k) {
+          const int t = (i * e1 + j) * e2 + k;
+          const float ww = __fmul_rn(wij, w1[2][k]);
+          am[t] = __fadd_rn(am[t], __fmul_rn(ww, uD));
+          aw[t] = __fadd_rn(aw[t], ww);
+        }
+      }
+    }
+    unsigned rp = box_axis_mask(D, D, 3u);  // every position on the normal axis
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) {
+      if (ax == D) continue;
+      rp &= m1[ax] == 3u ? box_axis_mask(D, ax, 3u) : box_axis_mask(D, ax, 6u);
+    }
+    reach |= rp;
+  }
+  // flush the reached box nodes (local coordinates -1..8)
+  const int b0 = cl[0] - (D == 0 ? 0 : 1), b1 = cl[1] - (D == 1 ? 0 : 1),
+            b2 = cl[2] - (D == 2 ? 0 : 1);
+  bool wide = false;
+#pragma unroll
+  for (int i = 0; i < e0; ++i) {
+#pragma unroll
+    for (int j = 0; j < e1; ++j) {
+#pragma unroll
+      for (int k = 0; k < e2; ++k) {
+        const int t = (i * e1 + j) * e2 + k;
+        if (!((reach >> t) & 1u)) continue;
+        const int o = node_index(b0 + i, b1 + j, b2 + k);
+        if (WIDE) {
+          atomicAdd(&sv[o], to_fix(am[t]));
+          atomicAdd(&sw[o], to_fix(aw[t]));
+        } else {
+          int hi, lo;
+          to_pieces(am[t], hi, lo);
+          wide = wide || !(fabsf(am[t]) < kPieceMax) || !(aw[t] < kPieceMax);
+          int* v = reinterpret_cast<int*>(sv);
+          atomicAdd(&v[o], hi);
+          atomicAdd(&v[kNodeBlock + o], lo);
+          to_pieces(aw[t], hi, lo);
+          int* w = reinterpret_cast<int*>(sw);
+          atomicAdd(&w[o], hi);
+          atomicAdd(&w[kNodeBlock + o], lo);
+        }
+        touched[o] = 1;
+      }
+    }
+  }
+  return wide;
+}
+
+template <int D, bool WIDE, int NT>
+__device__ __forceinline__ bool splat_leaf(const GridArgs& a, int s, const int org[3],
+                                           unsigned long long* sv, unsigned long long* sw,
+                                           uint8_t* touched) {
+  bool wide = false;
+  for (int c = threadIdx.x; c < 512; c += NT) {
     const int cl[3] = {c >> 6, (c >> 3) & 7, c & 7};
     const uint2 rg = a.cell_range[int64_t(s) * 512 + c];
     if (rg.x >= rg.y) continue;
     const int g[3] = {org[0] + cl[0], org[1] + cl[1], org[2] + cl[2]};
-#pragma unroll
-    for (int D = 0; D < 3; ++D) {
-      // box extents: 3 on the tangential axes, 2 on the normal axis D
-      constexpr int kE = 3;
-      const int e0 = D == 0 ? 2 : kE, e1 = D == 1 ? 2 : kE, e2 = D == 2 ? 2 : kE;
-      float am[18], aw[18];
-#pragma unroll
-      for (int t = 0; t < 18; ++t) { am[t] = 0.f; aw[t] = 0.f; }
-      unsigned reach = 0u;  // box nodes some particle's 8-node stencil includes
-      for (uint32_t q = rg.x; q < rg.y; ++q) {
-        if (a.check_dead && a.keys[q] == kDeadKey) continue;
-        const float uD = px[(3 + D) * cap + q];
-        float w1[3][3];   // per-axis weights over the box positions
-        unsigned m1[3];   // per-axis reached positions
-#pragma unroll
-        for (int ax = 0; ax < 3; ++ax) {
-          const float pa = px[ax * cap + q];
-          const float ga = float(g[ax]);
-          if (ax == D) {
-            const float x = __fsub_rn(pa, ga);
-            w1[ax][0] = __fsub_rn(1.0f, x); w1[ax][1] = x; w1[ax][2] = 0.f;
-            m1[ax] = 3u;
-          } else {
-            const float lo = __fadd_rn(ga, 0.5f);
-            if (pa < lo) {  // stencil starts one below the cell
-              const float f = __fsub_rn(pa, __fsub_rn(lo, 1.0f));
-              w1[ax][0] = __fsub_rn(1.0f, f); w1[ax][1] = f; w1[ax][2] = 0.f;
-              m1[ax] = 3u;
-            } else {
-              const float f = __fsub_rn(pa, lo);
-              w1[ax][0] = 0.f; w1[ax][1] = __fsub_rn(1.0f, f); w1[ax][2] = f;
-              m1[ax] = 6u;
-            }
-          }
-        }
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          if (i >= e0) continue;
-#pragma unroll
-          for (int j = 0; j < 3; ++j) {
-            if (j >= e1) continue;
-            const float wij = __fmul_rn(w1[0][i], w1[1][j]);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-              if (k >= e2) continue;
-              const int t = (i * e1 + j) * e2 + k;
-              const float ww = __fmul_rn(wij, w1[2][k]);
-              am[t] = __fadd_rn(am[t], __fmul_rn(ww, uD));
-              aw[t] = __fadd_rn(aw[t], ww);
-            }
-          }
-        }
-        unsigned rp = box_axis_mask(D, D, 3u);  // every position on the normal axis
-#pragma unroll
-        for (int ax = 0; ax < 3; ++ax) {
-          if (ax == D) continue;
-          rp &= m1[ax] == 3u ? box_axis_mask(D, ax, 3u) : box_axis_mask(D, ax, 6u);
-        }
-        reach |= rp;
-      }
-      // flush the reached box nodes (local coordinates -1..8)
-      const int b0 = cl[0] - (D == 0 ? 0 : 1), b1 = cl[1] - (D == 1 ? 0 : 1),
-                b2 = cl[2] - (D == 2 ? 0 : 1);
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        if (i >= e0) continue;
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          if (j >= e1) continue;
-#pragma unroll
-          for (int k = 0; k < 3; ++k) {
-            if (k >= e2) continue;
-            const int t = (i * e1 + j) * e2 + k;
-            if (!((reach >> t) & 1u)) continue;
-            const int o = node_index(b0 + i, b1 + j, b2 + k);
-            atomicAdd(&sv[D][o], to_fix(am[t]));
-            atomicAdd(&sw[D][o], to_fix(aw[t]));
-            touched[o] = 1;
-          }
-        }
-      }
-    }
+    wide = splat_cell<D, WIDE>(a, rg, cl, g, sv, sw, touched) || wide;
   }
+  return wide;
+}
+
+// ND = 3: one CTA per particle leaf takes the three components in turn.
+// ND = 1: a CTA per leaf and component (512 threads, a cell each; the touched
+// bits of the three CTAs are combined by atomics): launches of few leaves,
+// where a CTA's serial work is the kernel's time.
+template <int ND, int NT>
+__global__ void __launch_bounds__(NT) k_p2g_cells(const __grid_constant__ GridArgs a) {
+  __shared__ unsigned long long sv[ND][kNodeBlock];
+  __shared__ unsigned long long sw[ND][kNodeBlock];
+  __shared__ uint8_t touched[1024];
+  const int s = ND == 3 ? int(blockIdx.x) : int(blockIdx.x / 3u);  // particle leaf
+  const int tid = threadIdx.x;
+  const int d0 = ND == 3 ? 0 : int(blockIdx.x % 3u);
+  int org[3];
+  origin_of(a, s, org);
+  auto clear = [&]() {
+    for (int v = tid; v < kNodeBlock; v += NT) {
+#pragma unroll
+      for (int d = 0; d < ND; ++d) sv[d][v] = sw[d][v] = 0ull;
+    }
+  };
+  auto splat = [&](auto wide_tag) {
+    constexpr bool kWide = decltype(wide_tag)::value;
+    bool wide = false;
+    if (ND == 3 || d0 == 0) wide = splat_leaf<0, kWide, NT>(a, s, org, sv[0], sw[0], touched) || wide;
+    if (ND == 3 || d0 == 1)
+      wide = splat_leaf<1, kWide, NT>(a, s, org, sv[ND == 3 ? 1 : 0], sw[ND == 3 ? 1 : 0], touched) || wide;
+    if (ND == 3 || d0 == 2)
+      wide = splat_leaf<2, kWide, NT>(a, s, org, sv[ND == 3 ? 2 : 0], sw[ND == 3 ? 2 : 0], touched) || wide;
+    return wide;
+  };
+  clear();
+  for (int v = tid; v < 1024; v += NT) touched[v] = 0;
   __syncthreads();
+  const bool wide = __syncthreads_or(splat(std::false_type()));
+  if (wide) {  // a term of 65,536 or more: the same sums with 64-bit atomics
+    clear();
+    __syncthreads();
+    splat(std::true_type());
+    __syncthreads();
+  }
+  auto node = [&](const unsigned long long* sums, int v) {
+    if (wide) return sums[v];
+    const int* p = reinterpret_cast<const int*>(sums);
+    return static_cast<unsigned long long>(static_cast<long long>(p[v]) * (1ll << 27) +
+                                           p[kNodeBlock + v]);
+  };
   unsigned long long* out = a.p2g_nodes + int64_t(s) * 6 * kNodeBlock;
-  for (int v = tid; v < kNodeBlock; v += 256) {
+  for (int v = tid; v < kNodeBlock; v += NT) {
 #pragma unroll
-    for (int D = 0; D < 3; ++D) {
-      out[D * kNodeBlock + v] = sv[D][v];
-      out[(3 + D) * kNodeBlock + v] = sw[D][v];
+    for (int d = 0; d < ND; ++d) {
+      out[(d0 + d) * kNodeBlock + v] = node(sv[d], v);
+      out[(3 + d0 + d) * kNodeBlock + v] = node(sw[d], v);
     }
   }
-  for (int v = tid; v < 1024; v += 256) {
+  for (int v = tid; v < 1024; v += NT) {
     const unsigned bits = __ballot_sync(0xffffffffu, touched[v] != 0);
-    if ((tid & 31) == 0) a.p2g_touch[int64_t(s) * 32 + (v >> 5)] = bits;
+    if ((tid & 31) == 0) {
+      uint32_t* t = a.p2g_touch + int64_t(s) * 32 + (v >> 5);
+      if (ND == 3)
+        *t = bits;
+      else
+        atomicOr(t, bits);
+    }
   }
 }
 
@@ -842,6 +919,11 @@ GridArgs make_args(fsim_sim* s) {
 
 }  // namespace
 
+// P2G pass 1 runs by component below this many particle leaves per SM: 12
+// against 29 us at 24 leaves, 28 against 40 at 159, the same at 490, 783
+// against 707 at 8,320 (every component reads the positions again).
+constexpr int kP2gSplitLeaves = 2;
+
 int launch_p2g(fsim_sim* s, bool fused, float dt) {
   if (s->p2g_cap < s->cap_pleaf) {
     if (s->p2g_nodes) cudaFree(s->p2g_nodes);
@@ -869,7 +951,13 @@ int launch_p2g(fsim_sim* s, bool fused, float dt) {
   a.dt = dt;
   a.p2g_low = s->p2g_low;
   FSIM_CK(s, cudaMemsetAsync(s->p2g_low, 0, sizeof(uint32_t), s->stream));
-  FSIM_LAUNCH(s, fused ? "p2g_cells_fused" : "p2g_cells", k_p2g_cells, s->n_pleaf, 256, 0, a);
+  const char* cells = fused ? "p2g_cells_fused" : "p2g_cells";
+  if (s->n_pleaf < kP2gSplitLeaves * s->num_sms) {
+    FSIM_CK(s, cudaMemsetAsync(s->p2g_touch, 0, size_t(s->n_pleaf) * 32 * 4, s->stream));
+    FSIM_LAUNCH(s, cells, (k_p2g_cells<1, 512>), s->n_pleaf * 3, 512, 0, a);
+  } else {
+    FSIM_LAUNCH(s, cells, (k_p2g_cells<3, 256>), s->n_pleaf, 256, 0, a);
+  }
   const int lgrid = std::max(1, s->num_sms * 4);
   if (fused) {
     FSIM_LAUNCH(s, "p2g_fused", k_p2g_nodes<true>, s->n_gleaf, 256, 0, a);
