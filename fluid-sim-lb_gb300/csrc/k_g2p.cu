@@ -10,6 +10,8 @@
 // components from the source node the six ordered passes would copy from.
 // Each particle then interpolates v and dv (z, then y, then x lerps) and
 // writes vel = v + flip*((dv + vel) - v) and grid_velocity = v.
+#include <algorithm>
+
 #include "fsim_internal.cuh"
 
 namespace fsim {
@@ -29,6 +31,7 @@ struct G2PArgs {
   const uint32_t* vold_on;
   LeafMap lm;
   float flip;
+  int split;  // CTAs per leaf
 };
 
 __device__ __forceinline__ int side(int t) { return t < 0 ? -1 : (t > 7 ? 1 : 0); }
@@ -37,11 +40,12 @@ __device__ __forceinline__ float lerp_ref(float a, float b, float w) {
   return __fadd_rn(a, __fmul_rn(w, __fsub_rn(b, a)));
 }
 
+// The halo is staged as {v, dv} pairs, so that a stencil node is one 64-bit
+// shared load for both interpolations (their arithmetic is unchanged).
 __global__ void __launch_bounds__(256) k_g2p(const __grid_constant__ G2PArgs a) {
-  __shared__ float hv[3][1000];
-  __shared__ float hd[3][1000];
+  __shared__ float2 halo[3][1000];
   __shared__ int nb[27];
-  const int s = blockIdx.x;
+  const int s = int(blockIdx.x / unsigned(a.split));
   const int tid = threadIdx.x;
   if (tid < 27) nb[tid] = a.nbr[int64_t(s) * 27 + tid];
   int lx, ly, lz;
@@ -64,15 +68,15 @@ __global__ void __launch_bounds__(256) k_g2p(const __grid_constant__ G2PArgs a) 
         if ((a.vel_on[int64_t(ns) * 16 + (sv >> 5)] >> (sv & 31)) & 1u) v = a.vel[base];
         if ((a.vold_on[int64_t(ns) * 16 + (sv >> 5)] >> (sv & 31)) & 1u) d = a.vold[base];
       }
-      hv[D][h] = v;
-      hd[D][h] = d;
+      halo[D][h] = make_float2(v, d);
     }
   }
   __syncthreads();
   const uint2 lr = a.leaf_range[s];
   const int64_t cap = a.cap;
   float* P = a.part;
-  for (uint32_t q = lr.x + tid; q < lr.y; q += 256) {
+  for (uint32_t q = lr.x + (blockIdx.x % unsigned(a.split)) * 256u + tid; q < lr.y;
+       q += 256u * unsigned(a.split)) {
     const uint32_t key = a.keys[q];
     if (key == kDeadKey) continue;
     const float p[3] = {P[q], P[cap + q], P[2 * cap + q]};
@@ -94,17 +98,17 @@ __global__ void __launch_bounds__(256) k_g2p(const __grid_constant__ G2PArgs a) 
       const float w0 = __fsub_rn(p[0], lo[0]), w1 = __fsub_rn(p[1], lo[1]),
                   w2 = __fsub_rn(p[2], lo[2]);
       const int b = (st[0] * 10 + st[1]) * 10 + st[2];
-#pragma unroll
-      for (int f = 0; f < 2; ++f) {
-        const float* B = f == 0 ? hv[D] : hd[D];
-        const float v000 = B[b], v001 = B[b + 1], v010 = B[b + 10], v011 = B[b + 11];
-        const float v100 = B[b + 100], v101 = B[b + 101], v110 = B[b + 110], v111 = B[b + 111];
-        const float v00 = lerp_ref(v000, v001, w2), v01 = lerp_ref(v010, v011, w2);
-        const float v10 = lerp_ref(v100, v101, w2), v11 = lerp_ref(v110, v111, w2);
-        const float v0 = lerp_ref(v00, v01, w1), v1 = lerp_ref(v10, v11, w1);
-        const float r = lerp_ref(v0, v1, w0);
-        if (f == 0) vi[D] = r; else di[D] = r;
-      }
+      const float2* B = halo[D] + b;
+      const float2 v000 = B[0], v001 = B[1], v010 = B[10], v011 = B[11];
+      const float2 v100 = B[100], v101 = B[101], v110 = B[110], v111 = B[111];
+      auto tri = [&](float c000, float c001, float c010, float c011, float c100, float c101,
+                     float c110, float c111) {
+        const float v00 = lerp_ref(c000, c001, w2), v01 = lerp_ref(c010, c011, w2);
+        const float v10 = lerp_ref(c100, c101, w2), v11 = lerp_ref(c110, c111, w2);
+        return lerp_ref(lerp_ref(v00, v01, w1), lerp_ref(v10, v11, w1), w0);
+      };
+      vi[D] = tri(v000.x, v001.x, v010.x, v011.x, v100.x, v101.x, v110.x, v111.x);
+      di[D] = tri(v000.y, v001.y, v010.y, v011.y, v100.y, v101.y, v110.y, v111.y);
     }
 #pragma unroll
     for (int D = 0; D < 3; ++D) {
@@ -131,7 +135,12 @@ int launch_g2p(fsim_sim* s) {
   a.vold_on = s->vold_on;
   a.lm = s->lm;
   a.flip = s->cfg.flip_factor;
-  FSIM_LAUNCH(s, "g2p", k_g2p, s->n_pleaf, 256, 0, a);
+  // few leaves: several CTAs per leaf, each with its share of the particles
+  // (and a copy of the halo), up to about six CTAs per SM in all: a CTA's
+  // passes over its 2,000 to 4,000 particles are the kernel's time there
+  // (24 leaves: 26 us with one CTA each, 16 with eight; 159: 30 and 24)
+  a.split = std::max(1, std::min(8, 6 * s->num_sms / std::max(s->n_pleaf, 1)));
+  FSIM_LAUNCH(s, "g2p", k_g2p, s->n_pleaf * a.split, 256, 0, a);
   return FSIM_OK;
 }
 

@@ -335,101 +335,135 @@ constexpr float kLowWeight = 1e-3f;
 // in list order into its halo buffer (:853-868), and the buffers are added
 // into the grid leaf by leaf (:870-890).  Leaves of slot s's neighbourhood
 // only: a node of slot s is reached from cells within one cell of it.
-__device__ __noinline__ void ref_node_sums(const GridArgs& a, const int* nb, int s, int D,
-                                           const int g[3], float& tm, float& tw) {
+// The whole warp takes one node: a lane per cell first (at most 18, in
+// visiting order), then a lane per particle forms the terms, and only the
+// float additions run in sequence.
+__device__ __forceinline__ void ref_node_sums(const GridArgs& a, const int* nb, int s, int D,
+                                              const int g[3], uint4* cells, float& tm, float& tw) {
+  const int lane = threadIdx.x & 31;
   int sl[3];
   leaf_coords(a.lm, uint32_t(a.leaf_id[s]), sl[0], sl[1], sl[2]);
-  // cells that reach node g: c_D in {g_D - 1, g_D}, the others in g +- 1
-  int clo[3], chi[3], llo[3], lhi[3];
+  // cells that reach node g: c_D in {g_D - 1, g_D}, the others in g +- 1;
+  // lane L < 18 takes one of them
+  int c[3], leaf[3];
+  {
+    int r = lane;
 #pragma unroll
-  for (int ax = 0; ax < 3; ++ax) {
-    clo[ax] = g[ax] - 1;
-    chi[ax] = ax == D ? g[ax] : g[ax] + 1;
-    llo[ax] = fdiv(clo[ax], 8);
-    lhi[ax] = fdiv(chi[ax], 8);
+    for (int ax = 2; ax >= 0; --ax) {
+      const int e = ax == D ? 2 : 3;
+      c[ax] = g[ax] - 1 + r % e;
+      r /= e;
+      leaf[ax] = fdiv(c[ax], 8);
+    }
   }
-  // candidate leaves in OpenVDB order (at most 8)
-  uint32_t lid[8];
-  int lslot[8], lc[8][3], nl = 0;
-  for (int lx = llo[0]; lx <= lhi[0]; ++lx)
-    for (int ly = llo[1]; ly <= lhi[1]; ++ly)
-      for (int lz = llo[2]; lz <= lhi[2]; ++lz) {
-        const int dx = lx - sl[0], dy = ly - sl[1], dz = lz - sl[2];
-        if (dx < -1 || dx > 1 || dy < -1 || dy > 1 || dz < -1 || dz > 1) continue;
-        const int ns = nb[nb_index(dx, dy, dz)];
-        if (ns < 0 || ns >= a.n_pleaf) continue;  // no particles there
-        const uint32_t id = uint32_t(a.leaf_id[ns]);
-        int q = nl++;
-        while (q > 0 && lid[q - 1] > id) {  // insertion sort by leaf id
-          lid[q] = lid[q - 1];
-          lslot[q] = lslot[q - 1];
-          lc[q][0] = lc[q - 1][0]; lc[q][1] = lc[q - 1][1]; lc[q][2] = lc[q - 1][2];
-          --q;
-        }
-        lid[q] = id;
-        lslot[q] = ns;
-        lc[q][0] = lx; lc[q][1] = ly; lc[q][2] = lz;
+  uint2 rg = make_uint2(0u, 0u);
+  uint32_t id = 0xFFFFFFFFu;  // no particles there
+  if (lane < 18) {
+    const int dx = leaf[0] - sl[0], dy = leaf[1] - sl[1], dz = leaf[2] - sl[2];
+    if (dx >= -1 && dx <= 1 && dy >= -1 && dy <= 1 && dz >= -1 && dz <= 1) {
+      const int ns = nb[nb_index(dx, dy, dz)];
+      if (ns >= 0 && ns < a.n_pleaf) {
+        rg = a.cell_range[int64_t(ns) * 512 + (((c[0] & 7) << 6) | ((c[1] & 7) << 3) | (c[2] & 7))];
+        if (rg.y > rg.x) id = uint32_t(a.leaf_id[ns]);
       }
+    }
+  }
+  // the cells in visiting order (leaf by leaf in OpenVDB order, within a leaf
+  // as the lanes have them), and the particles before each
+  int rank = lane < 18 ? 0 : lane;
+  for (int l = 0; l < 18; ++l) {
+    const uint32_t oid = __shfl_sync(0xffffffffu, id, l);
+    if (lane < 18 && (oid < id || (oid == id && l < lane))) ++rank;
+  }
+  __syncwarp();  // the previous node's reads of the cells
+  cells[rank] = make_uint4(rg.x, id == 0xFFFFFFFFu ? 0u : rg.y - rg.x, id,
+                           uint32_t((c[0] - g[0] + 1) | ((c[1] - g[1] + 1) << 2) |
+                                    ((c[2] - g[2] + 1) << 4)));
+  __syncwarp();
+  const int np = lane < 18 ? int(cells[lane].y) : 0;
+  int upto = np;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, upto, o);
+    if (lane >= o) upto += t;
+  }
+  const int total = __shfl_sync(0xffffffffu, upto, 31);
+  const int before = upto - np;
   const float* px = a.part;
   const int64_t cap = a.cap;
-  float Tm = 0.f, Tw = 0.f;
-  for (int l = 0; l < nl; ++l) {
-    float Bm = 0.f, Bw = 0.f;
-    bool touched = false;
-    const int x0 = max(clo[0], lc[l][0] * 8), x1 = min(chi[0], lc[l][0] * 8 + 7);
-    const int y0 = max(clo[1], lc[l][1] * 8), y1 = min(chi[1], lc[l][1] * 8 + 7);
-    const int z0 = max(clo[2], lc[l][2] * 8), z1 = min(chi[2], lc[l][2] * 8 + 7);
-    for (int cx = x0; cx <= x1; ++cx)
-      for (int cy = y0; cy <= y1; ++cy)
-        for (int cz = z0; cz <= z1; ++cz) {
-          const int v = ((cx & 7) << 6) | ((cy & 7) << 3) | (cz & 7);
-          const uint2 rg = a.cell_range[int64_t(lslot[l]) * 512 + v];
-          const int c[3] = {cx, cy, cz};
-          for (uint32_t q = rg.x; q < rg.y; ++q) {
-            if (a.check_dead && a.keys[q] == kDeadKey) continue;
-            float f[3];
-            int corner[3];
-            bool reach = true;
+  float Tm = 0.f, Tw = 0.f, Bm = 0.f, Bw = 0.f;
+  uint32_t cur = 0xFFFFFFFFu;  // leaf being summed into Bm, Bw
+  bool touched = false;
+  for (int p0 = 0; p0 < total; p0 += 32) {
+    // the lane's particle, number p0 + lane: in the last cell that starts at or before it
+    const int mine = p0 + lane;
+    int cell = 0;
 #pragma unroll
-            for (int ax = 0; ax < 3; ++ax) {
-              const float pa = px[ax * cap + q];
-              float lo = float(c[ax]);
-              int st = c[ax];
-              if (ax != D) {
-                lo = __fadd_rn(lo, 0.5f);
-                if (pa < lo) { lo = __fsub_rn(lo, 1.0f); st -= 1; }
-              }
-              f[ax] = __fsub_rn(pa, lo);
-              corner[ax] = g[ax] - st;
-              reach = reach && (corner[ax] == 0 || corner[ax] == 1);
-            }
-            if (!reach) continue;
-            touched = true;
-            const float x = f[0], y = f[1], z = f[2];
-            const float xy = __fmul_rn(x, y), yz = __fmul_rn(y, z), xz = __fmul_rn(z, x);
-            const float xyz = __fmul_rn(xy, z);
-            const float w110 = __fsub_rn(xy, xyz), w101 = __fsub_rn(xz, xyz);
-            const float w001 = __fsub_rn(__fsub_rn(z, yz), w101);
-            const int k = (corner[0] << 2) | (corner[1] << 1) | corner[2];
-            float w;
-            switch (k) {
-              case 7: w = xyz; break;
-              case 6: w = w110; break;
-              case 5: w = w101; break;
-              case 4: w = __fsub_rn(__fsub_rn(x, xz), w110); break;
-              case 3: w = __fsub_rn(yz, xyz); break;
-              case 2: w = __fsub_rn(__fsub_rn(y, yz), w110); break;
-              case 1: w = w001; break;
-              default: w = __fsub_rn(__fadd_rn(__fsub_rn(__fsub_rn(1.0f, x), y), xy), w001);
-            }
-            Bm = __fadd_rn(Bm, __fmul_rn(w, px[(3 + D) * cap + q]));
-            Bw = __fadd_rn(Bw, w);
-          }
-        }
-    if (touched) {
-      Tm = __fadd_rn(Tm, Bm);
-      Tw = __fadd_rn(Tw, Bw);
+    for (int o = 16; o > 0; o >>= 1) {
+      const int b = __shfl_sync(0xffffffffu, before, min(cell + o, 31));
+      if (cell + o < 18 && b <= mine) cell += o;
     }
+    const int start = __shfl_sync(0xffffffffu, before, cell);
+    const uint4 ce = cells[cell];
+    const uint32_t q = ce.x + uint32_t(mine - start), pid = ce.z;
+    const int pc[3] = {g[0] - 1 + int(ce.w & 3u), g[1] - 1 + int((ce.w >> 2) & 3u),
+                       g[2] - 1 + int((ce.w >> 4) & 3u)};
+    bool reach = mine < total && !(a.check_dead && a.keys[q] == kDeadKey);
+    float wu = 0.f, w = 0.f;
+    if (reach) {
+      float f[3];
+      int corner[3];
+#pragma unroll
+      for (int ax = 0; ax < 3; ++ax) {
+        const float pa = px[ax * cap + q];
+        float lo = float(pc[ax]);
+        int st = pc[ax];
+        if (ax != D) {
+          lo = __fadd_rn(lo, 0.5f);
+          if (pa < lo) { lo = __fsub_rn(lo, 1.0f); st -= 1; }
+        }
+        f[ax] = __fsub_rn(pa, lo);
+        corner[ax] = g[ax] - st;
+        reach = reach && (corner[ax] == 0 || corner[ax] == 1);
+      }
+      const float x = f[0], y = f[1], z = f[2];
+      const float xy = __fmul_rn(x, y), yz = __fmul_rn(y, z), xz = __fmul_rn(z, x);
+      const float xyz = __fmul_rn(xy, z);
+      const float w110 = __fsub_rn(xy, xyz), w101 = __fsub_rn(xz, xyz);
+      const float w001 = __fsub_rn(__fsub_rn(z, yz), w101);
+      switch ((corner[0] << 2) | (corner[1] << 1) | corner[2]) {
+        case 7: w = xyz; break;
+        case 6: w = w110; break;
+        case 5: w = w101; break;
+        case 4: w = __fsub_rn(__fsub_rn(x, xz), w110); break;
+        case 3: w = __fsub_rn(yz, xyz); break;
+        case 2: w = __fsub_rn(__fsub_rn(y, yz), w110); break;
+        case 1: w = w001; break;
+        default: w = __fsub_rn(__fadd_rn(__fsub_rn(__fsub_rn(1.0f, x), y), xy), w001);
+      }
+      wu = __fmul_rn(w, px[(3 + D) * cap + q]);
+    }
+    // the additions, in order (every lane alike)
+    for (unsigned todo = __ballot_sync(0xffffffffu, reach); todo != 0u; todo &= todo - 1u) {
+      const int l = __ffs(int(todo)) - 1;
+      const uint32_t lid = __shfl_sync(0xffffffffu, pid, l);
+      const float am = __shfl_sync(0xffffffffu, wu, l), aw = __shfl_sync(0xffffffffu, w, l);
+      if (lid != cur) {
+        if (touched) {
+          Tm = __fadd_rn(Tm, Bm);
+          Tw = __fadd_rn(Tw, Bw);
+        }
+        cur = lid;
+        touched = true;
+        Bm = Bw = 0.f;
+      }
+      Bm = __fadd_rn(Bm, am);
+      Bw = __fadd_rn(Bw, aw);
+    }
+  }
+  if (touched) {
+    Tm = __fadd_rn(Tm, Bm);
+    Tw = __fadd_rn(Tw, Bw);
   }
   tm = Tm;
   tw = Tw;
@@ -552,18 +586,25 @@ __global__ void __launch_bounds__(256) k_p2g_nodes(const __grid_constant__ GridA
 // The low-weight faces pass 2 listed: the reference's float sums
 // (ref_node_sums), normalisation with the 1e-5 cut, and for the fused step
 // the rest of pass 2's per-face work (BC, SaveGridVelocities, AddGravity,
-// BC).  The faces are independent, so the list's order does not matter.
+// BC), one warp per face.  The faces are independent, so the list's order does
+// not matter.  A thread per face walked up to 18 cells' particles one after
+// the other, a latency chain: 25 us at 32^3, 33 at 64^3, 38 at 128^3 (few
+// listed faces) against 10, 14 and 23 with a warp; on the 256^3 dam break,
+// whose list fills the GPU, 101 against 137.
 template <bool FUSED>
 __global__ void __launch_bounds__(128) k_p2g_low(const __grid_constant__ GridArgs a) {
+  __shared__ uint4 cells[4][32];  // per warp: a node's cells in visiting order
   const unsigned n = *a.p2g_low;
-  for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+  const unsigned lane = threadIdx.x & 31u, wpb = blockDim.x / 32u;
+  for (unsigned e = blockIdx.x * wpb + (threadIdx.x >> 5); e < n; e += gridDim.x * wpb) {
     const unsigned code = a.p2g_low[1 + e];
     const int s = int(code / 1536u), D = int((code % 1536u) >> 9), v = int(code & 511u);
     int org[3];
     origin_of(a, s, org);
     const int g[3] = {org[0] + (v >> 6), org[1] + ((v >> 3) & 7), org[2] + (v & 7)};
     float ms, ws;
-    ref_node_sums(a, a.nbr + int64_t(s) * 27, s, D, g, ms, ws);
+    ref_node_sums(a, a.nbr + int64_t(s) * 27, s, D, g, cells[threadIdx.x >> 5], ms, ws);
+    if (lane != 0u) continue;
     const float val = (ws <= 1e-5f) ? 0.f : __fdiv_rn(ms, ws);
     const int64_t o = int64_t(s) * 1536 + D * 512 + v;
     if (FUSED) {
@@ -958,7 +999,7 @@ int launch_p2g(fsim_sim* s, bool fused, float dt) {
   } else {
     FSIM_LAUNCH(s, cells, (k_p2g_cells<3, 256>), s->n_pleaf, 256, 0, a);
   }
-  const int lgrid = std::max(1, s->num_sms * 4);
+  const int lgrid = std::max(1, s->num_sms * 12);
   if (fused) {
     FSIM_LAUNCH(s, "p2g_fused", k_p2g_nodes<true>, s->n_gleaf, 256, 0, a);
     FSIM_LAUNCH(s, "p2g_low_fused", k_p2g_low<true>, lgrid, 128, 0, a);
