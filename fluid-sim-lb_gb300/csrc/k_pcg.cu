@@ -304,6 +304,7 @@ struct PcgArgs {
   int init_r;       // setup: 1 -> r = b (x0 = 0); 0 -> r already holds the rhs
   int par;          // spmv / update: parity of the iteration this launch serves
   int withhold;     // bulk-copy spmv, test only: CTA 0's first stage withholds its flags copy
+  int down;         // update: a warp takes its half leaves last to first
   int res_withhold; // resident loop, test only: CTA 0 skips its first barrier arrival
   cudaGraphConditionalHandle cond;  // WHILE-node handle when run as a graph, else 0
   void* w[2];       // single-reduction CG: w = A M r (by parity), or null
@@ -553,6 +554,10 @@ __device__ __forceinline__ HalfLeaf half_pos(int hw, int lane) {
   h.ty = h.lx == 1 ? (h.cy < 4 ? 0 : 9) : h.cy + 1;
   return h;
 }
+// The last half leaf of a warp whose first one is hw0 (-1: it has none).
+__device__ __forceinline__ int last_half(int hw0, int nhw, int hstride) {
+  return hw0 < nhw ? hw0 + (nhw - 1 - hw0) / hstride * hstride : -1;
+}
 // The lane's halo column: leaf slot (-1: none) and first voxel.
 __device__ __forceinline__ void halo_col(const HalfLeaf& h, const int fs[6], int& hslot,
                                          int& hvox) {
@@ -630,10 +635,23 @@ __device__ __forceinline__ void ld_col_sh(const Tile<T>& t, int x, int y, Col<T>
   }
 }
 
+// A column whose eight cells are FLUID with six non-solid neighbours: diag 6
+// and its inverse are constants then (the table's values), and no cell is
+// off-fluid.  Four fifths of the 256^3 dam break's half leaves are all such
+// columns; where a whole warp's are, the pipelined kernels skip the flags' byte
+// extraction, the table reads and the off-fluid selects.  Per iteration, FP32
+// and MIXED: 33.0 -> 31.9 and 36.2 -> 34.6 us at 256^3 (8,320 leaves), 119.7
+// -> 118.2 and 129.9 -> 128.0 at 512^3 (35,312).  The same branch in the
+// resident loop gave 0-2% at 192^3 and above and lost up to 3% below.
+__device__ __forceinline__ bool inner_col(uint2 f) {
+  return f.x == 0x0D0D0D0Du && f.y == 0x0D0D0D0Du;
+}
+constexpr uint8_t kInnerFlags = 13;  // FLUID, diag 6
+
 // A p on the lane's column, summed in the reference's column order
 // (-x,-y,-z, diag, +z,+y,+x); 0 off-fluid.  The four x/y neighbour columns
 // come from the tile; zm / zp are the -z / +z face cells.
-template <typename T>
+template <typename T, bool INNER = false>
 __device__ __forceinline__ void stencil_col(const Tile<T>& t, const DiagInv<T>* tab, int lx,
                                             int cy, const Col<T>& P, uint2 f, T zm, T zp,
                                             Col<T>& out) {
@@ -650,20 +668,20 @@ __device__ __forceinline__ void stencil_col(const Tile<T>& t, const DiagInv<T>* 
     acc = tsub(acc, xm.v[z]);
     acc = tsub(acc, ym.v[z]);
     acc = tsub(acc, vzm);
-    acc = tadd(acc, tmul(tab[g & 15].d, P.v[z]));
+    acc = tadd(acc, tmul(INNER ? T(6) : tab[g & 15].d, P.v[z]));
     acc = tsub(acc, vzp);
     acc = tsub(acc, yp.v[z]);
     acc = tsub(acc, xp.v[z]);
-    out.v[z] = (g & 1) ? acc : T(0);
+    out.v[z] = INNER || (g & 1) ? acc : T(0);
   }
 }
 
 // p = z + beta p_old with z = r/diag.  Off-fluid both terms are 0 (the
 // table's inverse is 0 there and r, p are stored 0), and at the first
 // iteration beta = 0 and p_old was zeroed by the setup, so no select is needed.
-template <typename T>
+template <typename T, bool INNER = false>
 __device__ __forceinline__ T pnew_of(const DiagInv<T>* tab, uint8_t f, T r, T po, T beta) {
-  return tadd(tmul(tab[f & 15].inv, r), tmul(beta, po));
+  return tadd(tmul(INNER ? T(1.0 / 6.0) : tab[f & 15].inv, r), tmul(beta, po));
 }
 
 // Programmatic dependent launch (the graph's edges are of programmatic type
@@ -1223,29 +1241,38 @@ __global__ void __launch_bounds__(kHotThreads, 4) k_pcg_spmv_pl(const __grid_con
       nbl = hn + hstride < nhw ? face_slot_lane(a.nbr, (hn + hstride) >> 1, lane) : -1;
     }
     const HalfLeaf h = half_pos(hw, lane);
-    Col<T> P, H;
+    auto body = [&](auto tag) {
+      constexpr bool kIn = decltype(tag)::value;
+      Col<T> P, H;
 #pragma unroll
-    for (int z = 0; z < 8; ++z) {
-      P.v[z] = pnew_of<T>(tab, fbyte(cur.f, z), cur.rc.v[z], cur.pc.v[z], beta);
-      H.v[z] = pnew_of<T>(tab, fbyte(cur.hf, z), cur.hr.v[z], cur.hp.v[z], beta);
-    }
-    const T zm = pnew_of<T>(tab, cur.zf0, cur.zr0, cur.zq0, beta);
-    const T zp = pnew_of<T>(tab, cur.zf1, cur.zr1, cur.zq1, beta);
-    const unsigned o = unsigned(h.s) * 512u + unsigned(h.c);
-    stcol(pnew, o, P);
-    if constexpr (!ZD) {  // publish the z faces for the neighbours
-      T* zw = static_cast<T*>(a.zf) + (unsigned(h.s) * 384u + 128u * unsigned(qnew) + unsigned(h.fidx));
-      zw[0] = P.v[0];
-      zw[64] = P.v[7];
-    }
-    __syncwarp();
-    st_col_sh(tile, h.lx + 1, h.cy + 1, P);
-    if (h.lx != 2) st_col_sh(tile, h.tx, h.ty, H);
-    __syncwarp();
-    Col<T> ap;
-    stencil_col<T>(tile, tab, h.lx, h.cy, P, cur.f, zm, zp, ap);
+      for (int z = 0; z < 8; ++z) {
+        P.v[z] = pnew_of<T, kIn>(tab, fbyte(cur.f, z), cur.rc.v[z], cur.pc.v[z], beta);
+        H.v[z] = pnew_of<T, kIn>(tab, fbyte(cur.hf, z), cur.hr.v[z], cur.hp.v[z], beta);
+      }
+      const T zm = pnew_of<T, kIn>(tab, cur.zf0, cur.zr0, cur.zq0, beta);
+      const T zp = pnew_of<T, kIn>(tab, cur.zf1, cur.zr1, cur.zq1, beta);
+      const unsigned o = unsigned(h.s) * 512u + unsigned(h.c);
+      stcol(pnew, o, P);
+      if constexpr (!ZD) {  // publish the z faces for the neighbours
+        T* zw = static_cast<T*>(a.zf) + (unsigned(h.s) * 384u + 128u * unsigned(qnew) + unsigned(h.fidx));
+        zw[0] = P.v[0];
+        zw[64] = P.v[7];
+      }
+      __syncwarp();
+      st_col_sh(tile, h.lx + 1, h.cy + 1, P);
+      if (h.lx != 2) st_col_sh(tile, h.tx, h.ty, H);
+      __syncwarp();
+      Col<T> ap;
+      stencil_col<T, kIn>(tile, tab, h.lx, h.cy, P, cur.f, zm, zp, ap);
 #pragma unroll
-    for (int z = 0; z < 8; ++z) dp.add(P.v[z], ap.v[z]);
+      for (int z = 0; z < 8; ++z) dp.add(P.v[z], ap.v[z]);
+    };
+    const bool in = inner_col(cur.f) && (h.lx == 2 || inner_col(cur.hf)) &&
+                    cur.zf0 == kInnerFlags && cur.zf1 == kInnerFlags;
+    if (__all_sync(0xffffffffu, in))
+      body(std::true_type());
+    else
+      body(std::false_type());
     cur = nxt;
     hw = hn;
   }
@@ -1537,27 +1564,29 @@ __global__ void __launch_bounds__(kHotThreads, 4)
   const int qcur = 1 + par;
   const int lane = threadIdx.x & 31;
   const int wpb = kHotThreads / 32;
-  const int nhw = 2 * a.n_pleaf, hstride = gridDim.x * wpb;
-  int hw = blockIdx.x * wpb + (threadIdx.x >> 5);
+  const int nhw = 2 * a.n_pleaf, hw0 = blockIdx.x * wpb + int(threadIdx.x >> 5);
+  const int step = (a.down ? -1 : 1) * int(gridDim.x) * wpb;
+  auto has = [nhw](int hw) { return unsigned(hw) < unsigned(nhw); };
+  int hw = a.down ? last_half(hw0, nhw, -step) : hw0;
   fill_diag_table<T>(tab);
   UpdIn<T> cur;
   int nbl = -1;
   int fs[6];
   // before the wait: the neighbour table, flags, x and r (written by the
   // update two launches back) of the first half leaf
-  if (hw < nhw) {
+  if (has(hw)) {
     const int nb0 = face_slot_lane(a.nbr, hw >> 1, lane);
     const HalfLeaf h = half_pos(hw, lane);
     const unsigned o = unsigned(h.s) * 512u + unsigned(h.c);
     cur.f = ldflags(a.flags, o);
     ldcol(x, o, cur.x);
     ldcol(r, o, cur.r);
-    nbl = hw + hstride < nhw ? face_slot_lane(a.nbr, (hw + hstride) >> 1, lane) : -1;
+    nbl = has(hw + step) ? face_slot_lane(a.nbr, (hw + step) >> 1, lane) : -1;
     face_slots(nb0, fs);
   }
   pdl_wait();
   pdl_trigger();
-  if (hw < nhw) {
+  if (has(hw)) {
     const HalfLeaf h = half_pos(hw, lane);
     ldcol(p, unsigned(h.s) * 512u + unsigned(h.c), cur.P);
     upd_load_halo<T, ZD>(a, hw, lane, fs, p, qcur, cur);
@@ -1569,30 +1598,37 @@ __global__ void __launch_bounds__(kHotThreads, 4)
   const T nalpha = -alpha;
   Tile<T>& tile = tiles[threadIdx.x >> 5];
   Dot<DM> drr, drz;
-  while (hw < nhw) {
-    const int hn = hw + hstride;
+  while (has(hw)) {
+    const int hn = hw + step;
     UpdIn<T> nxt;
-    if (hn < nhw) {
+    if (has(hn)) {
       int fs[6];
       face_slots(nbl, fs);
       upd_load<T, ZD>(a, hn, lane, fs, p, x, r, qcur, nxt);
-      nbl = hn + hstride < nhw ? face_slot_lane(a.nbr, (hn + hstride) >> 1, lane) : -1;
+      nbl = has(hn + step) ? face_slot_lane(a.nbr, (hn + step) >> 1, lane) : -1;
     }
     const HalfLeaf h = half_pos(hw, lane);
     __syncwarp();
     st_col_sh(tile, h.lx + 1, h.cy + 1, cur.P);
     if (h.lx != 2) st_col_sh(tile, h.tx, h.ty, cur.H);
     __syncwarp();
-    Col<T> ap;
-    stencil_col<T>(tile, tab, h.lx, h.cy, cur.P, cur.f, cur.zm, cur.zp, ap);
+    auto body = [&](auto tag) {
+      constexpr bool kIn = decltype(tag)::value;
+      Col<T> ap;
+      stencil_col<T, kIn>(tile, tab, h.lx, h.cy, cur.P, cur.f, cur.zm, cur.zp, ap);
 #pragma unroll
-    for (int z = 0; z < 8; ++z) {
-      const uint8_t g = fbyte(cur.f, z);
-      cur.x.v[z] = tadd(tmul(alpha, cur.P.v[z]), cur.x.v[z]);
-      cur.r.v[z] = tadd(tmul(nalpha, ap.v[z]), cur.r.v[z]);
-      drr.add(cur.r.v[z], cur.r.v[z]);
-      drz.add(cur.r.v[z], tmul(tab[g & 15].inv, cur.r.v[z]));
-    }
+      for (int z = 0; z < 8; ++z) {
+        const uint8_t g = fbyte(cur.f, z);
+        cur.x.v[z] = tadd(tmul(alpha, cur.P.v[z]), cur.x.v[z]);
+        cur.r.v[z] = tadd(tmul(nalpha, ap.v[z]), cur.r.v[z]);
+        drr.add(cur.r.v[z], cur.r.v[z]);
+        drz.add(cur.r.v[z], tmul(kIn ? T(1.0 / 6.0) : tab[g & 15].inv, cur.r.v[z]));
+      }
+    };
+    if (__all_sync(0xffffffffu, inner_col(cur.f)))
+      body(std::true_type());
+    else
+      body(std::false_type());
     const unsigned o = unsigned(h.s) * 512u + unsigned(h.c);
     stcol(x, o, cur.x);
     stcol(r, o, cur.r);
@@ -2469,6 +2505,11 @@ int pcg_solve(fsim_sim* s, const fsim_pcg_params* prm, fsim_pcg_stats* st, const
   a.x64 = s->x64;
   a.dinner = s->pres;
   a.init_r = 1;
+  // Once the vectors exceed L2, the update starts on the half leaves that the
+  // spmv has just left there, and the next spmv on the update's: 512^3 FP32
+  // 118.2 -> 116.2 us per iteration, MIXED 128.0 -> 124.1.  While they fit it
+  // only costs (256^3: 31.9 -> 32.4 and 34.6 -> 35.4).
+  a.down = a.n_pleaf > kZDirectLeaves;
   a.withhold = s->tma_withhold;
   s->tma_withhold = 0;  // a test's withheld copy applies to one solve
   a.res_withhold = s->res_withhold;
