@@ -386,7 +386,7 @@ def host_link_floor(hp, stream, device, step_ms, kt, prof_steps):
     down = best_ms(lambda: flat.copy_(dbuf))
     del dbuf
     nbytes = flat.numel() * flat.element_size()
-    early = sum(kt[k][0] for k in ("advect_keys", "radix_sort(cub)") if k in kt) / prof_steps
+    early = sum(kt[k][0] for k in ("advect_keys", "bin_rows", "sort_leaves", "radix_sort(cub)") if k in kt) / prof_steps
     return {"link_h2d_gbs": nbytes / (up * 1e-3) / 1e9,
             "link_d2h_gbs": nbytes / (down * 1e-3) / 1e9,
             "link_floor_ms": e2e_floor_ms(up, down, step_ms, early)}

@@ -376,7 +376,11 @@ int fsim_create(const fsim_config* cfg, fsim_t** out) {
   const uint32_t D = s->lm.dense;
   if ((rc = dmalloc(s, &s->d_flag, D))) return bail(rc);
   if ((rc = dmalloc(s, &s->d_slot, D))) return bail(rc);
-  if ((rc = dmalloc(s, &s->d_scan, size_t(D) * 2))) return bail(rc);
+  if ((rc = dmalloc(s, &s->d_lcnt, D))) return bail(rc);
+  if ((rc = dmalloc(s, &s->d_lnext, D))) return bail(rc);
+  if ((rc = dmalloc(s, &s->d_tile, size_t(D) / 1024 + 1))) return bail(rc);
+  if (cudaEventCreateWithFlags(&s->ev_topo, cudaEventDisableTiming) != cudaSuccess)
+    return bail(FSIM_ERR_CUDA);
   if ((rc = dmalloc(s, &s->d_leaf_id, D))) return bail(rc);
   if ((rc = dmalloc(s, &s->d_cnt, 16))) return bail(rc);
   if ((rc = dmalloc(s, &s->d_sc, 1))) return bail(rc);
@@ -399,9 +403,10 @@ int fsim_destroy(fsim_t* s) {
   if (s->dev >= 0) cudaSetDevice(s->dev);
   if (s->stream) cudaStreamSynchronize(s->stream);
   for (int b = 0; b < 2; ++b) { dfree(s->part[b]); dfree(s->keys[b]); dfree(s->vals[b]); }
-  dfree(s->sort_tmp); dfree(s->scan_tmp); dfree(s->keys64[0]); dfree(s->keys64[1]);
+  dfree(s->sort_tmp); dfree(s->bins); dfree(s->keys64[0]); dfree(s->keys64[1]);
   if (s->src_tmp) cudaFree(s->src_tmp);
-  dfree(s->d_flag); dfree(s->d_slot); dfree(s->d_scan); dfree(s->d_leaf_id); dfree(s->d_nbr);
+  dfree(s->d_flag); dfree(s->d_slot); dfree(s->d_lcnt); dfree(s->d_lnext);
+  dfree(s->d_tile); dfree(s->d_leaf_id); dfree(s->d_nbr);
   dfree(s->d_cell_range); dfree(s->d_leaf_range);
   dfree(s->vel); dfree(s->vold); dfree(s->weight); dfree(s->vel_on); dfree(s->vold_on);
   dfree(s->marker); dfree(s->div); dfree(s->pres); dfree(s->r); dfree(s->p[0]); dfree(s->p[1]);
@@ -422,6 +427,7 @@ int fsim_destroy(fsim_t* s) {
   if (s->ev_main) cudaEventDestroy(s->ev_main);
   for (auto e : s->ev_loop)
     if (e) cudaEventDestroy(e);
+  if (s->ev_topo) cudaEventDestroy(s->ev_topo);
   if (s->ev_io) cudaEventDestroy(s->ev_io);
   dfree(s->io_stage);
   if (s->p2g_nodes) cudaFree(s->p2g_nodes);

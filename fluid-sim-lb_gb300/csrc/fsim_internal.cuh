@@ -230,13 +230,16 @@ struct fsim_sim {
   uint32_t* vals[2] = {nullptr, nullptr};
   void* sort_tmp = nullptr;
   size_t sort_tmp_bytes = 0;
+  void* bins = nullptr;  // the leaf sort's cells and old keys
+  size_t bin_bytes = 0;
 
   // topology
   uint8_t* d_flag = nullptr;     // dense
   int32_t* d_slot = nullptr;     // dense -> slot
-  uint64_t* d_scan = nullptr;    // dense scan buffer
-  void* scan_tmp = nullptr;
-  size_t scan_tmp_bytes = 0;
+  uint32_t* d_lcnt = nullptr;    // dense: particles with a key in the leaf
+  uint32_t* d_lnext = nullptr;   // dense: next place in the leaf's bin (its end after a sort)
+  uint4* d_tile = nullptr;       // totals per 1,024 leaves
+  cudaEvent_t ev_topo = nullptr; // the counts of a new topology have reached h_cnt
   int32_t* d_leaf_id = nullptr;  // slot -> dense id (capacity = dense)
   int32_t* d_nbr = nullptr;      // slot*27
   int64_t cap_leaf = 0;          // field capacity (slots)
@@ -376,9 +379,7 @@ struct ProfScope {
 int ensure_leaf_capacity(fsim_sim* s, int64_t n_gleaf, int64_t n_pleaf);
 // particle arrays for at least n particles (the current ones are kept)
 int grow_particle_capacity(fsim_sim* s, int64_t n);
-int rebuild_topology(fsim_sim* s);  // from keys[cur]/vals, n_total
-// the topology part, keys[0]/vals[0] sorted; gather: permute the particles by vals[0]
-int rebuild_after_sort(fsim_sim* s, bool gather = true);
+int rebuild_topology(fsim_sim* s);  // sorts and gathers by keys[1], counted in d_lcnt
 // upload: rebin the particles whose keys are in keys[1] (sort skipped when sorted)
 int rebin_uploaded(fsim_sim* s, int64_t* invalid);
 

@@ -4,11 +4,12 @@
 // 479-546) and DeleteParticlesInSolids (:202-219) as: one kernel that
 // advects every particle (pos += gvel*dt, IEEE round-to-nearest, no FMA
 // contraction), clamps it to [0,N] exactly as the reference does and emits
-// its cell key (dead key for particles in solids); a stable device radix sort
-// by key (this reproduces the reference's rebuilt cell lists, which keep
-// particles in visiting order); a gather of the 9 particle arrays; and the
-// leaf topology (particle leaves, one-leaf dilation, slots, 27-neighbour
-// table, per-cell particle ranges).
+// its cell key (dead key for particles in solids) and counts the leaves'
+// particles; the leaf topology from those counts (particle leaves, one-leaf
+// dilation, slots); a stable sort by key (this reproduces the reference's
+// rebuilt cell lists, which keep particles in visiting order): rows into
+// their leaf's bin, then one CTA per leaf orders its bin; a gather of the 9
+// particle arrays; the 27-neighbour table and the per-cell particle ranges.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -62,67 +63,68 @@ __device__ __forceinline__ bool in_regions(const SourceRegions& r, const float p
 __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float fmul(float a, float b) { return __fmul_rn(a, b); }
 
+// One more particle of each lane's key in its leaf's count, one atomic per
+// leaf in the warp.  Called by all 32 lanes.
+__device__ __forceinline__ void count_leaf(uint32_t* __restrict__ lcnt, uint32_t key) {
+  const unsigned same = __match_any_sync(0xffffffffu, key >> 9);
+  if (key != kDeadKey && int(threadIdx.x & 31) == __ffs(int(same)) - 1)
+    atomicAdd(lcnt + (key >> 9), unsigned(__popc(same)));
+}
+__global__ void k_count_leaves(const uint32_t* __restrict__ k, int64_t n,
+                               uint32_t* __restrict__ lcnt) {
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  count_leaf(lcnt, i < n ? k[i] : kDeadKey);
+}
+
 // mode 0: key from current position (upload); positions outside [0,N]
 //         are counted as invalid.
 // mode 1: advect by gvel*dt, clamp, delete in solids (MoveParticles).
-// mode 1 extras: particles inside a source region get the dead key
-// (DeleteFluidInSources right after MoveParticles); kout64 (optional) gets
-// (new key << 32 | old key), so that a stable sort on it orders particles as
-// the reference's rebuilt lists do when particles were appended to cell lists
-// (the visiting order is by old cell, then list position).
+// mode 1 extra: particles inside a source region get the dead key
+// (DeleteFluidInSources right after MoveParticles).
 __global__ void k_keys(float* __restrict__ part, int64_t cap, const uint32_t* __restrict__ kcur,
-                       uint32_t* __restrict__ kout, uint32_t* __restrict__ vout, int64_t n,
-                       LeafMap lm, SolidDesc sd, int mode, float dt,
-                       unsigned long long* __restrict__ invalid, const SourceRegions reg,
-                       unsigned long long* __restrict__ kout64) {
-  int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  vout[i] = uint32_t(i);
-  float* px = part;
-  float* gx = part + 6 * cap;
-  float p[3] = {px[i], px[cap + i], px[2 * cap + i]};
-  if (mode == 1) {
-    if (kcur[i] == kDeadKey) {
-      kout[i] = kDeadKey;
-      if (kout64) kout64[i] = ~0ull;
-      return;
-    }
-    const float g[3] = {gx[i], gx[cap + i], gx[2 * cap + i]};
+                       uint32_t* __restrict__ kout, int64_t n, LeafMap lm, SolidDesc sd, int mode,
+                       float dt, unsigned long long* __restrict__ invalid,
+                       const SourceRegions reg, uint32_t* __restrict__ lcnt) {
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  uint32_t k = kDeadKey;
+  if (i < n && (mode != 1 || kcur[i] != kDeadKey)) {
+    float* px = part;
+    const float* gx = part + 6 * cap;
+    float p[3] = {px[i], px[cap + i], px[2 * cap + i]};
     int id[3];
+    if (mode == 1) {
+      const float g[3] = {gx[i], gx[cap + i], gx[2 * cap + i]};
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      p[d] = fadd(p[d], fmul(g[d], dt));
-      id[d] = int(floorf(p[d]));
+      for (int d = 0; d < 3; ++d) {
+        p[d] = fadd(p[d], fmul(g[d], dt));
+        id[d] = int(floorf(p[d]));
+      }
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+        if (id[d] < 0) { id[d] = 0; p[d] = 0.f; }
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+        if (id[d] >= lm.n[d]) { id[d] = lm.n[d]; p[d] = float(lm.n[d]); }
+      px[i] = p[0];
+      px[cap + i] = p[1];
+      px[2 * cap + i] = p[2];
+      if (!is_solid(sd, id[0], id[1], id[2])) k = cell_key(lm, id[0], id[1], id[2]);
+      if (reg.n > 0 && in_regions(reg, p)) k = kDeadKey;
+    } else {
+      bool ok = true;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        ok &= (p[d] >= 0.f) && (p[d] <= float(lm.n[d]));
+        id[d] = int(floorf(p[d]));
+      }
+      if (ok)
+        k = cell_key(lm, id[0], id[1], id[2]);
+      else
+        atomicAdd(invalid, 1ull);
     }
-#pragma unroll
-    for (int d = 0; d < 3; ++d)
-      if (id[d] < 0) { id[d] = 0; p[d] = 0.f; }
-#pragma unroll
-    for (int d = 0; d < 3; ++d)
-      if (id[d] >= lm.n[d]) { id[d] = lm.n[d]; p[d] = float(lm.n[d]); }
-    px[i] = p[0];
-    px[cap + i] = p[1];
-    px[2 * cap + i] = p[2];
-    uint32_t k = is_solid(sd, id[0], id[1], id[2]) ? kDeadKey : cell_key(lm, id[0], id[1], id[2]);
-    if (reg.n > 0 && in_regions(reg, p)) k = kDeadKey;
-    kout[i] = k;
-    if (kout64)
-      kout64[i] = (k == kDeadKey) ? ~0ull : ((static_cast<unsigned long long>(k) << 32) | kcur[i]);
-  } else {
-    bool ok = true;
-    int id[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      ok &= (p[d] >= 0.f) && (p[d] <= float(lm.n[d]));
-      id[d] = int(floorf(p[d]));
-    }
-    if (!ok) {
-      atomicAdd(invalid, 1ull);
-      kout[i] = kDeadKey;
-      return;
-    }
-    kout[i] = cell_key(lm, id[0], id[1], id[2]);
   }
+  count_leaf(lcnt, k);
+  if (i < n) kout[i] = k;
 }
 
 // The keys of a step on a host-resident state (fsim_step_host), one pass over
@@ -135,9 +137,9 @@ __global__ void k_keys(float* __restrict__ part, int64_t cap, const uint32_t* __
 __global__ void __launch_bounds__(256)
     k_host_keys(const float* __restrict__ pos, const float* __restrict__ gvel,
                 float* __restrict__ part, int64_t cap, uint32_t* __restrict__ kold,
-                uint32_t* __restrict__ knew, uint32_t* __restrict__ vout, int64_t n, LeafMap lm,
-                SolidDesc sd, float dt, int keep_gvel, unsigned long long* __restrict__ invalid,
-                unsigned long long* __restrict__ unsorted) {
+                uint32_t* __restrict__ knew, int64_t n, LeafMap lm, SolidDesc sd, float dt,
+                int keep_gvel, unsigned long long* __restrict__ invalid,
+                unsigned long long* __restrict__ unsorted, uint32_t* __restrict__ lcnt) {
   const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   auto old_key = [&](int64_t r, float (&p)[3]) {
     bool ok = true;
@@ -160,72 +162,33 @@ __global__ void __launch_bounds__(256)
     if (desc) atomicAdd(unsorted, static_cast<unsigned long long>(__popc(desc)));
     if (bad) atomicAdd(invalid, static_cast<unsigned long long>(__popc(bad)));
   }
-  if (i >= n) return;
-  int id[3];
-  float g[3];
+  uint32_t k = kDeadKey;
+  if (i < n) {
+    int id[3];
+    float g[3];
 #pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    g[d] = gvel[3 * i + d];
-    p[d] = fadd(p[d], fmul(g[d], dt));
-    id[d] = int(floorf(p[d]));
-  }
-#pragma unroll
-  for (int d = 0; d < 3; ++d)
-    if (id[d] < 0) { id[d] = 0; p[d] = 0.f; }
-#pragma unroll
-  for (int d = 0; d < 3; ++d)
-    if (id[d] >= lm.n[d]) { id[d] = lm.n[d]; p[d] = float(lm.n[d]); }
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    part[d * cap + i] = p[d];
-    if (keep_gvel) part[(6 + d) * cap + i] = g[d];
-  }
-  kold[i] = old;
-  knew[i] = is_solid(sd, id[0], id[1], id[2]) ? kDeadKey : cell_key(lm, id[0], id[1], id[2]);
-  vout[i] = uint32_t(i);
-}
-
-__global__ void k_permute_keys(const uint32_t* __restrict__ in, const uint32_t* __restrict__ perm,
-                               uint32_t* __restrict__ out, int64_t n) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = in[perm[i]];
-}
-
-// Live particles = index of the first dead key: the keys are sorted and the
-// dead key is the largest value.  One block narrows [lo, hi] (which holds
-// that index; hi = n when no key is dead) by probing blockDim.x evenly spaced
-// keys per round, about 1000x per round, instead of reading all n keys.
-__global__ void k_count_live(const uint32_t* __restrict__ k, int64_t n, int64_t* cnt) {
-  __shared__ int64_t s_lo, s_hi;
-  __shared__ int s_first;
-  if (threadIdx.x == 0) {
-    s_lo = 0;
-    s_hi = n;
-  }
-  __syncthreads();
-  for (;;) {
-    const int64_t lo = s_lo, hi = s_hi;
-    if (lo >= hi) break;
-    const int64_t nb = blockDim.x;
-    const int64_t step = (hi - lo + nb - 1) / nb;
-    const int64_t pr = lo + int64_t(threadIdx.x) * step;  // this thread's probe
-    if (threadIdx.x == 0) s_first = INT_MAX;
-    __syncthreads();
-    if (pr < hi && k[pr] == kDeadKey) atomicMin(&s_first, int(threadIdx.x));
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      const int t = s_first;
-      if (t == INT_MAX) {  // every probe live: the first dead key lies past the last probe
-        const int64_t last = lo + ((hi - 1 - lo) / step) * step;
-        s_lo = last + 1;
-      } else {  // between the last live probe and probe t (dead)
-        s_lo = t == 0 ? lo : lo + int64_t(t - 1) * step + 1;
-        s_hi = lo + int64_t(t) * step;
-      }
+    for (int d = 0; d < 3; ++d) {
+      g[d] = gvel[3 * i + d];
+      p[d] = fadd(p[d], fmul(g[d], dt));
+      id[d] = int(floorf(p[d]));
     }
-    __syncthreads();
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      if (id[d] < 0) { id[d] = 0; p[d] = 0.f; }
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      if (id[d] >= lm.n[d]) { id[d] = lm.n[d]; p[d] = float(lm.n[d]); }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      part[d * cap + i] = p[d];
+      if (keep_gvel) part[(6 + d) * cap + i] = g[d];
+    }
+    if (!is_solid(sd, id[0], id[1], id[2])) k = cell_key(lm, id[0], id[1], id[2]);
+    kold[i] = old;
+    knew[i] = k;
   }
-  if (threadIdx.x == 0) cnt[0] = s_lo;
+  // (an invalid upload's rows may lie anywhere; nothing is set up from them)
+  count_leaf(lcnt, k);
 }
 
 // Four sorted keys per thread (one 16-byte load; key arrays start 256-byte
@@ -245,79 +208,307 @@ __device__ __forceinline__ void load_keys4(const uint32_t* __restrict__ k, int64
   }
 }
 
+// particles of a leaf that k_sort_leaf orders in shared memory, and the bit
+// set in cnt[1] when a leaf holds more
+constexpr int kLeafSort = 12288;
+constexpr int64_t kLeafOverflow = int64_t(1) << 40;
+
 // Permutes the first NF particle arrays (9: pos, vel, gvel; 6: pos, vel).
 template <int NF>
 __global__ void k_gather(const float* __restrict__ in, float* __restrict__ out, int64_t cap,
                          const uint32_t* __restrict__ perm, const int64_t* __restrict__ cnt) {
   int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int64_t n = cnt[0];
+  const int64_t n = cnt[1] & kLeafOverflow ? 0 : cnt[0];
   if (i >= n) return;
   const int64_t src = perm[i];
 #pragma unroll
   for (int f = 0; f < NF; ++f) out[f * cap + i] = in[f * cap + src];
 }
 
-__global__ void k_mark_pleaf(const uint32_t* __restrict__ k, const int64_t* __restrict__ cnt,
-                             uint8_t* __restrict__ flag) {
-  const int64_t n = cnt[0];
-  const int64_t i0 = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) * kKeysPerThread;
-  if (i0 >= n) return;
-  uint32_t v[kKeysPerThread];
-  load_keys4(k, i0, n, v);
-  uint32_t prev = i0 == 0 ? kDeadKey : (k[i0 - 1] >> 9);  // kDeadKey is no leaf id
+// The leaf topology from the particles' counts, in two kernels over tiles of
+// 1,024 leaf ids: k_leaf_flags marks the leaves with particles (1) and the
+// rest of their one-leaf dilation (2) and adds up its tile; k_leaf_slots adds
+// up the tiles before its own and numbers the leaves (those with particles
+// first) and the start of each leaf's particles.  The counts come with the
+// keys, so this needs no sorted keys and runs before the sort.  Both kernels
+// are a latency: 15 us at 4,096 leaf ids and 39 at 64,000 (launches timed one
+// by one), where finding the live keys, marking, dilation, a library scan and
+// the assignment, in seven launches, took 41 and 71.
+constexpr int kLeafTile = 1024;
+__global__ void __launch_bounds__(kLeafTile)
+    k_leaf_flags(const uint32_t* __restrict__ lcnt, uint8_t* __restrict__ flag,
+                 uint4* __restrict__ tile, LeafMap lm) {
+  __shared__ uint4 sh[kLeafTile / 32];
+  const uint32_t d = blockIdx.x * kLeafTile + threadIdx.x;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint32_t c = 0, f = 0;
+  if (d < lm.dense) {
+    c = lcnt[d];
+    f = c ? 1u : 0u;
+    int lx, ly, lz;
+    leaf_coords(lm, d, lx, ly, lz);
+    if (!c && leaf_valid(lm, lx, ly, lz)) {
+      uint32_t any = 0;  // independent loads: no early exit
 #pragma unroll
-  for (int j = 0; j < kKeysPerThread; ++j) {
-    if (i0 + j >= n) break;
-    const uint32_t l = v[j] >> 9;
-    if (l != prev) flag[l] = 1;
-    prev = l;
+      for (int q = 0; q < 27; ++q) {
+        const int ax = lx + q / 9 - 1, ay = ly + (q / 3) % 3 - 1, az = lz + q % 3 - 1;
+        if (leaf_valid(lm, ax, ay, az)) any |= lcnt[leaf_id(lm, ax, ay, az)];
+      }
+      f = any ? 2u : 0u;
+    }
+    flag[d] = uint8_t(f);
+  }
+  // tile totals: leaves with particles, dilated ones, particles; the fullest leaf
+  uint4 t = make_uint4(__popc(__ballot_sync(0xffffffffu, f == 1u)),
+                       __popc(__ballot_sync(0xffffffffu, f == 2u)), c, c);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    t.z += __shfl_xor_sync(0xffffffffu, t.z, o);
+    t.w = max(t.w, __shfl_xor_sync(0xffffffffu, t.w, o));
+  }
+  if (lane == 0) sh[w] = t;
+  __syncthreads();
+  if (w == 0) {
+    t = sh[lane];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
+      t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
+      t.z += __shfl_xor_sync(0xffffffffu, t.z, o);
+      t.w = max(t.w, __shfl_xor_sync(0xffffffffu, t.w, o));
+    }
+    if (lane == 0) tile[blockIdx.x] = t;
   }
 }
 
-__global__ void k_dilate(uint8_t* __restrict__ flag, LeafMap lm) {
-  uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
-  if (d >= lm.dense) return;
-  if (flag[d] & 1) return;
-  int lx, ly, lz;
-  leaf_coords(lm, d, lx, ly, lz);
-  if (!leaf_valid(lm, lx, ly, lz)) return;
-  for (int dx = -1; dx <= 1; ++dx)
-    for (int dy = -1; dy <= 1; ++dy)
-      for (int dz = -1; dz <= 1; ++dz) {
-        int ax = lx + dx, ay = ly + dy, az = lz + dz;
-        if (!leaf_valid(lm, ax, ay, az)) continue;
-        if (flag[leaf_id(lm, ax, ay, az)] & 1) {
-          flag[d] = 2;
-          return;
+// cnt: live particles; particle leaves, with kLeafOverflow when a leaf holds
+// more than kLeafSort; all leaves
+__global__ void __launch_bounds__(kLeafTile)
+    k_leaf_slots(const uint32_t* __restrict__ lcnt, const uint8_t* __restrict__ flag,
+                 const uint4* __restrict__ tile, int32_t* __restrict__ slot,
+                 int32_t* __restrict__ leaf_of, uint32_t* __restrict__ start, uint32_t n,
+                 int64_t* __restrict__ cnt) {
+  __shared__ uint4 sh[kLeafTile / 32], all[kLeafTile / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint32_t d = blockIdx.x * kLeafTile + threadIdx.x;
+  const uint32_t c = d < n ? lcnt[d] : 0u, f = d < n ? flag[d] : 0u;
+  uint4 b = make_uint4(0u, 0u, 0u, 0u), a = b;  // tiles before this one; all tiles
+  for (uint32_t q = threadIdx.x; q < gridDim.x; q += kLeafTile) {
+    const uint4 t = tile[q];
+    a.x += t.x;
+    a.y += t.y;
+    a.z += t.z;
+    a.w = max(a.w, t.w);
+    if (q < blockIdx.x) {
+      b.x += t.x;
+      b.y += t.y;
+      b.z += t.z;
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    b.x += __shfl_xor_sync(0xffffffffu, b.x, o);
+    b.y += __shfl_xor_sync(0xffffffffu, b.y, o);
+    b.z += __shfl_xor_sync(0xffffffffu, b.z, o);
+    a.x += __shfl_xor_sync(0xffffffffu, a.x, o);
+    a.y += __shfl_xor_sync(0xffffffffu, a.y, o);
+    a.z += __shfl_xor_sync(0xffffffffu, a.z, o);
+    a.w = max(a.w, __shfl_xor_sync(0xffffffffu, a.w, o));
+  }
+  // within the warp: leaves by ballot, particles by an inclusive scan
+  const unsigned m1 = __ballot_sync(0xffffffffu, f == 1u), m2 = __ballot_sync(0xffffffffu, f == 2u);
+  uint32_t incl = c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  // a warp's entry: its share of the tiles before, and its own totals
+  __shared__ uint4 own[kLeafTile / 32];
+  if (lane == 31) own[w] = make_uint4(__popc(m1), __popc(m2), incl, 0u);
+  if (lane == 0) {
+    sh[w] = b;
+    all[w] = a;
+  }
+  __syncthreads();
+  uint32_t np = 0, p1 = 0, p2 = 0, pc = 0;
+  a = all[lane];
+  b = sh[lane];
+  const uint4 o4 = own[lane];
+  if (lane < w) {
+    b.x += o4.x;
+    b.y += o4.y;
+    b.z += o4.z;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a.x += __shfl_xor_sync(0xffffffffu, a.x, o);
+    a.y += __shfl_xor_sync(0xffffffffu, a.y, o);
+    a.z += __shfl_xor_sync(0xffffffffu, a.z, o);
+    a.w = max(a.w, __shfl_xor_sync(0xffffffffu, a.w, o));
+    b.x += __shfl_xor_sync(0xffffffffu, b.x, o);
+    b.y += __shfl_xor_sync(0xffffffffu, b.y, o);
+    b.z += __shfl_xor_sync(0xffffffffu, b.z, o);
+  }
+  np = a.x;
+  const unsigned below = (1u << lane) - 1u;
+  p1 = b.x + __popc(m1 & below);
+  p2 = b.y + __popc(m2 & below);
+  pc = b.z + incl - c;
+  if (d == 0) {
+    cnt[0] = int64_t(a.z);
+    cnt[1] = int64_t(np) | (a.w > unsigned(kLeafSort) ? kLeafOverflow : 0);
+    cnt[2] = int64_t(np + a.y);
+  }
+  if (d >= n) return;
+  const int sl = f == 1u ? int(p1) : (f == 2u ? int(np + p2) : -1);
+  slot[d] = sl;
+  if (sl >= 0) leaf_of[sl] = int32_t(d);
+  start[d] = pc;
+}
+
+// ---- the stable sort by cell key ------------------------------------------------
+// The keys are a leaf's number and a cell's, and a leaf's particles fit in
+// shared memory, so two kernels do what a radix sort over all key bits takes
+// three to four passes through memory for; the old keys of a host step's rows
+// (those of appended source particles too) break ties there, instead of a
+// sort of their own before.  32.2 M rows, out of order: 630 us against 1,977
+// (two library sorts and a permutation); 52,894 rows: 22 against 57.  Bound
+// by the bins' traffic (18 to 26 B per row) and shared-memory atomics.
+//
+// k_bin_rows: each row's number, cell in the leaf and (OLD) old key to the
+// next place of its leaf's bin, one atomic per leaf in a warp (rows that were
+// in cell order before a move have one or two).  The places within a bin come
+// in any order; k_sort_leaf's order does not depend on it.
+template <bool OLD>
+__global__ void __launch_bounds__(256)
+    k_bin_rows(const uint32_t* __restrict__ knew, const uint32_t* __restrict__ kold, int64_t n,
+               uint32_t* __restrict__ next, uint32_t* __restrict__ row,
+               uint32_t* __restrict__ old, uint16_t* __restrict__ cell) {
+  constexpr int kPer = 4;
+  const int64_t i0 = (int64_t(blockIdx.x) * 256 + (threadIdx.x & ~31u)) * kPer + (threadIdx.x & 31);
+  const int lane = threadIdx.x & 31;
+  uint32_t k[kPer], q[kPer];
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) k[j] = i0 + 32 * j < n ? knew[i0 + 32 * j] : kDeadKey;
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    const unsigned same = __match_any_sync(0xffffffffu, k[j] >> 9);
+    const int lead = __ffs(int(same)) - 1;
+    uint32_t b = 0;
+    if (k[j] != kDeadKey && lane == lead) b = atomicAdd(next + (k[j] >> 9), unsigned(__popc(same)));
+    q[j] = __shfl_sync(0xffffffffu, b, lead) + __popc(same & ((1u << lane) - 1u));
+  }
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    if (k[j] == kDeadKey) continue;
+    row[q[j]] = uint32_t(i0 + 32 * j);
+    cell[q[j]] = uint16_t(k[j] & 511u);
+    if (OLD) old[q[j]] = kold[i0 + 32 * j];
+  }
+}
+
+// k_sort_leaf: a CTA orders a leaf's bin by (cell, old key, row): a counting
+// sort by cell into shared memory, then each cell's entries by one thread
+// (insertion; about 8 of them), or by the CTA (rank by counting) past
+// kCellSort.  keys and perm get the leaf's sorted keys and rows.
+constexpr int kLeafSortThreads = 1024;
+constexpr int kCellSort = 48;
+template <bool OLD>
+using SortEntry = typename std::conditional<OLD, unsigned long long, uint32_t>::type;
+template <bool OLD>
+__global__ void __launch_bounds__(kLeafSortThreads)
+    k_sort_leaf(const int32_t* __restrict__ leaf_of, const int64_t* __restrict__ cnt,
+                const uint32_t* __restrict__ lcnt, const uint32_t* __restrict__ next,
+                const uint32_t* __restrict__ row, const uint32_t* __restrict__ old,
+                const uint16_t* __restrict__ cell, uint32_t* __restrict__ keys,
+                uint32_t* __restrict__ perm) {
+  using E = SortEntry<OLD>;
+  extern __shared__ __align__(16) unsigned char sort_smem[];
+  E* ent = reinterpret_cast<E*>(sort_smem);  // kLeafSort entries
+  __shared__ int at[512];                    // a cell's count, then its next place
+  __shared__ int wsum[16];
+  __shared__ int big[kLeafSort / kCellSort], nbig;
+  if (cnt[1] & kLeafOverflow) return;  // the host sorts another way
+  const int np = int(cnt[1]), tid = threadIdx.x, lane = tid & 31;
+  for (int s = blockIdx.x; s < np; s += gridDim.x) {
+    const uint32_t d = uint32_t(leaf_of[s]);
+    const int m = int(lcnt[d]);
+    const uint32_t b = next[d] - uint32_t(m);  // k_bin_rows left it at the bin's end
+    if (tid < 512) at[tid] = 0;
+    if (tid == 0) nbig = 0;
+    __syncthreads();
+    for (int j = tid; j < m; j += kLeafSortThreads) atomicAdd(&at[cell[b + j]], 1);
+    __syncthreads();
+    int c = 0, first = 0;
+    if (tid < 512) {
+      c = at[tid];
+      first = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, first, o);
+        if (lane >= o) first += v;
+      }
+      if (lane == 31) wsum[tid >> 5] = first;
+    }
+    __syncthreads();
+    if (tid < 512) {
+      int before = lane < (tid >> 5) ? wsum[lane & 15] : 0;  // at most 15 warps before
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+      first += before - c;
+      at[tid] = first;
+    }
+    __syncthreads();
+    for (int j = tid; j < m; j += kLeafSortThreads) {
+      const int v = cell[b + j];
+      const int p = atomicAdd(&at[v], 1);
+      E e = row[b + j];
+      if constexpr (OLD) e |= static_cast<unsigned long long>(old[b + j]) << 32;
+      ent[p] = e;
+      keys[b + p] = (d << 9) | uint32_t(v);
+    }
+    __syncthreads();
+    if (tid < 512) {
+      if (c > kCellSort) {
+        big[atomicAdd(&nbig, 1)] = tid;
+      } else {
+        for (int x = first + 1; x < first + c; ++x) {
+          const E e = ent[x];
+          int y = x;
+          for (; y > first && ent[y - 1] > e; --y) ent[y] = ent[y - 1];
+          ent[y] = e;
         }
       }
-}
-
-__global__ void k_scan_in(const uint8_t* __restrict__ flag, uint64_t* __restrict__ v, uint32_t n) {
-  uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
-  if (d >= n) return;
-  uint8_t f = flag[d];
-  v[d] = uint64_t(f & 1) | (uint64_t(f == 2) << 32);
-}
-
-__global__ void k_assign(const uint8_t* __restrict__ flag, const uint64_t* __restrict__ in,
-                         const uint64_t* __restrict__ ex, int32_t* __restrict__ slot,
-                         int32_t* __restrict__ leaf_of, uint32_t n, int64_t* cnt) {
-  uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
-  if (d >= n) return;
-  const uint64_t tot = ex[n - 1] + in[n - 1];
-  const int np = int(tot & 0xFFFFFFFFull);
-  const int ng = int(tot >> 32);
-  if (d == 0) {
-    cnt[1] = np;
-    cnt[2] = np + ng;
+    }
+    __syncthreads();
+    for (int j = tid; j < m; j += kLeafSortThreads) perm[b + j] = uint32_t(ent[j]);
+    __syncthreads();
+    for (int q = 0; q < nbig; ++q) {
+      const int end = at[big[q]], beg = big[q] ? at[big[q] - 1] : 0;
+      for (int x = beg + tid; x < end; x += kLeafSortThreads) {
+        const E e = ent[x];
+        int rank = 0;
+        for (int y = beg; y < end; ++y) rank += ent[y] < e;
+        perm[b + beg + rank] = uint32_t(e);
+      }
+    }
+    __syncthreads();  // before the next leaf's counts
   }
-  uint8_t f = flag[d];
-  int s = -1;
-  if (f & 1) s = int(ex[d] & 0xFFFFFFFFull);
-  else if (f == 2) s = np + int(ex[d] >> 32);
-  slot[d] = s;
-  if (s >= 0) leaf_of[s] = int32_t(d);
+}
+
+// For the library sort of leaves too full for k_sort_leaf: row numbers, and
+// (new key << 32 | old key)
+__global__ void k_rows(uint32_t* __restrict__ v, int64_t n) {
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i < n) v[i] = uint32_t(i);
+}
+__global__ void k_join_keys(const uint32_t* __restrict__ knew, const uint32_t* __restrict__ kold,
+                            unsigned long long* __restrict__ k64, int64_t n) {
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t k = knew[i];
+  k64[i] = k == kDeadKey ? ~0ull : (static_cast<unsigned long long>(k) << 32) | kold[i];
 }
 
 __global__ void k_nbr(const int32_t* __restrict__ leaf_of, const int32_t* __restrict__ slot,
@@ -410,7 +601,7 @@ __device__ float pass_phi(const fsim_seed_pass& ps, const float p[3]) {
 // write == 1: reserve with the same aggregation and emit particles + keys.
 __global__ void k_seed(const __grid_constant__ SeedArgs a, LeafMap lm, SolidDesc sd, int write,
                        unsigned long long* __restrict__ counter, float* __restrict__ part,
-                       int64_t cap, uint32_t* __restrict__ kout, uint32_t* __restrict__ vout) {
+                       int64_t cap, uint32_t* __restrict__ kout) {
   const int64_t ncell = int64_t(lm.n[0]) * lm.n[1] * lm.n[2];
   int64_t c = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   int count = 0;
@@ -477,7 +668,6 @@ __global__ void k_seed(const __grid_constant__ SeedArgs a, LeafMap lm, SolidDesc
           part[(6 + d) * cap + o] = a.pass[ps].velocity[d];
         }
         kout[o] = key;
-        vout[o] = uint32_t(o);
       }
       ++o;
       ++pi;
@@ -636,132 +826,155 @@ int launch_host_keys(fsim_sim* s, const float* pos, const float* gvel, float dt,
   const int64_t n = s->n_total;
   unsigned long long* cnt = reinterpret_cast<unsigned long long*>(s->d_cnt);
   FSIM_CK(s, cudaMemsetAsync(s->d_cnt + 3, 0, 5 * sizeof(int64_t), s->stream));
+  FSIM_CK(s, cudaMemsetAsync(s->d_lcnt, 0, size_t(s->lm.dense) * 4, s->stream));
   FSIM_LAUNCH(s, "advect_keys", k_host_keys, nblk(n, 256), 256, 0, pos, gvel, s->part[s->cur],
-              s->cap_p, s->keys[0], s->keys[1], s->vals[1], n, s->lm, s->solid, dt,
-              keep_gvel ? 1 : 0, cnt + 3, cnt + 7);
+              s->cap_p, s->keys[0], s->keys[1], n, s->lm, s->solid, dt, keep_gvel ? 1 : 0, cnt + 3,
+              cnt + 7, s->d_lcnt);
   FSIM_CK(s, cudaMemcpyAsync(s->h_cnt + 3, s->d_cnt + 3, 5 * sizeof(int64_t),
                              cudaMemcpyDeviceToHost, s->stream));
   FSIM_CK(s, cudaStreamSynchronize(s->stream));
   *invalid = s->h_cnt[3];
-  s->composite_sort = false;
-  if (*invalid || s->h_cnt[7] == 0) return FSIM_OK;
-  // rows out of cell order: their old cells decide the order within a new cell,
-  // so they are sorted by old key first and by new key after (stable; one sort
-  // of (new, old) as 64-bit keys takes 2.8 ms at 32 M rows, these two 1.7)
-  int rc = ensure_keys64(s, (n + 1) / 2);
-  if (rc) return rc;
-  if ((rc = sort_pairs(s, s->keys[0], reinterpret_cast<uint32_t*>(s->keys64[0]), s->vals[1],
-                       s->vals[0], n)))
-    return rc;
-  FSIM_LAUNCH(s, "permute_keys", k_permute_keys, nblk(n, 256), 256, 0, s->keys[1], s->vals[0],
-              s->keys[0], n);
-  std::swap(s->keys[0], s->keys[1]);
-  std::swap(s->vals[0], s->vals[1]);
+  // rows out of cell order: their old cells decide the order within a new cell
+  s->composite_sort = s->h_cnt[7] != 0;
   return FSIM_OK;
 }
 
 int launch_keys_from_positions(fsim_sim* s, int mode, float dt) {
   const int64_t n = s->n_total;
   FSIM_CK(s, cudaMemsetAsync(s->d_cnt + 3, 0, sizeof(int64_t), s->stream));
+  FSIM_CK(s, cudaMemsetAsync(s->d_lcnt, 0, size_t(s->lm.dense) * 4, s->stream));
+  if (mode == 0) s->composite_sort = false;  // new particles: no old cells
   SourceRegions reg;
   memset(&reg, 0, sizeof(reg));
   if (mode == 1 && s->delete_in_sources) reg = regions_at(s, s->src_time);
-  unsigned long long* k64 = nullptr;
-  if (mode == 1 && s->composite_sort) {
-    const int rc = ensure_keys64(s, n);
-    if (rc) return rc;
-    k64 = reinterpret_cast<unsigned long long*>(s->keys64[1]);
-  }
   FSIM_LAUNCH(s, "advect_keys", k_keys, nblk(n, 256), 256, 0, s->part[s->cur], s->cap_p,
-              s->keys[0], s->keys[1], s->vals[1], n, s->lm, s->solid, mode, dt,
-              reinterpret_cast<unsigned long long*>(s->d_cnt + 3), reg, k64);
+              s->keys[0], s->keys[1], n, s->lm, s->solid, mode, dt,
+              reinterpret_cast<unsigned long long*>(s->d_cnt + 3), reg, s->d_lcnt);
   s->delete_in_sources = false;
   return FSIM_OK;
 }
 
-// Sorts keys[1]/vals[1] (n_total entries) into keys[0]/vals[0], gathers the
-// particles into the other buffer and rebuilds the leaf topology.
-int rebuild_topology(fsim_sim* s) {
-  const int64_t n = s->n_total;
-  const int bits = key_bits(s->lm);
-  if (s->composite_sort) {
-    // stable sort on (new key << 32 | old key), then the new keys back
-    unsigned long long* k64[2] = {reinterpret_cast<unsigned long long*>(s->keys64[0]),
-                                  reinterpret_cast<unsigned long long*>(s->keys64[1])};
-    size_t need = 0;
-    FSIM_CK(s, cub::DeviceRadixSort::SortPairs(nullptr, need, k64[1], k64[0], s->vals[1],
-                                               s->vals[0], n, 0, 32 + bits, s->stream));
-    if (need > s->sort_tmp_bytes) {
-      if (s->sort_tmp) cudaFree(s->sort_tmp);
-      s->sort_tmp = nullptr;
-      FSIM_CK(s, cudaMalloc(&s->sort_tmp, need));
-      s->sort_tmp_bytes = need;
-    }
-    if (n > 0) {
-      fsim::ProfScope ps(s, "radix_sort64(cub)");
-      FSIM_CK(s, cub::DeviceRadixSort::SortPairs(s->sort_tmp, need, k64[1], k64[0], s->vals[1],
-                                                 s->vals[0], n, 0, 32 + bits, s->stream));
-    }
-    FSIM_LAUNCH(s, "new_keys", k_hi_keys, nblk(n, 256), 256, 0, k64[0], s->keys[0], n);
-    s->composite_sort = false;
-    return rebuild_after_sort(s);
-  }
-  const int rc = sort_pairs(s, s->keys[1], s->keys[0], s->vals[1], s->vals[0], n);
-  if (rc) return rc;
-  return rebuild_after_sort(s);
+// the bins of k_bin_rows besides the row numbers (those are in vals[1])
+static int ensure_bins(fsim_sim* s, bool old) {
+  const size_t need = size_t(s->cap_p) * (old ? 6 : 2) + 256;
+  if (need <= s->bin_bytes) return FSIM_OK;
+  if (s->bins) cudaFree(s->bins);
+  s->bins = nullptr;
+  s->bin_bytes = 0;
+  FSIM_CK(s, cudaMalloc(&s->bins, need));
+  s->bin_bytes = need;
+  return FSIM_OK;
 }
 
-// keys[0]/vals[0] hold the sorted keys and permutation of n_total particles
-int rebuild_after_sort(fsim_sim* s, bool gather) {
+// keys[1] (with keys[0] as the old keys: OLD) into keys[0] and the rows' order
+// into vals[0]
+template <bool OLD>
+static int sort_by_leaf(fsim_sim* s) {
   const int64_t n = s->n_total;
-  FSIM_CK(s, cudaMemsetAsync(s->d_cnt, 0, 3 * sizeof(int64_t), s->stream));
-  FSIM_LAUNCH(s, "count_live", k_count_live, 1, 1024, 0, s->keys[0], n, s->d_cnt);
-  if (gather) {
-    // a velocity upload still in flight on the I/O stream (fsim_step_host)
-    if (s->io_vel_pending) {
-      FSIM_CK(s, cudaStreamWaitEvent(s->stream, s->ev_io, 0));
-      s->io_vel_pending = false;
-    }
-    if (s->gather_skip_gvel) {
-      FSIM_LAUNCH(s, "gather_particles", k_gather<6>, nblk(n, 256), 256, 0, s->part[s->cur],
-                  s->part[s->cur ^ 1], s->cap_p, s->vals[0], s->d_cnt);
-    } else {
-      FSIM_LAUNCH(s, "gather_particles", k_gather<9>, nblk(n, 256), 256, 0, s->part[s->cur],
-                  s->part[s->cur ^ 1], s->cap_p, s->vals[0], s->d_cnt);
+  const int rc = ensure_bins(s, OLD);
+  if (rc) return rc;
+  uint16_t* cell = static_cast<uint16_t*>(s->bins);
+  uint32_t* old = OLD ? reinterpret_cast<uint32_t*>(static_cast<char*>(s->bins) +
+                                                    (size_t(s->cap_p) * 2 + 255) / 256 * 256)
+                      : nullptr;
+  constexpr size_t smem = size_t(kLeafSort) * sizeof(SortEntry<OLD>);
+  FSIM_CK(s, cudaFuncSetAttribute(k_sort_leaf<OLD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  int(smem)));
+  FSIM_LAUNCH(s, "bin_rows", k_bin_rows<OLD>, nblk(n, 1024), 256, 0, s->keys[1], s->keys[0], n,
+              s->d_lnext, s->vals[1], old, cell);
+  FSIM_LAUNCH(s, "sort_leaves", k_sort_leaf<OLD>, 2 * s->num_sms, kLeafSortThreads, smem,
+              s->d_leaf_id, s->d_cnt, s->d_lcnt, s->d_lnext, s->vals[1], old, cell, s->keys[0],
+              s->vals[0]);
+  return FSIM_OK;
+}
+
+// The same order by the library's radix sort, for a state with a leaf of more
+// than kLeafSort particles (keys[0] and keys[1] are as they were).
+static int sort_by_library(fsim_sim* s, bool old) {
+  const int64_t n = s->n_total;
+  FSIM_LAUNCH(s, "sort_rows", k_rows, nblk(n, 256), 256, 0, s->vals[1], n);
+  if (!old) return sort_pairs(s, s->keys[1], s->keys[0], s->vals[1], s->vals[0], n);
+  // stable sort on (new key << 32 | old key), then the new keys back
+  const int bits = key_bits(s->lm);
+  int rc = ensure_keys64(s, n);
+  if (rc) return rc;
+  unsigned long long* k64[2] = {reinterpret_cast<unsigned long long*>(s->keys64[0]),
+                                reinterpret_cast<unsigned long long*>(s->keys64[1])};
+  FSIM_LAUNCH(s, "join_keys", k_join_keys, nblk(n, 256), 256, 0, s->keys[1], s->keys[0], k64[1], n);
+  size_t need = 0;
+  FSIM_CK(s, cub::DeviceRadixSort::SortPairs(nullptr, need, k64[1], k64[0], s->vals[1], s->vals[0],
+                                             n, 0, 32 + bits, s->stream));
+  if (need > s->sort_tmp_bytes) {
+    if (s->sort_tmp) cudaFree(s->sort_tmp);
+    s->sort_tmp = nullptr;
+    s->sort_tmp_bytes = 0;
+    FSIM_CK(s, cudaMalloc(&s->sort_tmp, need));
+    s->sort_tmp_bytes = need;
+  }
+  {
+    fsim::ProfScope ps(s, "radix_sort64(cub)");
+    FSIM_CK(s, cub::DeviceRadixSort::SortPairs(s->sort_tmp, need, k64[1], k64[0], s->vals[1],
+                                               s->vals[0], n, 0, 32 + bits, s->stream));
+  }
+  FSIM_LAUNCH(s, "new_keys", k_hi_keys, nblk(n, 256), 256, 0, k64[0], s->keys[0], n);
+  return FSIM_OK;
+}
+
+// Permutes the particles by vals[0] into the other buffer.
+static int gather_particles(fsim_sim* s) {
+  const int64_t n = s->n_total;
+  // a velocity upload still in flight on the I/O stream (fsim_step_host)
+  if (s->io_vel_pending) {
+    FSIM_CK(s, cudaStreamWaitEvent(s->stream, s->ev_io, 0));
+    s->io_vel_pending = false;
+  }
+  if (s->gather_skip_gvel) {
+    FSIM_LAUNCH(s, "gather_particles", k_gather<6>, nblk(n, 256), 256, 0, s->part[s->cur],
+                s->part[s->cur ^ 1], s->cap_p, s->vals[0], s->d_cnt);
+  } else {
+    FSIM_LAUNCH(s, "gather_particles", k_gather<9>, nblk(n, 256), 256, 0, s->part[s->cur],
+                s->part[s->cur ^ 1], s->cap_p, s->vals[0], s->d_cnt);
+  }
+  return FSIM_OK;
+}
+
+// The leaf topology of the n_total particles whose keys are in keys[1] and
+// counted in d_lcnt; sort: and their order (keys[0], vals[0]) and the
+// particles in it, else keys[0] holds the keys in order already.
+static int rebuild(fsim_sim* s, bool sort) {
+  const uint32_t D = s->lm.dense;
+  const unsigned tiles = nblk(int64_t(D), kLeafTile);
+  FSIM_LAUNCH(s, "leaf_flags", k_leaf_flags, tiles, kLeafTile, 0, s->d_lcnt, s->d_flag, s->d_tile,
+              s->lm);
+  FSIM_LAUNCH(s, "leaf_slots", k_leaf_slots, tiles, kLeafTile, 0, s->d_lcnt, s->d_flag, s->d_tile,
+              s->d_slot, s->d_leaf_id, s->d_lnext, D, s->d_cnt);
+  // the host reads the counts while the sort runs
+  FSIM_CK(s, cudaMemcpyAsync(s->h_cnt, s->d_cnt, 3 * sizeof(int64_t), cudaMemcpyDeviceToHost,
+                             s->stream));
+  FSIM_CK(s, cudaEventRecord(s->ev_topo, s->stream));
+  int rc;
+  const bool old = s->composite_sort;
+  if (sort && s->n_total > 0) {
+    if ((rc = old ? sort_by_leaf<true>(s) : sort_by_leaf<false>(s))) return rc;
+    if ((rc = gather_particles(s))) return rc;
+  }
+  FSIM_CK(s, cudaEventSynchronize(s->ev_topo));
+  if (sort) {
+    if (s->n_total > 0 && (s->h_cnt[1] & kLeafOverflow)) {
+      s->h_cnt[1] &= kLeafOverflow - 1;
+      FSIM_CK(s, cudaMemcpyAsync(s->d_cnt + 1, s->h_cnt + 1, sizeof(int64_t),
+                                 cudaMemcpyHostToDevice, s->stream));
+      if ((rc = sort_by_library(s, old))) return rc;
+      if ((rc = gather_particles(s))) return rc;
     }
     s->cur ^= 1;
   }
-  // leaves
-  const uint32_t D = s->lm.dense;
-  FSIM_CK(s, cudaMemsetAsync(s->d_flag, 0, D, s->stream));
-  FSIM_LAUNCH(s, "mark_leaves", k_mark_pleaf, nblk(n, 256 * kKeysPerThread), 256, 0, s->keys[0], s->d_cnt,
-              s->d_flag);
-  FSIM_LAUNCH(s, "dilate_leaves", k_dilate, nblk(D, 256), 256, 0, s->d_flag, s->lm);
-  FSIM_LAUNCH(s, "scan_input", k_scan_in, nblk(D, 256), 256, 0, s->d_flag, s->d_scan, D);
-  uint64_t* scan_out = s->d_scan + D;
-  size_t sneed = 0;
-  FSIM_CK(s, cub::DeviceScan::ExclusiveSum(nullptr, sneed, s->d_scan, scan_out, int(D), s->stream));
-  if (sneed > s->scan_tmp_bytes) {
-    if (s->scan_tmp) cudaFree(s->scan_tmp);
-    s->scan_tmp = nullptr;
-    FSIM_CK(s, cudaMalloc(&s->scan_tmp, sneed));
-    s->scan_tmp_bytes = sneed;
-  }
-  {
-    fsim::ProfScope ps(s, "leaf_scan(cub)");
-    FSIM_CK(s, cub::DeviceScan::ExclusiveSum(s->scan_tmp, sneed, s->d_scan, scan_out, int(D),
-                                             s->stream));
-  }
-  FSIM_LAUNCH(s, "assign_slots", k_assign, nblk(D, 256), 256, 0, s->d_flag, s->d_scan, scan_out,
-              s->d_slot, s->d_leaf_id, D, s->d_cnt);
-  FSIM_CK(s, cudaMemcpyAsync(s->h_cnt, s->d_cnt, 3 * sizeof(int64_t), cudaMemcpyDeviceToHost,
-                             s->stream));
-  FSIM_CK(s, cudaStreamSynchronize(s->stream));
+  s->composite_sort = false;
   s->n_live = s->h_cnt[0];
   s->n_total = s->n_live;
-  s->n_pleaf = int(s->h_cnt[1]);
+  s->n_pleaf = int(s->h_cnt[1] & (kLeafOverflow - 1));
   s->n_gleaf = int(s->h_cnt[2]);
-  int rc = ensure_leaf_capacity(s, s->n_gleaf, s->n_pleaf);
+  rc = ensure_leaf_capacity(s, s->n_gleaf, s->n_pleaf);
   if (rc != FSIM_OK) return rc;
   FSIM_LAUNCH(s, "neighbour_table", k_nbr, nblk(int64_t(s->n_gleaf) * 27, 256), 256, 0,
               s->d_leaf_id, s->d_slot, s->d_nbr, s->n_gleaf, s->lm);
@@ -777,6 +990,8 @@ int rebuild_after_sort(fsim_sim* s, bool gather) {
   s->deleted_outside = false;
   return FSIM_OK;
 }
+
+int rebuild_topology(fsim_sim* s) { return rebuild(s, true); }
 
 int seed_fluid(fsim_sim* s, const fsim_seed_pass* passes, int npasses, uint64_t seed) {
   if (npasses < 0 || npasses > 8) return fail(s, FSIM_ERR_INVALID, "npasses must be in [0,8]");
@@ -794,7 +1009,7 @@ int seed_fluid(fsim_sim* s, const fsim_seed_pass* passes, int npasses, uint64_t 
   unsigned long long* ctr = reinterpret_cast<unsigned long long*>(s->d_cnt + 5);
   FSIM_CK(s, cudaMemsetAsync(ctr, 0, sizeof(int64_t), s->stream));
   FSIM_LAUNCH(s, "seed_count", k_seed, nblk(ncell, 256), 256, 0, a, s->lm, s->solid, 0, ctr,
-              s->part[s->cur], s->cap_p, s->keys[1], s->vals[1]);
+              s->part[s->cur], s->cap_p, s->keys[1]);
   FSIM_CK(s, cudaMemcpyAsync(s->h_cnt + 5, s->d_cnt + 5, sizeof(int64_t), cudaMemcpyDeviceToHost,
                              s->stream));
   FSIM_CK(s, cudaStreamSynchronize(s->stream));
@@ -803,8 +1018,11 @@ int seed_fluid(fsim_sim* s, const fsim_seed_pass* passes, int npasses, uint64_t 
     return fail(s, FSIM_ERR_CAPACITY, "seeded particle count exceeds max_particles");
   FSIM_CK(s, cudaMemsetAsync(ctr, 0, sizeof(int64_t), s->stream));
   FSIM_LAUNCH(s, "seed_write", k_seed, nblk(ncell, 256), 256, 0, a, s->lm, s->solid, 1, ctr,
-              s->part[s->cur], s->cap_p, s->keys[1], s->vals[1]);
+              s->part[s->cur], s->cap_p, s->keys[1]);
   s->n_total = total;
+  s->composite_sort = false;
+  FSIM_CK(s, cudaMemsetAsync(s->d_lcnt, 0, size_t(s->lm.dense) * 4, s->stream));
+  FSIM_LAUNCH(s, "seed_leaves", k_count_leaves, nblk(total, 256), 256, 0, s->keys[1], total, s->d_lcnt);
   return rebuild_topology(s);
 }
 
@@ -824,7 +1042,7 @@ int rebin_uploaded(fsim_sim* s, int64_t* invalid) {
   if (*invalid) return FSIM_OK;
   if (s->h_cnt[7] == 0) {
     std::swap(s->keys[0], s->keys[1]);  // sorted already: keep the order
-    return rebuild_after_sort(s, false);
+    return rebuild(s, false);
   }
   return rebuild_topology(s);
 }
