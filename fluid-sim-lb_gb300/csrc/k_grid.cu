@@ -469,118 +469,128 @@ __device__ __forceinline__ void ref_node_sums(const GridArgs& a, const int* nb, 
   tw = Tw;
 }
 
+// Node sums of one neighbour block (zero when the block does not cover it).
+struct NodeSums {
+  unsigned long long v[3], w[3];
+  uint32_t on;
+};
+__device__ __forceinline__ void node_sums(const GridArgs& a, int ns, int o, bool use, NodeSums& q) {
+  const unsigned long long* blk = a.p2g_nodes + int64_t(use ? ns : 0) * 6 * kNodeBlock + o;
+#pragma unroll
+  for (int D = 0; D < 3; ++D) {
+    q.v[D] = use ? blk[D * kNodeBlock] : 0ull;
+    q.w[D] = use ? blk[(3 + D) * kNodeBlock] : 0ull;
+  }
+  q.on = use ? (a.p2g_touch[int64_t(ns) * 32 + (o >> 5)] >> (o & 31)) & 1u : 0u;
+}
+__device__ __forceinline__ void node_add(NodeSums& t, const NodeSums& q) {
+#pragma unroll
+  for (int D = 0; D < 3; ++D) {
+    t.v[D] += q.v[D];
+    t.w[D] += q.w[D];
+  }
+  t.on |= q.on;
+}
+
+// A thread's node takes its own leaf's sums and those of the neighbours whose
+// outer layer covers it: in each axis one side at most (e), so eight blocks at
+// most, and the x side is the same for a whole warp.  The loads of two blocks
+// are issued together (integer sums: their order does not matter).  Bound by
+// latency, so by warps in flight and short CTAs: a quarter leaf per CTA of 64
+// registers takes 8.2 us at 156 leaves, 33 at 128^3 and 156 / 280 (plain /
+// fused) at 256^3; a whole leaf 8.2, -, 201 / 317; all four blocks of an x
+// side at once 10, -, 333 / 451; the loop over neighbours before, one load
+// after another for two nodes per thread, 13.6, 38.6, 187 / 335.
+constexpr int kNodeThreads = 128;
 template <bool FUSED>
-__global__ void __launch_bounds__(256) k_p2g_nodes(const __grid_constant__ GridArgs a) {
+__global__ void __launch_bounds__(kNodeThreads, 8) k_p2g_nodes(const __grid_constant__ GridArgs a) {
   __shared__ int nb[27];
-  const int s = blockIdx.x;  // grid leaf
-  const int tid = threadIdx.x;
-  if (tid < 27) nb[tid] = a.nbr[int64_t(s) * 27 + tid];
+  const int s = blockIdx.x / (512 / kNodeThreads);  // grid leaf
+  const int v = threadIdx.x + int(blockIdx.x % (512 / kNodeThreads)) * kNodeThreads;
+  if (threadIdx.x < 27) nb[threadIdx.x] = a.nbr[int64_t(s) * 27 + threadIdx.x];
   __syncthreads();
   int org[3];
   origin_of(a, s, org);
-  float* vel = a.vel + int64_t(s) * 1536;
-  // this leaf's own block entries for both of the thread's nodes, loaded
-  // before either is used; the node loop then adds the neighbour particle
-  // leaves that cover a node with their outer layer (integer sums: the order
-  // does not matter)
-  unsigned long long own_v[2][3], own_w[2][3];
-  bool own_on[2];
-  {
-    const int ns = nb[nb_index(0, 0, 0)];
-    const bool own = ns >= 0 && ns < a.n_pleaf;
-    const unsigned long long* blk = a.p2g_nodes + int64_t(own ? ns : 0) * 6 * kNodeBlock;
+  const int x = v >> 6, y = (v >> 3) & 7, z = v & 7;
+  const int g[3] = {org[0] + x, org[1] + y, org[2] + z};
+  const int e[3] = {x == 0 ? -1 : (x == 7 ? 1 : 0), y == 0 ? -1 : (y == 7 ? 1 : 0),
+                    z == 0 ? -1 : (z == 7 ? 1 : 0)};
+  NodeSums sum = {};
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int v = tid + 256 * j;
-      const int o = node_index(v >> 6, (v >> 3) & 7, v & 7);
+  for (int h = 0; h < 2; ++h) {
+    const int dx = h ? e[0] : 0;
+    if (h && dx == 0) break;  // the same for the whole warp
 #pragma unroll
-      for (int D = 0; D < 3; ++D) {
-        own_v[j][D] = own ? blk[D * kNodeBlock + o] : 0ull;
-        own_w[j][D] = own ? blk[(3 + D) * kNodeBlock + o] : 0ull;
+    for (int c0 = 0; c0 < 4; c0 += 2) {
+      NodeSums q[2];
+#pragma unroll
+      for (int c = c0; c < c0 + 2; ++c) {
+        const int dy = (c & 2) ? e[1] : 0, dz = (c & 1) ? e[2] : 0;
+        const int ns = nb[nb_index(dx, dy, dz)];
+        const bool use = ns >= 0 && ns < a.n_pleaf && (!(c & 2) || dy != 0) && (!(c & 1) || dz != 0);
+        node_sums(a, ns, node_index(x - 8 * dx, y - 8 * dy, z - 8 * dz), use, q[c - c0]);
       }
-      own_on[j] = own && ((a.p2g_touch[int64_t(ns) * 32 + (o >> 5)] >> (o & 31)) & 1u);
+#pragma unroll
+      for (int c = 0; c < 2; ++c) node_add(sum, q[c]);
     }
   }
+  const unsigned long long (&sv)[3] = sum.v, (&sw)[3] = sum.w;
+  const bool on = sum.on != 0u;
+  float* vel = a.vel + int64_t(s) * 1536;
+  float val[3];
+  float wsum[3];
 #pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    const int v = tid + 256 * j;
-    const int x = v >> 6, y = (v >> 3) & 7, z = v & 7;
-    const int g[3] = {org[0] + x, org[1] + y, org[2] + z};
-    unsigned long long sv[3] = {own_v[j][0], own_v[j][1], own_v[j][2]};
-    unsigned long long sw[3] = {own_w[j][0], own_w[j][1], own_w[j][2]};
-    bool on = own_on[j];
-    const int dlo[3] = {x == 0 ? -1 : 0, y == 0 ? -1 : 0, z == 0 ? -1 : 0};
-    const int dhi[3] = {x == 7 ? 1 : 0, y == 7 ? 1 : 0, z == 7 ? 1 : 0};
-    for (int dx = dlo[0]; dx <= dhi[0]; ++dx)
-      for (int dy = dlo[1]; dy <= dhi[1]; ++dy)
-        for (int dz = dlo[2]; dz <= dhi[2]; ++dz) {
-          if (dx == 0 && dy == 0 && dz == 0) continue;  // the own block, loaded above
-          const int ns = nb[nb_index(dx, dy, dz)];
-          if (ns < 0 || ns >= a.n_pleaf) continue;
-          const int o = node_index(x - 8 * dx, y - 8 * dy, z - 8 * dz);
-          const unsigned long long* blk = a.p2g_nodes + int64_t(ns) * 6 * kNodeBlock;
-#pragma unroll
-          for (int D = 0; D < 3; ++D) {
-            sv[D] += blk[D * kNodeBlock + o];
-            sw[D] += blk[(3 + D) * kNodeBlock + o];
-          }
-          on |= (a.p2g_touch[int64_t(ns) * 32 + (o >> 5)] >> (o & 31)) & 1u;
-        }
-    float val[3];
-    float wsum[3];
+  for (int D = 0; D < 3; ++D) {
+    const float ws = from_fix(sw[D]);
+    const float ms = from_fix(sv[D]);
+    if (on && ws < kLowWeight)  // re-summed by k_p2g_low, which rewrites this face
+      a.p2g_low[1 + atomicAdd(a.p2g_low, 1u)] = unsigned(s) * 1536u + unsigned(D * 512 + v);
+    wsum[D] = ws;
+    // THRESH is a double literal in the reference: float ws < 1e-5 (double)
+    // is ws <= 1e-5f
+    val[D] = on ? ((ws <= 1e-5f) ? 0.f : __fdiv_rn(ms, ws)) : 0.f;
+  }
+  // marker: FLUID for in-box cells holding particles
+  bool has = false;
+  if (s < a.n_pleaf) {
+    const uint2 rg = a.cell_range[int64_t(s) * 512 + v];
+    has = rg.y > rg.x;
+  }
+  int m = (has && in_box(a.lm.n, g[0], g[1], g[2])) ? FSIM_FLUID : FSIM_AIR;
+  const unsigned ball = __ballot_sync(0xffffffffu, on);
+  if (FUSED) {
+    const bool sc = is_solid(a.sd, g[0], g[1], g[2]);
+    if (sc) m = FSIM_SOLID;
+    bool zero[3];
+    zero[0] = sc != is_solid(a.sd, g[0] - 1, g[1], g[2]);
+    zero[1] = sc != is_solid(a.sd, g[0], g[1] - 1, g[2]);
+    zero[2] = sc != is_solid(a.sd, g[0], g[1], g[2] - 1);
+    float* vold = a.vold + int64_t(s) * 1536;
+    const float gf[3] = {__fmul_rn(a.dt, a.fx), __fmul_rn(a.dt, a.fy), __fmul_rn(a.dt, a.fz)};
 #pragma unroll
     for (int D = 0; D < 3; ++D) {
-      const float ws = from_fix(sw[D]);
-      const float ms = from_fix(sv[D]);
-      if (on && ws < kLowWeight)  // re-summed by k_p2g_low, which rewrites this face
-        a.p2g_low[1 + atomicAdd(a.p2g_low, 1u)] = unsigned(s) * 1536u + unsigned(D * 512 + v);
-      wsum[D] = ws;
-      // THRESH is a double literal in the reference: float ws < 1e-5 (double)
-      // is ws <= 1e-5f
-      val[D] = on ? ((ws <= 1e-5f) ? 0.f : __fdiv_rn(ms, ws)) : 0.f;
+      float vv = val[D];
+      if (on && zero[D]) vv = 0.f;                 // ApplyBoundaryConditions
+      vold[D * 512 + v] = vv;                      // SaveGridVelocities
+      if (on) vv = (D == 1) ? __fsub_rn(vv, gf[1]) : __fadd_rn(vv, gf[D]);  // AddGravity
+      if (on && zero[D]) vv = 0.f;                 // ApplyBoundaryConditions
+      vel[D * 512 + v] = vv;
     }
-    // marker: FLUID for in-box cells holding particles
-    bool has = false;
-    if (s < a.n_pleaf) {
-      const uint2 rg = a.cell_range[int64_t(s) * 512 + v];
-      has = rg.y > rg.x;
+    if ((threadIdx.x & 31) == 0) {
+      a.vold_on[int64_t(s) * 16 + (v >> 5)] = ball;
     }
-    int m = (has && in_box(a.lm.n, g[0], g[1], g[2])) ? FSIM_FLUID : FSIM_AIR;
-    const unsigned ball = __ballot_sync(0xffffffffu, on);
-    if (FUSED) {
-      const bool sc = is_solid(a.sd, g[0], g[1], g[2]);
-      if (sc) m = FSIM_SOLID;
-      bool zero[3];
-      zero[0] = sc != is_solid(a.sd, g[0] - 1, g[1], g[2]);
-      zero[1] = sc != is_solid(a.sd, g[0], g[1] - 1, g[2]);
-      zero[2] = sc != is_solid(a.sd, g[0], g[1], g[2] - 1);
-      float* vold = a.vold + int64_t(s) * 1536;
-      const float gf[3] = {__fmul_rn(a.dt, a.fx), __fmul_rn(a.dt, a.fy), __fmul_rn(a.dt, a.fz)};
+  } else {
+    float* wt = a.weight + int64_t(s) * 1536;
 #pragma unroll
-      for (int D = 0; D < 3; ++D) {
-        float vv = val[D];
-        if (on && zero[D]) vv = 0.f;                 // ApplyBoundaryConditions
-        vold[D * 512 + v] = vv;                      // SaveGridVelocities
-        if (on) vv = (D == 1) ? __fsub_rn(vv, gf[1]) : __fadd_rn(vv, gf[D]);  // AddGravity
-        if (on && zero[D]) vv = 0.f;                 // ApplyBoundaryConditions
-        vel[D * 512 + v] = vv;
-      }
-      if ((threadIdx.x & 31) == 0) {
-        a.vold_on[int64_t(s) * 16 + (v >> 5)] = ball;
-      }
-    } else {
-      float* wt = a.weight + int64_t(s) * 1536;
-#pragma unroll
-      for (int D = 0; D < 3; ++D) {
-        vel[D * 512 + v] = val[D];
-        wt[D * 512 + v] = on ? wsum[D] : 0.f;
-      }
-      // ClearGridData left the saved velocity empty
-      if ((threadIdx.x & 31) == 0) a.vold_on[int64_t(s) * 16 + (v >> 5)] = 0u;
+    for (int D = 0; D < 3; ++D) {
+      vel[D * 512 + v] = val[D];
+      wt[D * 512 + v] = on ? wsum[D] : 0.f;
     }
-    if ((threadIdx.x & 31) == 0) a.vel_on[int64_t(s) * 16 + (v >> 5)] = ball;
-    a.marker[int64_t(s) * 512 + v] = int8_t(m);
+    // ClearGridData left the saved velocity empty
+    if ((threadIdx.x & 31) == 0) a.vold_on[int64_t(s) * 16 + (v >> 5)] = 0u;
   }
+  if ((threadIdx.x & 31) == 0) a.vel_on[int64_t(s) * 16 + (v >> 5)] = ball;
+  a.marker[int64_t(s) * 512 + v] = int8_t(m);
 }
 
 // The low-weight faces pass 2 listed: the reference's float sums
@@ -1001,10 +1011,10 @@ int launch_p2g(fsim_sim* s, bool fused, float dt) {
   }
   const int lgrid = std::max(1, s->num_sms * 12);
   if (fused) {
-    FSIM_LAUNCH(s, "p2g_fused", k_p2g_nodes<true>, s->n_gleaf, 256, 0, a);
+    FSIM_LAUNCH(s, "p2g_fused", k_p2g_nodes<true>, s->n_gleaf * (512 / kNodeThreads), kNodeThreads, 0, a);
     FSIM_LAUNCH(s, "p2g_low_fused", k_p2g_low<true>, lgrid, 128, 0, a);
   } else {
-    FSIM_LAUNCH(s, "p2g", k_p2g_nodes<false>, s->n_gleaf, 256, 0, a);
+    FSIM_LAUNCH(s, "p2g", k_p2g_nodes<false>, s->n_gleaf * (512 / kNodeThreads), kNodeThreads, 0, a);
     FSIM_LAUNCH(s, "p2g_low", k_p2g_low<false>, lgrid, 128, 0, a);
   }
   return FSIM_OK;
