@@ -53,26 +53,31 @@ __global__ void __launch_bounds__(256) k_g2p(const __grid_constant__ G2PArgs a) 
   const int org[3] = {lx * 8, ly * 8, lz * 8};
   __syncthreads();
   const int* n = a.lm.n;
+  const uint2 lr = a.leaf_range[s];
+  // values and on-bits of a node's three components at once, then the selects
+#pragma unroll 2
   for (int h = tid; h < 1000; h += 256) {
     const int c[3] = {org[0] - 1 + h / 100, org[1] - 1 + (h / 10) % 10, org[2] - 1 + h % 10};
+    float v[3], d[3];
+    uint32_t von[3], don[3];
 #pragma unroll
     for (int D = 0; D < 3; ++D) {
       int src[3];
       ghost_source(n, D, c, src);
       const int ns = nb[(side(src[0] - org[0]) + 1) * 9 + (side(src[1] - org[1]) + 1) * 3 +
                         (side(src[2] - org[2]) + 1)];
-      float v = 0.f, d = 0.f;
-      if (ns >= 0) {
-        const int sv = ((src[0] & 7) << 6) | ((src[1] & 7) << 3) | (src[2] & 7);
-        const int64_t base = int64_t(ns) * 1536 + D * 512 + sv;
-        if ((a.vel_on[int64_t(ns) * 16 + (sv >> 5)] >> (sv & 31)) & 1u) v = a.vel[base];
-        if ((a.vold_on[int64_t(ns) * 16 + (sv >> 5)] >> (sv & 31)) & 1u) d = a.vold[base];
-      }
-      halo[D][h] = make_float2(v, d);
+      const int sv = ((src[0] & 7) << 6) | ((src[1] & 7) << 3) | (src[2] & 7);
+      const int64_t base = int64_t(ns) * 1536 + D * 512 + sv, bits = int64_t(ns) * 16 + (sv >> 5);
+      v[D] = ns >= 0 ? a.vel[base] : 0.f;
+      d[D] = ns >= 0 ? a.vold[base] : 0.f;
+      von[D] = ns >= 0 ? a.vel_on[bits] >> (sv & 31) : 0u;
+      don[D] = ns >= 0 ? a.vold_on[bits] >> (sv & 31) : 0u;
     }
+#pragma unroll
+    for (int D = 0; D < 3; ++D)
+      halo[D][h] = make_float2((von[D] & 1u) ? v[D] : 0.f, (don[D] & 1u) ? d[D] : 0.f);
   }
   __syncthreads();
-  const uint2 lr = a.leaf_range[s];
   const int64_t cap = a.cap;
   float* P = a.part;
   for (uint32_t q = lr.x + (blockIdx.x % unsigned(a.split)) * 256u + tid; q < lr.y;
