@@ -372,8 +372,8 @@ __global__ void __launch_bounds__(kLeafTile)
 // shared memory, so two kernels do what a radix sort over all key bits takes
 // three to four passes through memory for; the old keys of a host step's rows
 // (those of appended source particles too) break ties there, instead of a
-// sort of their own before.  32.2 M rows, out of order: 630 us against 1,977
-// (two library sorts and a permutation); 52,894 rows: 22 against 57.  Bound
+// sort of their own before.  32.2 M rows, out of order: 600 us against 1,977
+// (two library sorts and a permutation); 52,894 rows: 20 against 57.  Bound
 // by the bins' traffic (18 to 26 B per row) and shared-memory atomics.
 //
 // k_bin_rows: each row's number, cell in the leaf and (OLD) old key to the
@@ -409,11 +409,10 @@ __global__ void __launch_bounds__(256)
 }
 
 // k_sort_leaf: a CTA orders a leaf's bin by (cell, old key, row): a counting
-// sort by cell into shared memory, then each cell's entries by one thread
-// (insertion; about 8 of them), or by the CTA (rank by counting) past
-// kCellSort.  keys and perm get the leaf's sorted keys and rows.
+// sort by cell into shared memory, then each entry's rank among its cell's
+// (about 8, most of them one broadcast for the warp).  keys and perm get the
+// leaf's sorted keys and rows.
 constexpr int kLeafSortThreads = 1024;
-constexpr int kCellSort = 48;
 template <bool OLD>
 using SortEntry = typename std::conditional<OLD, unsigned long long, uint32_t>::type;
 template <bool OLD>
@@ -428,7 +427,6 @@ __global__ void __launch_bounds__(kLeafSortThreads)
   E* ent = reinterpret_cast<E*>(sort_smem);  // kLeafSort entries
   __shared__ int at[512];                    // a cell's count, then its next place
   __shared__ int wsum[16];
-  __shared__ int big[kLeafSort / kCellSort], nbig;
   if (cnt[1] & kLeafOverflow) return;  // the host sorts another way
   const int np = int(cnt[1]), tid = threadIdx.x, lane = tid & 31;
   for (int s = blockIdx.x; s < np; s += gridDim.x) {
@@ -436,7 +434,6 @@ __global__ void __launch_bounds__(kLeafSortThreads)
     const int m = int(lcnt[d]);
     const uint32_t b = next[d] - uint32_t(m);  // k_bin_rows left it at the bin's end
     if (tid < 512) at[tid] = 0;
-    if (tid == 0) nbig = 0;
     __syncthreads();
     for (int j = tid; j < m; j += kLeafSortThreads) atomicAdd(&at[cell[b + j]], 1);
     __syncthreads();
@@ -469,29 +466,13 @@ __global__ void __launch_bounds__(kLeafSortThreads)
       keys[b + p] = (d << 9) | uint32_t(v);
     }
     __syncthreads();
-    if (tid < 512) {
-      if (c > kCellSort) {
-        big[atomicAdd(&nbig, 1)] = tid;
-      } else {
-        for (int x = first + 1; x < first + c; ++x) {
-          const E e = ent[x];
-          int y = x;
-          for (; y > first && ent[y - 1] > e; --y) ent[y] = ent[y - 1];
-          ent[y] = e;
-        }
-      }
-    }
-    __syncthreads();
-    for (int j = tid; j < m; j += kLeafSortThreads) perm[b + j] = uint32_t(ent[j]);
-    __syncthreads();
-    for (int q = 0; q < nbig; ++q) {
-      const int end = at[big[q]], beg = big[q] ? at[big[q] - 1] : 0;
-      for (int x = beg + tid; x < end; x += kLeafSortThreads) {
-        const E e = ent[x];
-        int rank = 0;
-        for (int y = beg; y < end; ++y) rank += ent[y] < e;
-        perm[b + beg + rank] = uint32_t(e);
-      }
+    for (int j = tid; j < m; j += kLeafSortThreads) {
+      const int v = cell[b + j], end = at[v], beg = v ? at[v - 1] : 0;
+      E e = row[b + j];
+      if constexpr (OLD) e |= static_cast<unsigned long long>(old[b + j]) << 32;
+      int rank = 0;
+      for (int y = beg; y < end; ++y) rank += ent[y] < e;
+      perm[b + beg + rank] = uint32_t(e);
     }
     __syncthreads();  // before the next leaf's counts
   }
