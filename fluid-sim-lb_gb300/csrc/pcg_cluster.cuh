@@ -4,11 +4,11 @@
 // A small system's iteration is latency: the spmv / update pair spends 6.4 to
 // 6.9 us on two launches whatever the size (24 to 160 particle leaves), and
 // the resident loop's grid barriers go through L2 as well.  Here one cluster
-// of kClCtas CTAs, one per SM, holds the whole system: a warp owns KH leaves
-// for the whole solve, a lane two z-columns of each (x-neighbours: three
+// of kClCtas CTAs, one per SM, holds the whole system: a warp owns a leaf
+// for the whole solve, a lane two of its z-columns (x-neighbours: three
 // neighbour columns are read per own column instead of four, and shared
-// memory bandwidth is what bounds the larger systems here), with r and z in
-// registers, p in shared memory and, for KH = 1, p and x in registers too.
+// memory bandwidth is what bounds the larger systems here), with r, z, p
+// and x in registers and p in shared memory too.
 // Every exchange of an iteration stays inside the cluster:
 //   S: p = z + beta p on the own columns and on the columns of other CTAs'
 //      leaves that touch them (kept here too, formed with the owner's
@@ -29,21 +29,22 @@
 // of the dot products differs.  Scalars stay off the narrow FP64 pipe: fp32
 // for FP32 (as the reference), double-float pairs for MIXED.
 // Measured us per iteration, against the pair (sphere drop; particle leaves):
-//   leaves        24          84          156         189         232
-//   FP32     2.15 / 6.57  2.65 / 6.42  3.21 / 6.51  3.43 / 6.48  5.10 / 6.66
-//   MIXED    3.58 / 10.1  4.17 / 9.32  4.88 / 9.17  5.04 / 9.51  (8.28 / 9.90)
-// (the resident loop: 5.0 to 5.5 for FP32, 7.4 to 7.7 for MIXED).  At 24 leaves it is latency (two one-way
-// pushes, four CTA barriers, six warp reductions); from about 100 on also the
-// bandwidth of shared memory.
+//   leaves        24          84          156         189
+//   FP32     2.13 / 6.57  2.62 / 6.42  3.13 / 6.51  3.36 / 6.48
+//   MIXED    3.42 / 10.1  4.06 / 9.32  4.74 / 9.17  4.92 / 9.51
+// (the resident loop: 4.3 to 4.8 for FP32, 5.7 to 6.3 for MIXED).  At 24
+// leaves it is latency (two one-way pushes, four CTA barriers, six warp
+// reductions); from about 100 on also the bandwidth of shared memory.
 //
 // The polls are bounded (kClPolls): a CTA whose wait gives up leaves the loop,
 // the other CTAs' waits run out in turn, and all meet at a last cluster
 // barrier, so no CTA's shared memory goes while another may still reach it.
 constexpr int kClCtas = 16;                       // CTAs of the cluster (one per SM)
 constexpr int kClWarps = 12;                      // warps per CTA, at most (168 registers)
-constexpr int kClPerWarp = 2;                     // leaves per warp, at most (FP32)
-constexpr int kClLeaves = 256;                    // particle leaves: FP32
-constexpr int kClLeavesMixed = kClCtas * kClWarps;  // 192: MIXED, one per warp
+// leaves per warp (written as loops over them: without, the compiler's schedule
+// takes 2.38 us per iteration at 24 leaves instead of 2.13)
+constexpr int kClPerWarp = 1;
+constexpr int kClLeaves = kClCtas * kClWarps * kClPerWarp;  // 192 particle leaves
 constexpr unsigned kClPolls = 1u << 22;
 
 // p of a CTA's leaves in shared memory (here and in the resident loop), in 16-byte chunk planes: float4 element
@@ -269,30 +270,29 @@ __device__ __forceinline__ bool cl_stop(const ClStop<float2>& q, float2 rr) {
   return !q.fixed && (rr.x < q.thr.x || (rr.x == q.thr.x && rr.y <= q.thr.y));
 }
 
-// Shared memory of a CTA with W warps of KH leaves: p of its leaves and a zero
+// Shared memory of a CTA with W warps, a leaf each: p of its leaves and a zero
 // leaf for missing neighbours, z of its leaves, the halo columns (32 per leaf:
 // -x, +x faces by y; then -y, +y faces, column x at 16 + x / 2 + 8 (x & 1) and
 // 4 further for +y, so that a lane's second column is 8 further, as in a
 // leaf) in blocks of 64 columns, all in the resident loop's chunk planes; the
 // halo's z cells ([-z, +z][64] per leaf, a lane's second 32 further); where
-// each lane's halo comes from; x (KH > 1).
+// each lane's halo comes from.
 struct ClLayout {
-  unsigned ps, zs, halo, zc, src, xs, bytes;
+  unsigned ps, zs, halo, zc, src, bytes;
 };
-__host__ __device__ inline ClLayout cl_layout(int W, int KH) {
+__host__ __device__ inline ClLayout cl_layout(int W) {
   ClLayout l;
-  const unsigned nl = unsigned(W * KH);
+  const unsigned nl = unsigned(W * kClPerWarp);
   l.ps = 0;
   l.zs = l.ps + (nl + 1) * 2048u;
   l.halo = l.zs + nl * 2048u;
   l.zc = l.halo + (nl + 1) / 2 * 2048u;
   l.src = l.zc + nl * 512u;
-  l.xs = l.src + nl * 512u;
-  l.bytes = l.xs + (KH > 1 ? nl * 2048u : 0u);
+  l.bytes = l.src + nl * 512u;
   return l;
 }
 
-template <int DM, int KH>
+template <int DM>
 __global__ void __launch_bounds__(kClWarps * 32, 1)
     k_pcg_cluster(const __grid_constant__ PcgArgs a, int per) {
   using P = PartT<DM>;
@@ -318,11 +318,10 @@ __global__ void __launch_bounds__(kClWarps * 32, 1)
   const unsigned dst_a = cl_map(src_a + rank * wa, from), dst_u = cl_map(src_u + rank * 2u * wa, from);
   src_a += from * wa;
   src_u += from * 2u * wa;
-  const ClLayout l = cl_layout(W, KH);
-  const int nl = W * KH;  // leaf places of the CTA; the last ones may be empty
+  const ClLayout l = cl_layout(W);
+  const int nl = W * kClPerWarp;  // leaf places of the CTA; the last ones may be empty
   float* const mem = reinterpret_cast<float*>(cl_mem);
   float* const zs = reinterpret_cast<float*>(cl_mem + l.zs);
-  float* const xs = reinterpret_cast<float*>(cl_mem + l.xs);
   PcgScalars* sc = a.sc;
   const int L0 = int(rank) * per;
   const int x0 = 2 * (lane >> 3), y = lane & 7;  // the lane's columns: (x0, y), (x0 + 1, y)
@@ -337,14 +336,14 @@ __global__ void __launch_bounds__(kClWarps * 32, 1)
   // memory (a leaf, halo columns or the zero leaf; float4 indices of chunk 0
   // of the first column, float indices for the z cells).  rem: bits 0 x face,
   // 1 y face, 2 -z, 3 +z come from another CTA.
-  bool own[KH];
-  int xm_i[KH], xp_i[KH], ym_i[KH], yp_i[KH], zm_i[KH], zp_i[KH];
-  unsigned rem[KH];
-  bool read[KH];  // another CTA reads the lane's z
-  uint2 f[KH][2];
-  Col<float> R[KH][2], Z[KH][2], Pc[2], X[2];  // Pc, X: KH = 1 only
+  bool own[kClPerWarp];
+  int xm_i[kClPerWarp], xp_i[kClPerWarp], ym_i[kClPerWarp], yp_i[kClPerWarp], zm_i[kClPerWarp], zp_i[kClPerWarp];
+  unsigned rem[kClPerWarp];
+  bool read[kClPerWarp];  // another CTA reads the lane's z
+  uint2 f[kClPerWarp][2];
+  Col<float> R[kClPerWarp][2], Z[kClPerWarp][2], Pc[2], X[2];
 #pragma unroll
-  for (int k = 0; k < KH; ++k) {
+  for (int k = 0; k < kClPerWarp; ++k) {
     const int j = warp + k * W;
     const int s = L0 + j;
     own[k] = j < per && s < a.n_pleaf;
@@ -413,20 +412,15 @@ __global__ void __launch_bounds__(kClWarps * 32, 1)
         make_uint4(from[0], from[1], from[2], from[3]);
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
-      if (KH == 1) {
 #pragma unroll
-        for (int z = 0; z < 8; ++z) Pc[q].v[z] = X[q].v[z] = 0.f;
-      }
+      for (int z = 0; z < 8; ++z) Pc[q].v[z] = X[q].v[z] = 0.f;
       if (own[k]) {
         const unsigned og = unsigned(s) * 512u + unsigned(((x0 + q) << 6) | (y << 3));
         f[k][q] = ldflags(a.flags, og);
         ldcol(static_cast<const float*>(a.r), og, R[k][q]);
         Col<float> p0;
         ldcol(pold, og, p0);  // zero before the first iteration
-        if (KH == 1)
-          Pc[q] = p0;
-        else
-          ps_st4(mem, ps_col4(j, x0 + q, y), p0);
+        Pc[q] = p0;
 #pragma unroll
         for (int z = 0; z < 8; ++z)
           Z[k][q].v[z] = tmul(tab[fbyte(f[k][q], z) & 15].inv, R[k][q].v[z]);
@@ -434,18 +428,18 @@ __global__ void __launch_bounds__(kClWarps * 32, 1)
       }
     }
   }
-  // KH = 1: the inverse diagonal unpacked
+  // the inverse diagonal unpacked
   float inv[2][8];
 #pragma unroll
   for (int q = 0; q < 2; ++q)
 #pragma unroll
     for (int z = 0; z < 8; ++z) inv[q][z] = tab[fbyte(f[0][q], z) & 15].inv;
   // the remote z of the halo, loaded as soon as it is published
-  Col<float> hx[KH], hy[KH][2];
-  float hz[KH][4];
+  Col<float> hx[kClPerWarp], hy[kClPerWarp][2];
+  float hz[kClPerWarp][4];
   auto load_halo = [&]() {
 #pragma unroll
-    for (int k = 0; k < KH; ++k) {
+    for (int k = 0; k < kClPerWarp; ++k) {
       if (rem[k]) {
         const uint4 from =
             reinterpret_cast<const uint4*>(cl_mem + l.src)[(warp + k * W) * 32 + lane];
@@ -492,21 +486,18 @@ __global__ void __launch_bounds__(kClWarps * 32, 1)
   while (go) {
     // S: p = z + beta p, on the own and the halo columns
 #pragma unroll
-    for (int k = 0; k < KH; ++k) {
+    for (int k = 0; k < kClPerWarp; ++k) {
       if (own[k]) {
         const int j = warp + k * W;
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
           const int mine = ps_col4(j, x0 + q, y);
           Col<float> p;
-          if (KH == 1)
-            p = Pc[q];
-          else
-            ps_ld4(mem, mine, p);
+          p = Pc[q];
 #pragma unroll
           for (int z = 0; z < 8; ++z) p.v[z] = tadd(Z[k][q].v[z], tmul(beta, p.v[z]));
           ps_st4(mem, mine, p);
-          if (KH == 1) Pc[q] = p;
+ Pc[q] = p;
         }
         if (rem[k] & 1u) halo_col(x0 == 0 ? xm_i[k] : xp_i[k], hx[k], beta);
         if (rem[k] & 2u) {
@@ -528,7 +519,7 @@ __global__ void __launch_bounds__(kClWarps * 32, 1)
     // A p in the reference's column order: -x, -y, -z, diag, +z, +y, +x
     Dot<DM> dp;
 #pragma unroll
-    for (int k = 0; k < KH; ++k) {
+    for (int k = 0; k < kClPerWarp; ++k) {
       if (own[k]) {
         const int j = warp + k * W;
         Col<float> p[2], xm, xp, ym[2], yp[2];
@@ -540,10 +531,7 @@ __global__ void __launch_bounds__(kClWarps * 32, 1)
         ps_ld4(mem, xp_i[k], xp);
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-          if (KH == 1)
-            p[q] = Pc[q];
-          else
-            ps_ld4(mem, ps_col4(j, x0 + q, y), p[q]);
+          p[q] = Pc[q];
         }
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
@@ -580,28 +568,19 @@ __global__ void __launch_bounds__(kClWarps * 32, 1)
     Dot<DM> drr, drz;
     const float nalpha = -alpha;
 #pragma unroll
-    for (int k = 0; k < KH; ++k) {
+    for (int k = 0; k < kClPerWarp; ++k) {
       if (own[k]) {
         const int j = warp + k * W;
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
           const int mine = ps_col4(j, x0 + q, y);
-          if (KH == 1) {
 #pragma unroll
-            for (int z = 0; z < 8; ++z) X[q].v[z] = tadd(tmul(alpha, Pc[q].v[z]), X[q].v[z]);
-          } else {
-            Col<float> p, x;
-            ps_ld4(mem, mine, p);
-            ps_ld4(xs, mine, x);
-#pragma unroll
-            for (int z = 0; z < 8; ++z) x.v[z] = tadd(tmul(alpha, p.v[z]), x.v[z]);
-            ps_st4(xs, mine, x);
-          }
+          for (int z = 0; z < 8; ++z) X[q].v[z] = tadd(tmul(alpha, Pc[q].v[z]), X[q].v[z]);
 #pragma unroll
           for (int z = 0; z < 8; ++z) {
             R[k][q].v[z] = tadd(tmul(nalpha, Z[k][q].v[z]), R[k][q].v[z]);
             drr.add(R[k][q].v[z], R[k][q].v[z]);
-            Z[k][q].v[z] = tmul(KH == 1 ? inv[q][z] : tab[fbyte(f[k][q], z) & 15].inv,
+            Z[k][q].v[z] = tmul(inv[q][z],
                                 R[k][q].v[z]);
             drz.add(R[k][q].v[z], Z[k][q].v[z]);
           }
@@ -628,7 +607,7 @@ __global__ void __launch_bounds__(kClWarps * 32, 1)
     sc->bar_err = 1u;
   }
 #pragma unroll
-  for (int k = 0; k < KH; ++k) {
+  for (int k = 0; k < kClPerWarp; ++k) {
     if (own[k]) {
       const int j = warp + k * W;
 #pragma unroll
@@ -636,10 +615,7 @@ __global__ void __launch_bounds__(kClWarps * 32, 1)
         const unsigned og = unsigned(L0 + j) * 512u + unsigned(((x0 + q) << 6) | (y << 3));
         const int mine = ps_col4(j, x0 + q, y);
         Col<float> v;
-        if (KH == 1)
-          v = X[q];
-        else
-          ps_ld4(xs, mine, v);
+        v = X[q];
         stcol(static_cast<float*>(a.x), og, v);
         // MIXED: the next segment continues with this search direction
         if (DM == 1 && it > it0) {
@@ -667,13 +643,9 @@ __global__ void __launch_bounds__(kClWarps * 32, 1)
 template <int DM>
 int run_cluster(fsim_sim* s, PcgArgs& a) {
   const int per = (a.n_pleaf + kClCtas - 1) / kClCtas;
-  const int KH = per <= kClWarps ? 1 : kClPerWarp;
-  const int W = (per + KH - 1) / KH;
-  const void* fn = reinterpret_cast<const void*>(k_pcg_cluster<DM, 1>);
-  if constexpr (DM == 0) {
-    if (KH > 1) fn = reinterpret_cast<const void*>(k_pcg_cluster<DM, kClPerWarp>);
-  }
-  const int most = int(cl_layout(kClWarps, KH).bytes);
+  const int W = (per + kClPerWarp - 1) / kClPerWarp;
+  const void* fn = reinterpret_cast<const void*>(k_pcg_cluster<DM>);
+  const int most = int(cl_layout(kClWarps).bytes);
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
@@ -684,7 +656,7 @@ int run_cluster(fsim_sim* s, PcgArgs& a) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kClCtas);
     cfg.blockDim = dim3(unsigned(W) * 32u);
-    cfg.dynamicSmemBytes = cl_layout(W, KH).bytes;
+    cfg.dynamicSmemBytes = cl_layout(W).bytes;
     cfg.stream = s->stream;
     cudaLaunchAttribute at = {};
     at.id = cudaLaunchAttributeClusterDimension;

@@ -29,10 +29,11 @@
 // a MIXED solve's next segment.  Barrier waits are bounded (kResPolls); a CTA
 // that gives up sets bar_err and every CTA leaves the loop
 // (FSIM_ERR_TIMEOUT), freeing its tensor memory.
-// Measured us per iteration (particle leaves; 152 SMs), against the pair:
+// Measured us per iteration (particle leaves; 152 SMs), against the pair (up
+// to eight leaves per SM by k_pcg_resident1, below):
 //   leaves        24          488        1,148       3,204       8,320
-//   FP32     4.98 / 6.56  5.60 / 8.42  6.16 / 12.5  9.09 / 18.6  15.4 / 33.0
-//   MIXED    7.45 / 10.0  7.58 / 10.7  8.26 / 13.5  11.9 / 19.7  19.9 / 36.2
+//   FP32     4.28 / 6.56  4.88 / 8.42  5.60 / 12.5  9.09 / 18.6  15.4 / 31.9
+//   MIXED    5.85 / 10.0  6.40 / 10.7  7.32 / 13.5  11.8 / 19.7  19.8 / 34.6
 // (before the fixed-point barrier FP32 took 5.90, 6.57, 6.96, 9.80 and 15.9).
 constexpr int kResWarps = 28;
 constexpr int kResThreads = kResWarps * 32;
@@ -534,17 +535,15 @@ __device__ __forceinline__ void res_face_col(const float (&v)[4], int c, Col<flo
   for (int z = 0; z < 8; ++z) out.v[z] = __shfl_sync(0xffffffffu, v[z & 3], 2 * c + (z >> 2));
 }
 
-// A p on the lane's column (xb + lx, y) of leaf s (own values P), in the
-// reference's column order; 0 off-fluid.  Called by all 32 lanes of the
-// warp together (res_faces, res_face_col).
-__device__ __forceinline__ void res_ap(const ResFrame& fr, const PcgArgs& a, const float* pm_old,
-                                       const DiagInv<float>* tab, float beta, int s, int xb, int lx,
-                                       int y, int lane, const int fs[6], const Col<float>& P,
-                                       uint2 f, Col<float>& ap) {
+// A p on the lane's column (xb + lx, y) of leaf s (own values P), with the
+// faces fv of other CTAs' leaves (res_faces) and the -z / +z face cells.
+template <typename ZL, typename ZH>
+__device__ __forceinline__ void res_stencil(const ResFrame& fr, const DiagInv<float>* tab, int s,
+                                            int xb, int lx, int y, const int fs[6],
+                                            const Col<float>& P, uint2 f, const float (&fv)[4],
+                                            ZL&& zlo, ZH&& zhi, Col<float>& ap) {
   const int x = xb + lx;
   const int own = ps_col4(s - fr.L0, x, y);
-  float fv[4];
-  res_faces(fr, a, pm_old, tab, beta, xb, fs, lane, fv);
   // one neighbour column at a time, in the reference's order: -x, -y, -z,
   // diag, +z, +y, +x
   Col<float> nc;
@@ -567,8 +566,7 @@ __device__ __forceinline__ void res_ap(const ResFrame& fr, const PcgArgs& a, con
     nc = gy;
 #pragma unroll
   for (int z = 0; z < 8; ++z) ap.v[z] = tsub(ap.v[z], nc.v[z]);
-  const float zm = res_pcell(fr, a, pm_old, tab, beta, fs[4], x, y, 7);
-  const float zp = res_pcell(fr, a, pm_old, tab, beta, fs[5], x, y, 0);
+  const float zm = zlo(), zp = zhi();
 #pragma unroll
   for (int z = 0; z < 8; ++z) {
     const uint8_t g = fbyte(f, z);
@@ -597,6 +595,19 @@ __device__ __forceinline__ void res_ap(const ResFrame& fr, const PcgArgs& a, con
   }
 }
 
+// A p on the lane's column (xb + lx, y) of leaf s (own values P), in the
+// reference's column order; 0 off-fluid.  Called by all 32 lanes of the
+// warp together (res_faces, res_face_col).
+__device__ __forceinline__ void res_ap(const ResFrame& fr, const PcgArgs& a, const float* pm_old,
+                                       const DiagInv<float>* tab, float beta, int s, int xb, int lx,
+                                       int y, int lane, const int fs[6], const Col<float>& P,
+                                       uint2 f, Col<float>& ap) {
+  float fv[4];
+  res_faces(fr, a, pm_old, tab, beta, xb, fs, lane, fv);
+  res_stencil(fr, tab, s, xb, lx, y, fs, P, f, fv,
+              [&] { return res_pcell(fr, a, pm_old, tab, beta, fs[4], xb + lx, y, 7); },
+              [&] { return res_pcell(fr, a, pm_old, tab, beta, fs[5], xb + lx, y, 0); }, ap);
+}
 // r and A p of the CTA's cells live in tensor memory (TMEM): all 512
 // columns, allocated by warp 0; warp w uses TMEM lanes 32 (w % 4) .. + 31
 // (the quarter it may access), and for its half leaf k columns (w / 4) * 32
@@ -890,6 +901,164 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(const __grid_co
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(s_taddr),
                  "r"(kResTmemCols)
                  : "memory");
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) res_finish(q, sc, it);
+}
+
+// ---- one half leaf per warp -------------------------------------------------------
+// Systems of at most kRes1Leaves leaves per SM: the same loop with every vector
+// of a lane's column in registers (no tensor memory, x and the flags not in
+// shared memory either), as many warps as the CTA has half leaves, and the
+// loads of the faces in other CTAs' leaves issued before S, whose work and CTA
+// barrier then hide part of their latency.  The operations and their order are
+// k_pcg_resident's, so the bits are too.  Bound by the iteration's chain of
+// latencies (two grid barriers, one round trip to L2 for the faces, the CTA
+// barriers).  us per iteration, FP32 and MIXED, this kernel against
+// k_pcg_resident: 488 leaves 4.88 / 5.61 and 6.40 / 7.60; 672 leaves 5.12 /
+// 5.78 and 6.84 / 7.80; 1,148 leaves (8 per SM) 5.60 / 6.07 and 7.32 / 8.17.
+// With more than 16 warps the registers no longer hold a lane's state (28
+// warps, 72 registers, 1,278 leaves: 6.55 / 6.25 and 9.34 / 8.52), so the rule
+// stops at 8 leaves per SM.
+constexpr int kRes1Warps = 16;  // 128 registers a thread
+constexpr int kRes1Leaves = kRes1Warps / 2;
+constexpr size_t kRes1Leaf = 512 * sizeof(float);  // shared memory per leaf: p
+
+template <int DM>
+__global__ void __launch_bounds__(kRes1Warps * 32, 1) k_pcg_resident1(const __grid_constant__ PcgArgs a) {
+  using P = PartT<DM>;
+  extern __shared__ __align__(16) unsigned char res_smem[];
+  float* ps = reinterpret_cast<float*>(res_smem);
+  __shared__ DiagInv<float> tab[16];
+  __shared__ int s_done;
+  __shared__ ResScalars<P> q;
+  __shared__ ResShared<P, kRes1Warps> sh;
+  PcgScalars* sc = a.sc;
+  const int G = int(gridDim.x);
+  const int per = (a.n_pleaf + G - 1) / G;  // the host checks per <= kRes1Leaves
+  ResFrame fr;
+  fr.ps = ps;
+  fr.fsm = nullptr;
+  fr.L0 = int(blockIdx.x) * per;
+  fr.nl = max(0, min(per, a.n_pleaf - fr.L0));
+  fr.n_pleaf = a.n_pleaf;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  fill_diag_table<float>(tab);
+  // partials of the warps that a smaller block does not have
+  for (int i = threadIdx.x; i < kRes1Warps; i += int(blockDim.x))
+    sh.wp[0][i] = sh.wp[1][i] = pzero<P>();
+  const bool mine = warp < 2 * fr.nl;
+  const HalfLeaf h = half_pos(2 * fr.L0 + warp, lane);
+  const int own = ps_col4(warp >> 1, h.xb + h.lx, h.cy);
+  const unsigned og = unsigned(h.s) * 512u + unsigned(h.c);
+  float* rmir = static_cast<float*>(a.r);  // during the loop: the mirror of z = M r
+  uint2 f = make_uint2(0u, 0u);
+  Col<float> p, x, r, z;
+  int fs[6] = {-1, -1, -1, -1, -1, -1};
+  bool mir = false;
+  int it = sc->iter;
+  const int it0 = it;
+  __syncthreads();  // the diagonal's table
+  if (mine) {
+    f = ldflags(a.flags, og);
+    ldcol(rmir, og, r);
+    ldcol(static_cast<const float*>((it & 1) ? a.p0 : a.p1), og, p);
+    ldcol(static_cast<const float*>(a.x), og, x);
+    face_slots(face_slot_lane(a.nbr, h.s, lane), fs);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) z.v[k] = tmul(tab[fbyte(f, k) & 15].inv, r.v[k]);
+    const bool xo = h.xb == 0 ? (h.lx == 0 && !res_local(fr, fs[0]))
+                              : (h.lx == 3 && !res_local(fr, fs[1]));
+    const bool yo = (h.cy == 0 && !res_local(fr, fs[2])) || (h.cy == 7 && !res_local(fr, fs[3]));
+    mir = xo || yo || !res_local(fr, fs[4]) || !res_local(fr, fs[5]);
+    if (mir) stcol(rmir, og, z);  // the mirror of z for the first iteration
+  }
+  if (threadIdx.x == 0) {
+    res_scalars(q, sc);
+    res_start(sh.bar, sc);
+    s_done = sc->done || it >= q.max_iter || cl_stop(q.stop, q.rr);  // PCGDriver::Solve's loop test
+  }
+  const bool zl = res_local(fr, fs[4]), zh = res_local(fr, fs[5]);
+  P* const rows = part_rows<DM>(a);
+  __syncthreads();
+  bool ok = res_first(a, sh, rows + a.maxb);
+  while (ok && !s_done) {
+    float* pm_new = static_cast<float*>((it & 1) ? a.p1 : a.p0);
+    const float* pm_old = static_cast<const float*>((it & 1) ? a.p0 : a.p1);
+    const float fbeta = q.beta;
+    Col<float> ap;
+    Dot<DM> dp;
+    float fv[4], zr0 = 0.f, zr1 = 0.f;
+    if (mine) {
+      // the remote faces: loads in flight over S
+      res_faces(fr, a, pm_old, tab, fbeta, h.xb, fs, lane, fv);
+      if (!zl) zr0 = res_pcell(fr, a, pm_old, tab, fbeta, fs[4], h.xb + h.lx, h.cy, 7);
+      if (!zh) zr1 = res_pcell(fr, a, pm_old, tab, fbeta, fs[5], h.xb + h.lx, h.cy, 0);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) p.v[k] = tadd(z.v[k], tmul(fbeta, p.v[k]));  // pnew_of's operations
+      ps_st4(ps, own, p);
+      if (mir) stcol(pm_new, og, p);
+    }
+    __syncthreads();
+    if (mine) {
+      res_stencil(fr, tab, h.s, h.xb, h.lx, h.cy, fs, p, f, fv,
+                  [&] { return zl ? ps[(ps_col4(fs[4] - fr.L0, h.xb + h.lx, h.cy) + 64) * 4 + 3] : zr0; },
+                  [&] { return zh ? ps[ps_col4(fs[5] - fr.L0, h.xb + h.lx, h.cy) * 4] : zr1; }, ap);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) dp.add(p.v[k], ap.v[k]);
+    }
+    {
+      P v[1] = {dp.pvalue()};
+      const P like[1] = {it == it0 ? q.rz : q.pAp};
+      ok = res_sync<P, 1, false>(a, v, like, sh, rows, 0, [&](const P (&tot)[1]) {
+        q.pAp = tot[0];
+        q.alpha = cl_div(q.rz, q.pAp);
+        if (!(q.alpha <= 1e5f)) {  // CHECK_LE(alpha, LARGE_FLOAT)
+          q.status = FSIM_ERR_BREAKDOWN;
+          s_done = 1;
+        }
+      });
+      if (!ok || s_done) break;
+    }
+    const float fa = q.alpha, fna = -fa;
+    Dot<DM> drr, drz;
+    if (mine) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        x.v[k] = tadd(tmul(fa, p.v[k]), x.v[k]);
+        r.v[k] = tadd(tmul(fna, ap.v[k]), r.v[k]);
+        z.v[k] = tmul(tab[fbyte(f, k) & 15].inv, r.v[k]);
+      }
+      if (mir) stcol(rmir, og, z);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        drr.add(r.v[k], r.v[k]);
+        drz.add(r.v[k], z.v[k]);
+      }
+    }
+    {
+      P v[2] = {drr.pvalue(), drz.pvalue()};
+      const P like[2] = {q.rr, q.rz};
+      ok = res_sync<P, 2, true>(a, v, like, sh, rows + a.maxb, 1, [&](const P (&tot)[2]) {
+        q.rr = tot[0];
+        q.rz_old = q.rz;
+        q.rz = tot[1];
+        q.beta = cl_div(q.rz, q.rz_old);
+        if (!(q.beta <= 1e5f)) {  // CHECK_LE(beta, LARGE_FLOAT)
+          q.status = FSIM_ERR_BREAKDOWN;
+          s_done = 1;
+        } else {
+          s_done = (it + 1 >= q.max_iter) || cl_stop(q.stop, q.rr);  // the next loop test
+        }
+      });
+      if (!ok) break;
+      ++it;
+    }
+  }
+  if (!ok && threadIdx.x == 0) q.status = FSIM_ERR_TIMEOUT;
+  // x back to global memory, and p for a MIXED solve's next segment
+  if (mine) {
+    stcol(static_cast<float*>(a.x), og, x);
+    if (DM == 1 && it > it0) stcol(static_cast<float*>((it & 1) ? a.p0 : a.p1), og, p);
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) res_finish(q, sc, it);
 }
@@ -1189,6 +1358,12 @@ int run_resident(fsim_sim* s, PcgArgs& a) {
   } else {
     fn = reinterpret_cast<void*>(k_pcg_resident<DM>);
     name = DM == 0 ? "pcg_resident" : "pcg_resident_mixed";
+    const int per = (s->n_pleaf + s->num_sms - 1) / s->num_sms;
+    if (per <= kRes1Leaves) {
+      fn = reinterpret_cast<void*>(k_pcg_resident1<DM>);
+      smem = kRes1Leaf * per;
+      threads = 64 * per;
+    }
   }
   int occ = 0;
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) !=

@@ -1,5 +1,5 @@
-"""The cluster loop: FP32 solves of at most 256 particle leaves and MIXED ones
-of at most 192 run every iteration inside one 16-CTA thread-block cluster.
+"""The cluster loop: FP32 and MIXED solves of at most 192 particle leaves run
+every iteration inside one 16-CTA thread-block cluster.
 Its element-wise arithmetic is the spmv / update pair's and its dot products
 are summed in another order, so the bars are the solver's own, as for the
 resident loop: fixed iteration counts track the oracle and the pair, relative
@@ -61,8 +61,8 @@ def _first_leaves(dims, n):
     return full[: dims[0], : dims[1], : dims[2]]
 
 
-# 1, 2: most CTAs hold nothing; 15 - 17: one and two leaves per CTA; 192:
-# MIXED's largest; 193: two leaves per warp; 256: FP32's largest; 257: past it
+# 1, 2: most CTAs hold nothing; 15 - 17: one and two leaves per CTA; 192: the
+# largest; 193 and above: past it
 @pytest.mark.parametrize("n", [1, 2, 15, 16, 17, 45, 159, 192, 193, 209, 256, 257])
 @pytest.mark.parametrize("prec", [fsim.PREC_FP32, fsim.PREC_MIXED])
 def test_tracks_the_pair_over_leaf_counts(monkeypatch, n, prec):
@@ -80,7 +80,7 @@ def test_tracks_the_pair_over_leaf_counts(monkeypatch, n, prec):
                    fsim.pcg_params(fsim.PCG_RELATIVE, prec, it, tolerance=1e-14,
                                    inner_tolerance=1e-14, max_refinements=1))
             st, cluster = _solve(sim, prm)
-            assert cluster == (res is None and n <= (256 if prec == fsim.PREC_FP32 else 192))
+            assert cluster == (res is None and n <= 192)
             assert st.iterations == it
             got[res, it] = (st.rr, sim.field(fsim.FIELD_PRESSURE)[0])
         sim.close()
