@@ -59,16 +59,19 @@ ALG_BYTES = {"pcg_spmv": 13, "pcg_update": 21, "pcg_spmv_mixed": 13, "pcg_update
              # single-reduction iteration (FSIM_PCG_CG1=1): read flags, x, p, r, w, s;
              # write x, p, r, w, s
              "pcg_cg1": 41,
-             # resident loop: the pair's fused iteration (34 B per unknown when
-             # streamed); it keeps x, r, p and the flags on chip, so its own traffic
-             # is lower (the r and p mirrors written, 8 B, and the remote halo read)
-             "pcg_resident": 34}
+             # on-chip loops (resident, cluster): the pair's fused iteration (34 B per
+             # unknown when streamed, 66 with fp64 vectors); they keep the vectors on
+             # chip, so their own traffic is lower
+             "pcg_resident": 34, "pcg_resident_mixed": 34, "pcg_resident_f64": 66,
+             "pcg_spmv_update_cluster": 34, "pcg_spmv_update_cluster_mixed": 34}
 # The same iteration in the textbook formulation, where z = M^-1 r and Ap are stored:
 #   Ap = A p and p.Ap:                read p, flags; write Ap                 =  9 B
 #   x += a p; r -= a Ap; z; r.r, r.z: read x, p, r, Ap, flags; write x, r, z  = 29 B
 #   p = z + b p:                      read z, p; write p                      = 12 B
 # (fp32 vectors), keyed by the spmv kernel of the pair.
-UNFUSED_BYTES = {"pcg_spmv": 50, "pcg_spmv_mixed": 50, "pcg_cg1": 50, "pcg_resident": 50}
+UNFUSED_BYTES = {"pcg_spmv": 50, "pcg_spmv_mixed": 50, "pcg_cg1": 50, "pcg_resident": 50,
+                 "pcg_resident_mixed": 50, "pcg_spmv_update_cluster": 50,
+                 "pcg_spmv_update_cluster_mixed": 50}
 # DRAM traffic per unknown per launch (dram__bytes_read.sum + dram__bytes_write.sum) from ncu
 # captures of `bench.py --pcg-micro`.  The fp32 pair: the 256^3 dam-break system (4,021,250
 # unknowns), host-launched loop (FSIM_PCG_GRAPH=0), caches NOT flushed between launches
@@ -96,7 +99,10 @@ PCG_PAIRS = {"pcg_spmv": "pcg_update", "pcg_update": "pcg_spmv",
              "pcg_spmv_mixed": "pcg_update_mixed", "pcg_update_mixed": "pcg_spmv_mixed",
              "pcg_spmv_f64": "pcg_update_f64", "pcg_update_f64": "pcg_spmv_f64"}
 # Kernels that are a whole PCG iteration on their own.
-PCG_SINGLE = {"pcg_cg1", "pcg_resident"}  # pcg_cg1 with its per-pass s re-forming (pcg_cg1_s), in loop_ms
+# (pcg_cg1 with its per-pass s re-forming, pcg_cg1_s, in loop_ms)
+PCG_ON_CHIP = {"pcg_resident", "pcg_resident_mixed", "pcg_resident_f64",
+               "pcg_spmv_update_cluster", "pcg_spmv_update_cluster_mixed"}
+PCG_SINGLE = {"pcg_cg1"} | PCG_ON_CHIP
 
 
 def peaks():
@@ -426,7 +432,9 @@ def roofline(res):
         loop = sum(lms)
         achieved = tot_bytes / (loop * 1e-3) / 1e9
         n_rows = float(np.mean(rws))
-        loop_form = "one cooperative launch per solve" if name == "pcg_resident" else "graph loop"
+        loop_form = ("graph loop" if name not in PCG_ON_CHIP else
+                     "one cluster launch per solve" if "cluster" in name else
+                     "one cooperative launch per solve")
         out.update(kernel="pcg_iteration (" + " + ".join(names) + ", " + loop_form + ")",
                    achieved=achieved, frac=achieved / peak, alg_bytes_per_unknown=per,
                    alg_bytes_per_launch=per * n_rows, unknowns=n_rows,
@@ -442,11 +450,11 @@ def roofline(res):
             out["traffic"] = sum(NCU_TRAFFIC_PER_UNKNOWN[k] for k in names) * n_rows
             out["traffic_source"] = (f"ncu capture ({NCU_TRAFFIC_SOURCE[names[0]]}) of "
                                      f"{' + '.join(names)}, per iteration, scaled by unknowns")
-        if name == "pcg_resident":
-            out["note"] = ("the resident loop keeps every vector of the iteration on chip (shared and "
-                           "tensor memory); achieved counts the streamed formulation's 34 B per unknown, "
+        if name in PCG_ON_CHIP:
+            out["note"] = ("the on-chip loop keeps every vector of the iteration on chip (shared and "
+                           f"tensor memory, registers); achieved counts the streamed formulation's {per} B per unknown, "
                            "so frac above 1 means the loop beats the HBM roofline of a streaming "
-                           "iteration; its own DRAM traffic is `traffic`")
+                           "iteration; its own DRAM traffic is `traffic`, where a capture has it")
         pit = sum(res["piters"])
         prow = sum(r * it for r, it in zip(res["prows"], res["piters"]))
         out["per_kernel_profiled"] = {
