@@ -324,9 +324,9 @@ struct fsim_sim {
   // fp32 solves by the single-reduction (Chronopoulos-Gear) iteration, one
   // kernel per iteration (FSIM_PCG_CG1=1; opt-in)
   int pcg_cg1 = 0;
-  // fp32 solves by the resident loop (one persistent CTA per SM holding r, p
-  // and the flags on chip): -1 by system size, 0 never, 1 wherever it fits
-  // (FSIM_PCG_RES)
+  // solves by the resident loop (one persistent CTA per SM, the vectors on
+  // chip): -1 by system size, 0 never, 1 wherever it fits, ahead of the
+  // cluster loop (FSIM_PCG_RES)
   int pcg_res = -1;
   // small FP32 and MIXED solves by one thread-block cluster (where pcg_res is
   // by size); false once a cluster launch has been refused
@@ -337,8 +337,8 @@ struct fsim_sim {
   double time = 0.0;
   uint64_t seed = 0;         // of the last seeding (source draws use it)
   int64_t source_calls = 0;  // AddContributionFromSources calls (draw stream)
-  // the next sort orders by (new key, old key): particles were appended
-  // after the sorted array (source particles)
+  // the next sort orders by (new key, old key): particles were appended after
+  // the sorted array (source particles), or uploaded out of cell order
   bool composite_sort = false;
   // regions whose particles the next advection deletes (DeleteFluidInSources)
   bool delete_in_sources = false;

@@ -11,9 +11,11 @@
 // the column order of the reference's sorted sparse rows (-x,-y,-z, diag,
 // +z,+y,+x), which makes it bit-identical to the oracle for identical p.
 //
-// Per iteration two kernels run back to back on device-resident scalars
-// (FSIM_PCG_CG1=1 runs fp32 solves by the single-reduction form below
-// instead, one kernel per iteration):
+// Systems that fit on chip run their whole loop in one launch
+// (pcg_cluster.cuh, pcg_resident.cuh; use_cluster and use_resident below).
+// For the others, per iteration two kernels run back to back on
+// device-resident scalars (FSIM_PCG_CG1=1 runs fp32 solves by the
+// single-reduction form below instead, one kernel per iteration):
 //   spmv:   head: beta_{j-1} from the previous update's r.r, r.z partials
 //           and the loop test; then p_j = z_j + beta_{j-1} p_{j-1} (z =
 //           r/diag recomputed, never stored) and p_j.(A p_j) partials.

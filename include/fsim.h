@@ -309,8 +309,9 @@ int fsim_step(fsim_t* sim, float dt, const fsim_pcg_params* params,
  * velocity upload runs while positions are binned and sorted, and the
  * position download runs during the pressure solve (positions are final
  * after the sort).  Outputs may alias the inputs of the same name.  Host
- * buffers should be pinned for full copy bandwidth.  With sources or the
- * tank boundary the three calls run in sequence. */
+ * buffers should be pinned for full copy bandwidth.  With
+ * sources the three calls run in sequence; with the tank boundary the
+ * positions come down after the step, which may delete some of them. */
 int fsim_step_host(fsim_t* sim, float dt, const fsim_pcg_params* params, const float* pos,
                    const float* vel, const float* gvel, int64_t n, float* out_pos,
                    float* out_vel, float* out_gvel, int64_t capacity, int64_t* n_out,
