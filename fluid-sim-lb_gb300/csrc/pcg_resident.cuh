@@ -32,7 +32,7 @@
 // Measured us per iteration (particle leaves; 152 SMs), against the pair (up
 // to eight leaves per SM by k_pcg_resident1, below):
 //   leaves        24          488        1,148       3,204       8,320
-//   FP32     4.28 / 6.56  4.88 / 8.42  5.60 / 12.5  9.09 / 18.6  15.4 / 31.9
+//   FP32     4.28 / 6.56  4.88 / 8.42  5.60 / 12.5  9.09 / 18.6  15.2 / 31.9
 //   MIXED    5.85 / 10.0  6.40 / 10.7  7.32 / 13.5  11.8 / 19.7  19.8 / 34.6
 // (before the fixed-point barrier FP32 took 5.90, 6.57, 6.96, 9.80 and 15.9).
 constexpr int kResWarps = 28;
@@ -536,8 +536,14 @@ __device__ __forceinline__ void res_face_col(const float (&v)[4], int c, Col<flo
 }
 
 // A p on the lane's column (xb + lx, y) of leaf s (own values P), with the
-// faces fv of other CTAs' leaves (res_faces) and the -z / +z face cells.
-template <typename ZL, typename ZH>
+// faces fv of other CTAs' leaves (res_faces) and the -z / +z face cells.  The
+// diagonal comes from the flags' bits (TABLE: from the table in shared
+// memory, the same values): 28 warps contend for shared memory more than for
+// the ALUs (us per iteration at 3,204, 4,444 and 8,320 leaves 9.19 -> 9.09,
+// 11.71 -> 11.29, 15.37 -> 15.18; MIXED 11.96 -> 11.84, 15.03 -> 14.71, 19.86
+// -> 19.76), while at one half leaf per warp the table is as fast or faster
+// (MIXED at 1,148 leaves 7.33 / 7.43).
+template <bool TABLE, typename ZL, typename ZH>
 __device__ __forceinline__ void res_stencil(const ResFrame& fr, const DiagInv<float>* tab, int s,
                                             int xb, int lx, int y, const int fs[6],
                                             const Col<float>& P, uint2 f, const float (&fv)[4],
@@ -572,7 +578,7 @@ __device__ __forceinline__ void res_stencil(const ResFrame& fr, const DiagInv<fl
     const uint8_t g = fbyte(f, z);
     const float vzm = z == 0 ? zm : P.v[(z + 7) & 7], vzp = z == 7 ? zp : P.v[(z + 1) & 7];
     ap.v[z] = tsub(ap.v[z], vzm);
-    ap.v[z] = tadd(ap.v[z], tmul(tab[g & 15].d, P.v[z]));
+    ap.v[z] = tadd(ap.v[z], tmul(TABLE ? tab[g & 15].d : cl_diag(g), P.v[z]));
     ap.v[z] = tsub(ap.v[z], vzp);
   }
   if (y < 7)
@@ -604,7 +610,7 @@ __device__ __forceinline__ void res_ap(const ResFrame& fr, const PcgArgs& a, con
                                        uint2 f, Col<float>& ap) {
   float fv[4];
   res_faces(fr, a, pm_old, tab, beta, xb, fs, lane, fv);
-  res_stencil(fr, tab, s, xb, lx, y, fs, P, f, fv,
+  res_stencil<false>(fr, tab, s, xb, lx, y, fs, P, f, fv,
               [&] { return res_pcell(fr, a, pm_old, tab, beta, fs[4], xb + lx, y, 7); },
               [&] { return res_pcell(fr, a, pm_old, tab, beta, fs[5], xb + lx, y, 0); }, ap);
 }
@@ -1000,7 +1006,7 @@ __global__ void __launch_bounds__(kRes1Warps * 32, 1) k_pcg_resident1(const __gr
     }
     __syncthreads();
     if (mine) {
-      res_stencil(fr, tab, h.s, h.xb, h.lx, h.cy, fs, p, f, fv,
+      res_stencil<true>(fr, tab, h.s, h.xb, h.lx, h.cy, fs, p, f, fv,
                   [&] { return zl ? ps[(ps_col4(fs[4] - fr.L0, h.xb + h.lx, h.cy) + 64) * 4 + 3] : zr0; },
                   [&] { return zh ? ps[ps_col4(fs[5] - fr.L0, h.xb + h.lx, h.cy) * 4] : zr1; }, ap);
 #pragma unroll
