@@ -32,8 +32,8 @@
 // Measured us per iteration (particle leaves; 152 SMs), against the pair (up
 // to eight leaves per SM by k_pcg_resident1, below):
 //   leaves        24          488        1,148       3,204       8,320
-//   FP32     4.28 / 6.56  4.88 / 8.42  5.60 / 12.5  9.09 / 18.6  15.2 / 31.9
-//   MIXED    5.85 / 10.0  6.40 / 10.7  7.32 / 13.5  11.8 / 19.7  19.8 / 34.6
+//   FP32     4.28 / 6.56  4.88 / 8.42  5.60 / 12.5  8.96 / 18.6  14.9 / 31.9
+//   MIXED    5.85 / 10.0  6.40 / 10.7  7.32 / 13.5  11.8 / 19.7  19.7 / 34.6
 // (before the fixed-point barrier FP32 took 5.90, 6.57, 6.96, 9.80 and 15.9).
 constexpr int kResWarps = 28;
 constexpr int kResThreads = kResWarps * 32;
@@ -614,6 +614,15 @@ __device__ __forceinline__ void res_ap(const ResFrame& fr, const PcgArgs& a, con
               [&] { return res_pcell(fr, a, pm_old, tab, beta, fs[4], xb + lx, y, 7); },
               [&] { return res_pcell(fr, a, pm_old, tab, beta, fs[5], xb + lx, y, 0); }, ap);
 }
+// The Jacobi inverse by flags & 15 (the table's values).  U of k_pcg_resident
+// reads it from constant memory, off the shared-memory path: most warps ask
+// for one entry (us per iteration at 3,204 and 8,320 leaves 9.09 -> 8.96 and
+// 15.19 -> 14.93; MIXED the same within 0.3%; by warp shuffles 9.04 and 15.32,
+// by a chain of selects 9.93 and 17.40).
+__constant__ float c_inv16[16] = {0.f, __builtin_inff(), 0.f, 1.0f, 0.f, 0.5f,
+                                  0.f, float(1.0 / 3.0), 0.f, 0.25f, 0.f, float(1.0 / 5.0),
+                                  0.f, float(1.0 / 6.0), 0.f, float(1.0 / 7.0)};
+
 // r and A p of the CTA's cells live in tensor memory (TMEM): all 512
 // columns, allocated by warp 0; warp w uses TMEM lanes 32 (w % 4) .. + 31
 // (the quarter it may access), and for its half leaf k columns (w / 4) * 32
@@ -845,7 +854,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(const __grid_co
           const uint8_t g = fbyte(f, z);
           R.v[z] = tadd(tmul(fna, ap[z]), R.v[z]);
           drr.add(R.v[z], R.v[z]);
-          ap[z] = tmul(tab[g & 15].inv, R.v[z]);  // z = M r, for r.z and the next S
+          ap[z] = tmul(c_inv16[g & 15], R.v[z]);  // z = M r, for r.z and the next S
           drz.add(R.v[z], ap[z]);
         }
         tmem_st8(tbase + 8u * k, R.v);
