@@ -2234,9 +2234,9 @@ int end_one_launch(fsim_sim* s, const PcgArgs& a, LoopTimer& lt) {
 
 // The cluster loop takes FP32 and MIXED solves of at most a leaf per warp of
 // its 16 CTAs, 192, unless another loop is asked for by its switch: at 189
-// leaves 3.36 us per iteration against the resident loop's 4.84 (MIXED 4.92 /
-// 6.22).  With two leaves per warp it took 5.0 to 5.1 at 227 to 238 leaves,
-// where the resident loop takes 4.7 to 4.8 (MIXED 8.3 against 6.1).  FP64 is
+// leaves 3.36 us per iteration against the resident loop's 4.2 (MIXED 4.92 /
+// 5.6).  With two leaves per warp it took 5.0 to 5.1 at 227 to 238 leaves,
+// where the resident loop takes 4.2 (MIXED 8.3 against 5.6).  FP64 is
 // bound by the FP64 pipe, which 16 SMs hold too little of.
 bool use_cluster(const fsim_sim* s, int precision) {
   return precision != FSIM_PREC_FP64 && s->pcg_res < 0 && s->pcg_cluster && s->n_pleaf > 0 &&
@@ -2247,8 +2247,8 @@ bool use_cluster(const fsim_sim* s, int precision) {
 
 // The resident loop takes every other solve that fits on chip (56 particle
 // leaves per SM, 13 for FP64): it beats the pair at all such sizes (tables in
-// pcg_resident.cuh; at one leaf per SM 4.5 against 6.5 us per iteration for
-// FP32, 5.9 / 9.2 for MIXED, 9.6 / 19.7 for FP64).  FSIM_PCG_RES=0 / 1 turns
+// pcg_resident.cuh; at one leaf per SM 4.1 against 6.5 us per iteration for
+// FP32, 5.5 / 9.2 for MIXED, 9.6 / 19.7 for FP64).  FSIM_PCG_RES=0 / 1 turns
 // it off / on ahead of the cluster loop.  FSIM_PCG_CG1=1 keeps the sizes at
 // which its loop was ever chosen, below two leaves per SM.
 bool use_resident(const fsim_sim* s, int precision) {

@@ -32,8 +32,8 @@
 // Measured us per iteration (particle leaves; 152 SMs), against the pair (up
 // to eight leaves per SM by k_pcg_resident1, below):
 //   leaves        24          488        1,148       3,204       8,320
-//   FP32     4.28 / 6.56  4.88 / 8.42  5.60 / 12.5  8.96 / 18.6  14.9 / 31.9
-//   MIXED    5.85 / 10.0  6.40 / 10.7  7.32 / 13.5  11.8 / 19.7  19.7 / 34.6
+//   FP32     4.09 / 6.56  4.43 / 8.42  5.00 / 12.5  8.96 / 18.6  14.9 / 31.9
+//   MIXED    5.57 / 10.0  5.89 / 10.7  6.73 / 13.5  11.8 / 19.7  19.7 / 34.6
 // (before the fixed-point barrier FP32 took 5.90, 6.57, 6.96, 9.80 and 15.9).
 constexpr int kResWarps = 28;
 constexpr int kResThreads = kResWarps * 32;
@@ -925,12 +925,15 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(const __grid_co
 // of a lane's column in registers (no tensor memory, x and the flags not in
 // shared memory either), as many warps as the CTA has half leaves, and the
 // loads of the faces in other CTAs' leaves issued before S, whose work and CTA
-// barrier then hide part of their latency.  The operations and their order are
-// k_pcg_resident's, so the bits are too.  Bound by the iteration's chain of
-// latencies (two grid barriers, one round trip to L2 for the faces, the CTA
-// barriers).  us per iteration, FP32 and MIXED, this kernel against
-// k_pcg_resident: 488 leaves 4.88 / 5.61 and 6.40 / 7.60; 672 leaves 5.12 /
-// 5.78 and 6.84 / 7.80; 1,148 leaves (8 per SM) 5.60 / 6.07 and 7.32 / 8.17.
+// barrier then hide part of their latency.  p of those faces stays with its
+// reader, formed from the owner's z like the owner's own p, so z is all that
+// CTAs exchange.  The operations and their order are k_pcg_resident's, so the
+// bits are too.  Bound by the iteration's chain of latencies (two grid
+// barriers, one round trip to L2 for the faces, the CTA barriers).  us per
+// iteration, FP32 and MIXED, this kernel (in brackets with p mirrored as well)
+// against k_pcg_resident: 488 leaves 4.43 (4.88) / 5.61 and 5.89 (6.40) /
+// 7.60; 672 leaves 4.60 (5.12) / 5.78 and 6.23 (6.84) / 7.80; 1,148 leaves (8
+// per SM) 5.00 (5.60) / 6.07 and 6.73 (7.32) / 8.17.
 // With more than 16 warps the registers no longer hold a lane's state (28
 // warps, 72 registers, 1,278 leaves: 6.55 / 6.25 and 9.34 / 8.52), so the rule
 // stops at 8 leaves per SM.
@@ -970,6 +973,12 @@ __global__ void __launch_bounds__(kRes1Warps * 32, 1) k_pcg_resident1(const __gr
   Col<float> p, x, r, z;
   int fs[6] = {-1, -1, -1, -1, -1, -1};
   bool mir = false;
+  // the lane's share of the half leaf's faces in other CTAs' leaves (lanes and
+  // cells as in res_faces) and its own -z / +z cells there: where the owners
+  // mirror z, and p, which stays here
+  bool face = false, zl = false, zh = false;
+  unsigned fo = 0, zo0 = 0, zo1 = 0;
+  float gp[4] = {0.f, 0.f, 0.f, 0.f}, gz0 = 0.f, gz1 = 0.f;
   int it = sc->iter;
   const int it0 = it;
   __syncthreads();  // the diagonal's table
@@ -981,10 +990,25 @@ __global__ void __launch_bounds__(kRes1Warps * 32, 1) k_pcg_resident1(const __gr
     face_slots(face_slot_lane(a.nbr, h.s, lane), fs);
 #pragma unroll
     for (int k = 0; k < 8; ++k) z.v[k] = tmul(tab[fbyte(f, k) & 15].inv, r.v[k]);
-    const bool xo = h.xb == 0 ? (h.lx == 0 && !res_local(fr, fs[0]))
-                              : (h.lx == 3 && !res_local(fr, fs[1]));
-    const bool yo = (h.cy == 0 && !res_local(fr, fs[2])) || (h.cy == 7 && !res_local(fr, fs[3]));
-    mir = xo || yo || !res_local(fr, fs[4]) || !res_local(fr, fs[5]);
+    auto far = [&](int slot) { return slot >= 0 && slot < a.n_pleaf && !res_local(fr, slot); };
+    const bool xo = h.xb == 0 ? (h.lx == 0 && far(fs[0])) : (h.lx == 3 && far(fs[1]));
+    const bool yo = (h.cy == 0 && far(fs[2])) || (h.cy == 7 && far(fs[3]));
+    zl = far(fs[4]);
+    zh = far(fs[5]);
+    mir = xo || yo || zl || zh;
+    const float* pold = static_cast<const float*>((it & 1) ? a.p0 : a.p1);
+    const int t = lane >> 1;
+    const int slot = t < 8 ? (h.xb == 0 ? fs[0] : fs[1]) : (t < 12 ? fs[2] : fs[3]);
+    face = far(slot);
+    if (face) {
+      fo = unsigned(slot) * 512u + 4u * unsigned(lane & 1) +
+           unsigned(t < 8 ? (h.xb == 0 ? 7 : 0) * 64 + t * 8
+                          : (t < 12 ? (h.xb + t - 8) * 64 + 56 : (h.xb + t - 12) * 64));
+      const float4 v = *reinterpret_cast<const float4*>(pold + fo);
+      gp[0] = v.x; gp[1] = v.y; gp[2] = v.z; gp[3] = v.w;
+    }
+    if (zl) gz0 = pold[zo0 = unsigned(fs[4]) * 512u + unsigned(h.c) + 7u];
+    if (zh) gz1 = pold[zo1 = unsigned(fs[5]) * 512u + unsigned(h.c)];
     if (mir) stcol(rmir, og, z);  // the mirror of z for the first iteration
   }
   if (threadIdx.x == 0) {
@@ -992,32 +1016,39 @@ __global__ void __launch_bounds__(kRes1Warps * 32, 1) k_pcg_resident1(const __gr
     res_start(sh.bar, sc);
     s_done = sc->done || it >= q.max_iter || cl_stop(q.stop, q.rr);  // PCGDriver::Solve's loop test
   }
-  const bool zl = res_local(fr, fs[4]), zh = res_local(fr, fs[5]);
   P* const rows = part_rows<DM>(a);
   __syncthreads();
   bool ok = res_first(a, sh, rows + a.maxb);
   while (ok && !s_done) {
-    float* pm_new = static_cast<float*>((it & 1) ? a.p1 : a.p0);
-    const float* pm_old = static_cast<const float*>((it & 1) ? a.p0 : a.p1);
     const float fbeta = q.beta;
     Col<float> ap;
     Dot<DM> dp;
-    float fv[4], zr0 = 0.f, zr1 = 0.f;
     if (mine) {
-      // the remote faces: loads in flight over S
-      res_faces(fr, a, pm_old, tab, fbeta, h.xb, fs, lane, fv);
-      if (!zl) zr0 = res_pcell(fr, a, pm_old, tab, fbeta, fs[4], h.xb + h.lx, h.cy, 7);
-      if (!zh) zr1 = res_pcell(fr, a, pm_old, tab, fbeta, fs[5], h.xb + h.lx, h.cy, 0);
+      // z of the remote faces: loads in flight over S
+      float4 zv = make_float4(0.f, 0.f, 0.f, 0.f);
+      float z0 = 0.f, z1 = 0.f;
+      if (face) zv = __ldcg(reinterpret_cast<const float4*>(rmir + fo));
+      if (zl) z0 = __ldcg(rmir + zo0);
+      if (zh) z1 = __ldcg(rmir + zo1);
 #pragma unroll
       for (int k = 0; k < 8; ++k) p.v[k] = tadd(z.v[k], tmul(fbeta, p.v[k]));  // pnew_of's operations
       ps_st4(ps, own, p);
-      if (mir) stcol(pm_new, og, p);
+      gp[0] = tadd(zv.x, tmul(fbeta, gp[0]));
+      gp[1] = tadd(zv.y, tmul(fbeta, gp[1]));
+      gp[2] = tadd(zv.z, tmul(fbeta, gp[2]));
+      gp[3] = tadd(zv.w, tmul(fbeta, gp[3]));
+      gz0 = tadd(z0, tmul(fbeta, gz0));
+      gz1 = tadd(z1, tmul(fbeta, gz1));
     }
     __syncthreads();
     if (mine) {
-      res_stencil<true>(fr, tab, h.s, h.xb, h.lx, h.cy, fs, p, f, fv,
-                  [&] { return zl ? ps[(ps_col4(fs[4] - fr.L0, h.xb + h.lx, h.cy) + 64) * 4 + 3] : zr0; },
-                  [&] { return zh ? ps[ps_col4(fs[5] - fr.L0, h.xb + h.lx, h.cy) * 4] : zr1; }, ap);
+      auto zcell = [&](int slot, float ghost, int chunk, int e) {
+        return res_local(fr, slot)
+                   ? ps[(ps_col4(slot - fr.L0, h.xb + h.lx, h.cy) + chunk) * 4 + e] : ghost;
+      };
+      res_stencil<true>(fr, tab, h.s, h.xb, h.lx, h.cy, fs, p, f, gp,
+                        [&] { return zcell(fs[4], gz0, 64, 3); },
+                        [&] { return zcell(fs[5], gz1, 0, 0); }, ap);
 #pragma unroll
       for (int k = 0; k < 8; ++k) dp.add(p.v[k], ap.v[k]);
     }
