@@ -1120,8 +1120,8 @@ __global__ void __launch_bounds__(kRes1Warps * 32, 1) k_pcg_resident1(const __gr
 // that one leaf already keeps all four schedulers busy.  All vectors are in
 // shared memory: p in 16-byte chunk planes ((leaf * 4 + chunk) * 8 + x) * 8 +
 // y, the others by unit, chunk and lane.  Measured us per iteration, against
-// the pair: 7.7 / 19.4 at 24 leaves, 13.8 / 30.4 at 488 (96^3 sphere drop), 23.0
-// / 54.2 at 1,148 (128^3), 31.6 / 81.0 at 1,784.
+// the pair: 7.1 / 19.4 at 24 leaves, 12.7 / 30.4 at 488 (96^3 sphere drop), 20.3
+// / 54.2 at 1,148 (128^3), 24.3 at 1,456.
 constexpr int kR64Warps = 16;
 constexpr int kR64Threads = kR64Warps * 32;
 constexpr int kR64Leaves = 13;
@@ -1150,31 +1150,37 @@ __device__ __forceinline__ void r64_st(double2* p, int i, int stride, const Quad
   p[i + stride] = make_double2(q.v[2], q.v[3]);
 }
 
-// p (current iteration) of four cells or one cell of leaf slot: shared memory,
-// the mirrors of z and the previous p, or zero where there is no leaf
+// p (current iteration) of four cells of leaf slot: shared memory, or the
+// given cells of another CTA's leaf.  Those a unit needs (its outward x face
+// and both y faces, 64 cells) are formed by all 32 lanes, two each, and handed
+// out by shuffles: formed where they are used they cost 16 instructions of the
+// FP64 pipe for the few lanes at the faces (us per iteration at 156, 488 and
+// 1,148 leaves 9.60 -> 8.84, 13.98 -> 12.69, 22.83 -> 20.34; with the first
+// unit's loads issued before S 8.69, 12.95, 20.73).
 struct R64Frame {
   const double2* ps;
   const double *zm, *pm;
   int L0, nl, n_pleaf;
   double beta;
 };
-__device__ __forceinline__ void r64_pquad(const R64Frame& f, int slot, int x, int y, int zh, Quad& c) {
-  if (slot >= f.L0 && slot < f.L0 + f.nl) {
-    r64_ld(f.ps, r64_col(slot - f.L0, x, y, zh), 64, c);
-  } else if (slot >= 0 && slot < f.n_pleaf) {
-    const unsigned o = unsigned(slot) * 512u + unsigned(x * 64 + y * 8 + 4 * zh);
-    Quad z;
-    const double2* zq = reinterpret_cast<const double2*>(f.zm + o);
-    const double2* pq = reinterpret_cast<const double2*>(f.pm + o);
-    quad_set(z, __ldcg(zq), __ldcg(zq + 1));
-    quad_set(c, __ldcg(pq), __ldcg(pq + 1));
-#pragma unroll
-    for (int k = 0; k < 4; ++k) c.v[k] = __fma_rn(f.beta, c.v[k], z.v[k]);
-  } else {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) c.v[k] = 0.0;
-  }
+__device__ __forceinline__ bool r64_local(const R64Frame& f, int slot) {
+  return slot >= f.L0 && slot < f.L0 + f.nl;
 }
+__device__ __forceinline__ void r64_pquad(const R64Frame& f, int slot, int x, int y, int zh,
+                                          const Quad& ghost, Quad& c) {
+  if (r64_local(f, slot))
+    r64_ld(f.ps, r64_col(slot - f.L0, x, y, zh), 64, c);
+  else
+    c = ghost;
+}
+// one cell of another CTA's leaf, from the mirrors; 0 where the CTA has the
+// leaf or there is none
+__device__ __forceinline__ double r64_far(const R64Frame& f, int slot, unsigned o) {
+  if (slot < 0 || slot >= f.n_pleaf || r64_local(f, slot)) return 0.0;
+  o += unsigned(slot) * 512u;
+  return __fma_rn(f.beta, __ldcg(f.pm + o), __ldcg(f.zm + o));
+}
+// p of cell z of column (x, y) of leaf slot
 __device__ __forceinline__ double r64_pcell(const R64Frame& f, int slot, int x, int y, int z) {
   if (slot >= f.L0 && slot < f.L0 + f.nl) {
     const double2 v = f.ps[r64_col(slot - f.L0, x, y, 0) + (z >> 1) * 64];
@@ -1295,9 +1301,19 @@ __global__ void __launch_bounds__(kR64Threads, 1) k_pcg_resident64(const __grid_
       const int s = fr.L0 + t.j, x = t.x, y = t.y;
       const int* nb = nbs[t.j];
       const unsigned f = flags4(t);
-      Quad p, w, c;
-      r64_pquad(fr, x > 0 ? s : nb[0], (x + 7) & 7, y, t.zh, w);
-      r64_pquad(fr, y > 0 ? s : nb[2], x, (y + 7) & 7, t.zh, c);
+      const int xb = x & 4, cell = 4 * t.zh + (lane & 3);
+      const double gx = r64_far(fr, xb ? nb[1] : nb[0],
+                                unsigned((xb ? 0 : 448) + (lane >> 2) * 8 + cell));
+      const double gy = r64_far(fr, lane < 16 ? nb[2] : nb[3],
+                                unsigned((xb + ((lane >> 2) & 3)) * 64 + (lane < 16 ? 56 : 0) + cell));
+      Quad p, w, c, fx, fy;
+#pragma unroll
+      for (int z = 0; z < 4; ++z) {
+        fx.v[z] = __shfl_sync(0xffffffffu, gx, 4 * y + z);
+        fy.v[z] = __shfl_sync(0xffffffffu, gy, (y == 0 ? 0 : 16) + 4 * (x & 3) + z);
+      }
+      r64_pquad(fr, x > 0 ? s : nb[0], (x + 7) & 7, y, t.zh, fx, w);
+      r64_pquad(fr, y > 0 ? s : nb[2], x, (y + 7) & 7, t.zh, fy, c);
 #pragma unroll
       for (int z = 0; z < 4; ++z) w.v[z] = __dsub_rn(-w.v[z], c.v[z]);
       r64_ld(ps, r64_col(t.j, x, y, t.zh), 64, p);
@@ -1309,10 +1325,10 @@ __global__ void __launch_bounds__(kR64Threads, 1) k_pcg_resident64(const __grid_
         w.v[z] = __fma_rn(tab[(f >> (8 * z)) & 15].d, p.v[z], w.v[z]);
         w.v[z] = __dsub_rn(w.v[z], z == 3 ? zp : p.v[(z + 1) & 3]);
       }
-      r64_pquad(fr, y < 7 ? s : nb[3], x, (y + 1) & 7, t.zh, c);
+      r64_pquad(fr, y < 7 ? s : nb[3], x, (y + 1) & 7, t.zh, fy, c);
 #pragma unroll
       for (int z = 0; z < 4; ++z) w.v[z] = __dsub_rn(w.v[z], c.v[z]);
-      r64_pquad(fr, x < 7 ? s : nb[1], (x + 1) & 7, y, t.zh, c);
+      r64_pquad(fr, x < 7 ? s : nb[1], (x + 1) & 7, y, t.zh, fx, c);
 #pragma unroll
       for (int z = 0; z < 4; ++z) {
         w.v[z] = ((f >> (8 * z)) & 1u) ? __dsub_rn(w.v[z], c.v[z]) : 0.0;
