@@ -2248,7 +2248,7 @@ bool use_cluster(const fsim_sim* s, int precision) {
 // The resident loop takes every other solve that fits on chip (56 particle
 // leaves per SM, 13 for FP64): it beats the pair at all such sizes (tables in
 // pcg_resident.cuh; at one leaf per SM 4.1 against 6.5 us per iteration for
-// FP32, 5.5 / 9.2 for MIXED, 9.6 / 19.7 for FP64).  FSIM_PCG_RES=0 / 1 turns
+// FP32, 5.5 / 9.2 for MIXED, 8.9 / 19.7 for FP64).  FSIM_PCG_RES=0 / 1 turns
 // it off / on ahead of the cluster loop.  FSIM_PCG_CG1=1 keeps the sizes at
 // which its loop was ever chosen, below two leaves per SM.
 bool use_resident(const fsim_sim* s, int precision) {

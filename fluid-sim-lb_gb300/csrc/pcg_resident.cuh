@@ -1120,7 +1120,7 @@ __global__ void __launch_bounds__(kRes1Warps * 32, 1) k_pcg_resident1(const __gr
 // that one leaf already keeps all four schedulers busy.  All vectors are in
 // shared memory: p in 16-byte chunk planes ((leaf * 4 + chunk) * 8 + x) * 8 +
 // y, the others by unit, chunk and lane.  Measured us per iteration, against
-// the pair: 7.1 / 19.4 at 24 leaves, 12.7 / 30.4 at 488 (96^3 sphere drop), 20.3
+// the pair: 7.5 / 19.4 at 24 leaves, 12.7 / 30.4 at 488 (96^3 sphere drop), 20.3
 // / 54.2 at 1,148 (128^3), 24.3 at 1,456.
 constexpr int kR64Warps = 16;
 constexpr int kR64Threads = kR64Warps * 32;
