@@ -29,11 +29,11 @@
 // a MIXED solve's next segment.  Barrier waits are bounded (kResPolls); a CTA
 // that gives up sets bar_err and every CTA leaves the loop
 // (FSIM_ERR_TIMEOUT), freeing its tensor memory.
-// Measured us per iteration (particle leaves; 152 SMs), against the pair (up
-// to eight leaves per SM by k_pcg_resident1, below):
+// Measured us per iteration (particle leaves; 152 SMs), against the pair (the
+// first three columns by k_pcg_resident1, below):
 //   leaves        24          488        1,148       3,204       8,320
-//   FP32     4.09 / 6.56  4.43 / 8.42  5.00 / 12.5  8.96 / 18.6  14.9 / 31.9
-//   MIXED    5.57 / 10.0  5.89 / 10.7  6.73 / 13.5  11.8 / 19.7  19.7 / 34.6
+//   FP32     4.12 / 6.56  4.33 / 8.42  4.73 / 12.5  8.96 / 18.6  14.9 / 31.9
+//   MIXED    5.59 / 10.0  5.78 / 10.7  6.42 / 13.5  11.8 / 19.7  19.7 / 34.6
 // (before the fixed-point barrier FP32 took 5.90, 6.57, 6.96, 9.80 and 15.9).
 constexpr int kResWarps = 28;
 constexpr int kResThreads = kResWarps * 32;
@@ -920,28 +920,29 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(const __grid_co
   if (blockIdx.x == 0 && threadIdx.x == 0) res_finish(q, sc, it);
 }
 
-// ---- one half leaf per warp -------------------------------------------------------
-// Systems of at most kRes1Leaves leaves per SM: the same loop with every vector
-// of a lane's column in registers (no tensor memory, x and the flags not in
-// shared memory either), as many warps as the CTA has half leaves, and the
-// loads of the faces in other CTAs' leaves issued before S, whose work and CTA
-// barrier then hide part of their latency.  p of those faces stays with its
+// ---- one or two half leaves per warp -------------------------------------------
+// Systems of at most KH kRes1Leaves leaves per SM, KH half leaves per warp: the
+// same loop with the vectors of a lane's columns in registers (no tensor
+// memory; x in shared memory for KH = 2), and the loads of the faces in other
+// CTAs' leaves issued before S, whose work and CTA barrier then hide part of
+// their latency.  p of those faces stays with its
 // reader, formed from the owner's z like the owner's own p, so z is all that
 // CTAs exchange.  The operations and their order are k_pcg_resident's, so the
 // bits are too.  Bound by the iteration's chain of latencies (two grid
 // barriers, one round trip to L2 for the faces, the CTA barriers).  us per
-// iteration, FP32 and MIXED, this kernel (in brackets with p mirrored as well)
-// against k_pcg_resident: 488 leaves 4.43 (4.88) / 5.61 and 5.89 (6.40) /
-// 7.60; 672 leaves 4.60 (5.12) / 5.78 and 6.23 (6.84) / 7.80; 1,148 leaves (8
-// per SM) 5.00 (5.60) / 6.07 and 6.73 (7.32) / 8.17.
-// With more than 16 warps the registers no longer hold a lane's state (28
-// warps, 72 registers, 1,278 leaves: 6.55 / 6.25 and 9.34 / 8.52), so the rule
-// stops at 8 leaves per SM.
+// iteration against k_pcg_resident, FP32 and MIXED (leaves per SM):
+//   KH = 1   488 (4): 4.33 / 5.61, 5.78 / 7.60   1,148 (8): 4.73 / 6.07, 6.42 / 8.17
+//   KH = 2   1,278 (9): 5.99 / 6.23, 8.62 / 8.42   1,456 (10): 6.01 / 6.40, 8.63 / 8.54
+//            1,584 (11): 6.09 / 6.55, 8.73 / 8.89   1,920 (13): 6.23 / 6.92, 8.97 / 9.37
+// (with p mirrored as well, KH = 1 took 4.88 and 6.40, 5.60 and 7.32).  MIXED
+// spills a little with KH = 2, so it takes it from 11 leaves per SM on.  More
+// than 16 warps leave too few registers (28 warps of 72, KH = 1, 1,278 leaves:
+// 6.55 and 9.34).
 constexpr int kRes1Warps = 16;  // 128 registers a thread
 constexpr int kRes1Leaves = kRes1Warps / 2;
 constexpr size_t kRes1Leaf = 512 * sizeof(float);  // shared memory per leaf: p
 
-template <int DM>
+template <int DM, int KH>
 __global__ void __launch_bounds__(kRes1Warps * 32, 1) k_pcg_resident1(const __grid_constant__ PcgArgs a) {
   using P = PartT<DM>;
   extern __shared__ __align__(16) unsigned char res_smem[];
@@ -952,7 +953,8 @@ __global__ void __launch_bounds__(kRes1Warps * 32, 1) k_pcg_resident1(const __gr
   __shared__ ResShared<P, kRes1Warps> sh;
   PcgScalars* sc = a.sc;
   const int G = int(gridDim.x);
-  const int per = (a.n_pleaf + G - 1) / G;  // the host checks per <= kRes1Leaves
+  const int per = (a.n_pleaf + G - 1) / G;  // the host checks per <= KH * kRes1Leaves
+  float4* const xs = reinterpret_cast<float4*>(res_smem + kRes1Leaf * per);  // x, KH > 1
   ResFrame fr;
   fr.ps = ps;
   fr.fsm = nullptr;
@@ -964,52 +966,69 @@ __global__ void __launch_bounds__(kRes1Warps * 32, 1) k_pcg_resident1(const __gr
   // partials of the warps that a smaller block does not have
   for (int i = threadIdx.x; i < kRes1Warps; i += int(blockDim.x))
     sh.wp[0][i] = sh.wp[1][i] = pzero<P>();
-  const bool mine = warp < 2 * fr.nl;
-  const HalfLeaf h = half_pos(2 * fr.L0 + warp, lane);
-  const int own = ps_col4(warp >> 1, h.xb + h.lx, h.cy);
-  const unsigned og = unsigned(h.s) * 512u + unsigned(h.c);
+  // the warp's half leaf k: half leaf warp + k W of the CTA
+  const int W = int(blockDim.x) >> 5;
+  auto has = [&](int k) { return warp + k * W < 2 * fr.nl; };
+  auto half = [&](int k) { return half_pos(2 * fr.L0 + warp + k * W, lane); };
   float* rmir = static_cast<float*>(a.r);  // during the loop: the mirror of z = M r
-  uint2 f = make_uint2(0u, 0u);
-  Col<float> p, x, r, z;
-  int fs[6] = {-1, -1, -1, -1, -1, -1};
-  bool mir = false;
+  uint2 f[KH];
+  Col<float> p[KH], x[1], r[KH], z[KH];  // z: A p from the stencil to U
+  int fs[KH][6];
+  bool mir[KH];
   // the lane's share of the half leaf's faces in other CTAs' leaves (lanes and
   // cells as in res_faces) and its own -z / +z cells there: where the owners
   // mirror z, and p, which stays here
-  bool face = false, zl = false, zh = false;
-  unsigned fo = 0, zo0 = 0, zo1 = 0;
-  float gp[4] = {0.f, 0.f, 0.f, 0.f}, gz0 = 0.f, gz1 = 0.f;
+  bool face[KH], zl[KH], zh[KH];
+  unsigned fo[KH];
+  float gp[KH][4], gz0[KH], gz1[KH];
+  auto zo0 = [&](int k, const HalfLeaf& h) { return unsigned(fs[k][4]) * 512u + unsigned(h.c) + 7u; };
+  auto zo1 = [&](int k, const HalfLeaf& h) { return unsigned(fs[k][5]) * 512u + unsigned(h.c); };
   int it = sc->iter;
   const int it0 = it;
   __syncthreads();  // the diagonal's table
-  if (mine) {
-    f = ldflags(a.flags, og);
-    ldcol(rmir, og, r);
-    ldcol(static_cast<const float*>((it & 1) ? a.p0 : a.p1), og, p);
-    ldcol(static_cast<const float*>(a.x), og, x);
-    face_slots(face_slot_lane(a.nbr, h.s, lane), fs);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) z.v[k] = tmul(tab[fbyte(f, k) & 15].inv, r.v[k]);
-    auto far = [&](int slot) { return slot >= 0 && slot < a.n_pleaf && !res_local(fr, slot); };
-    const bool xo = h.xb == 0 ? (h.lx == 0 && far(fs[0])) : (h.lx == 3 && far(fs[1]));
-    const bool yo = (h.cy == 0 && far(fs[2])) || (h.cy == 7 && far(fs[3]));
-    zl = far(fs[4]);
-    zh = far(fs[5]);
-    mir = xo || yo || zl || zh;
-    const float* pold = static_cast<const float*>((it & 1) ? a.p0 : a.p1);
-    const int t = lane >> 1;
-    const int slot = t < 8 ? (h.xb == 0 ? fs[0] : fs[1]) : (t < 12 ? fs[2] : fs[3]);
-    face = far(slot);
-    if (face) {
-      fo = unsigned(slot) * 512u + 4u * unsigned(lane & 1) +
-           unsigned(t < 8 ? (h.xb == 0 ? 7 : 0) * 64 + t * 8
-                          : (t < 12 ? (h.xb + t - 8) * 64 + 56 : (h.xb + t - 12) * 64));
-      const float4 v = *reinterpret_cast<const float4*>(pold + fo);
-      gp[0] = v.x; gp[1] = v.y; gp[2] = v.z; gp[3] = v.w;
+  for (int k = 0; k < KH; ++k) {
+    face[k] = zl[k] = zh[k] = mir[k] = false;
+    fo[k] = 0;
+    gz0[k] = gz1[k] = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) gp[k][e] = 0.f;
+    f[k] = make_uint2(0u, 0u);
+    if (has(k)) {
+      const HalfLeaf h = half(k);
+      const unsigned og = unsigned(h.s) * 512u + unsigned(h.c);
+      const float* pold = static_cast<const float*>((it & 1) ? a.p0 : a.p1);
+      f[k] = ldflags(a.flags, og);
+      ldcol(rmir, og, r[k]);
+      ldcol(pold, og, p[k]);
+      ldcol(static_cast<const float*>(a.x), og, x[0]);
+      if (KH > 1) {
+        xs[((k * kRes1Warps + warp) * 2 + 0) * 32 + lane] = make_float4(x[0].v[0], x[0].v[1], x[0].v[2], x[0].v[3]);
+        xs[((k * kRes1Warps + warp) * 2 + 1) * 32 + lane] = make_float4(x[0].v[4], x[0].v[5], x[0].v[6], x[0].v[7]);
+      }
+      face_slots(face_slot_lane(a.nbr, h.s, lane), fs[k]);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) z[k].v[e] = tmul(tab[fbyte(f[k], e) & 15].inv, r[k].v[e]);
+      auto far = [&](int slot) { return slot >= 0 && slot < a.n_pleaf && !res_local(fr, slot); };
+      const bool xo = h.xb == 0 ? (h.lx == 0 && far(fs[k][0])) : (h.lx == 3 && far(fs[k][1]));
+      const bool yo = (h.cy == 0 && far(fs[k][2])) || (h.cy == 7 && far(fs[k][3]));
+      zl[k] = far(fs[k][4]);
+      zh[k] = far(fs[k][5]);
+      mir[k] = xo || yo || zl[k] || zh[k];
+      const int t = lane >> 1;
+      const int slot = t < 8 ? (h.xb == 0 ? fs[k][0] : fs[k][1]) : (t < 12 ? fs[k][2] : fs[k][3]);
+      face[k] = far(slot);
+      if (face[k]) {
+        fo[k] = unsigned(slot) * 512u + 4u * unsigned(lane & 1) +
+                unsigned(t < 8 ? (h.xb == 0 ? 7 : 0) * 64 + t * 8
+                               : (t < 12 ? (h.xb + t - 8) * 64 + 56 : (h.xb + t - 12) * 64));
+        const float4 v = *reinterpret_cast<const float4*>(pold + fo[k]);
+        gp[k][0] = v.x; gp[k][1] = v.y; gp[k][2] = v.z; gp[k][3] = v.w;
+      }
+      if (zl[k]) gz0[k] = pold[zo0(k, h)];
+      if (zh[k]) gz1[k] = pold[zo1(k, h)];
+      if (mir[k]) stcol(rmir, og, z[k]);  // the mirror of z for the first iteration
     }
-    if (zl) gz0 = pold[zo0 = unsigned(fs[4]) * 512u + unsigned(h.c) + 7u];
-    if (zh) gz1 = pold[zo1 = unsigned(fs[5]) * 512u + unsigned(h.c)];
-    if (mir) stcol(rmir, og, z);  // the mirror of z for the first iteration
   }
   if (threadIdx.x == 0) {
     res_scalars(q, sc);
@@ -1021,36 +1040,54 @@ __global__ void __launch_bounds__(kRes1Warps * 32, 1) k_pcg_resident1(const __gr
   bool ok = res_first(a, sh, rows + a.maxb);
   while (ok && !s_done) {
     const float fbeta = q.beta;
-    Col<float> ap;
     Dot<DM> dp;
-    if (mine) {
-      // z of the remote faces: loads in flight over S
-      float4 zv = make_float4(0.f, 0.f, 0.f, 0.f);
-      float z0 = 0.f, z1 = 0.f;
-      if (face) zv = __ldcg(reinterpret_cast<const float4*>(rmir + fo));
-      if (zl) z0 = __ldcg(rmir + zo0);
-      if (zh) z1 = __ldcg(rmir + zo1);
+    // z of the remote faces: loads in flight over S
+    float4 zv[KH];
+    float z0[KH], z1[KH];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) p.v[k] = tadd(z.v[k], tmul(fbeta, p.v[k]));  // pnew_of's operations
-      ps_st4(ps, own, p);
-      gp[0] = tadd(zv.x, tmul(fbeta, gp[0]));
-      gp[1] = tadd(zv.y, tmul(fbeta, gp[1]));
-      gp[2] = tadd(zv.z, tmul(fbeta, gp[2]));
-      gp[3] = tadd(zv.w, tmul(fbeta, gp[3]));
-      gz0 = tadd(z0, tmul(fbeta, gz0));
-      gz1 = tadd(z1, tmul(fbeta, gz1));
+    for (int k = 0; k < KH; ++k) {
+      zv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      z0[k] = z1[k] = 0.f;
+      if (has(k)) {
+        const HalfLeaf h = half(k);
+        if (face[k]) zv[k] = __ldcg(reinterpret_cast<const float4*>(rmir + fo[k]));
+        if (zl[k]) z0[k] = __ldcg(rmir + zo0(k, h));
+        if (zh[k]) z1[k] = __ldcg(rmir + zo1(k, h));
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < KH; ++k) {
+      if (has(k)) {
+        const HalfLeaf h = half(k);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) p[k].v[e] = tadd(z[k].v[e], tmul(fbeta, p[k].v[e]));  // pnew_of's operations
+        ps_st4(ps, ps_col4(h.s - fr.L0, h.xb + h.lx, h.cy), p[k]);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < KH; ++k) {
+      gp[k][0] = tadd(zv[k].x, tmul(fbeta, gp[k][0]));
+      gp[k][1] = tadd(zv[k].y, tmul(fbeta, gp[k][1]));
+      gp[k][2] = tadd(zv[k].z, tmul(fbeta, gp[k][2]));
+      gp[k][3] = tadd(zv[k].w, tmul(fbeta, gp[k][3]));
+      gz0[k] = tadd(z0[k], tmul(fbeta, gz0[k]));
+      gz1[k] = tadd(z1[k], tmul(fbeta, gz1[k]));
     }
     __syncthreads();
-    if (mine) {
-      auto zcell = [&](int slot, float ghost, int chunk, int e) {
-        return res_local(fr, slot)
-                   ? ps[(ps_col4(slot - fr.L0, h.xb + h.lx, h.cy) + chunk) * 4 + e] : ghost;
-      };
-      res_stencil<true>(fr, tab, h.s, h.xb, h.lx, h.cy, fs, p, f, gp,
-                        [&] { return zcell(fs[4], gz0, 64, 3); },
-                        [&] { return zcell(fs[5], gz1, 0, 0); }, ap);
 #pragma unroll
-      for (int k = 0; k < 8; ++k) dp.add(p.v[k], ap.v[k]);
+    for (int k = 0; k < KH; ++k) {
+      if (has(k)) {
+        const HalfLeaf h = half(k);
+        auto zcell = [&](int slot, float ghost, int chunk, int e) {
+          return res_local(fr, slot)
+                     ? ps[(ps_col4(slot - fr.L0, h.xb + h.lx, h.cy) + chunk) * 4 + e] : ghost;
+        };
+        res_stencil<true>(fr, tab, h.s, h.xb, h.lx, h.cy, fs[k], p[k], f[k], gp[k],
+                          [&] { return zcell(fs[k][4], gz0[k], 64, 3); },
+                          [&] { return zcell(fs[k][5], gz1[k], 0, 0); }, z[k]);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) dp.add(p[k].v[e], z[k].v[e]);
+      }
     }
     {
       P v[1] = {dp.pvalue()};
@@ -1067,18 +1104,32 @@ __global__ void __launch_bounds__(kRes1Warps * 32, 1) k_pcg_resident1(const __gr
     }
     const float fa = q.alpha, fna = -fa;
     Dot<DM> drr, drz;
-    if (mine) {
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        x.v[k] = tadd(tmul(fa, p.v[k]), x.v[k]);
-        r.v[k] = tadd(tmul(fna, ap.v[k]), r.v[k]);
-        z.v[k] = tmul(tab[fbyte(f, k) & 15].inv, r.v[k]);
-      }
-      if (mir) stcol(rmir, og, z);
+    for (int k = 0; k < KH; ++k) {
+      if (has(k)) {
+        const HalfLeaf h = half(k);
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        drr.add(r.v[k], r.v[k]);
-        drz.add(r.v[k], z.v[k]);
+        for (int e = 0; e < 8; ++e) {
+          r[k].v[e] = tadd(tmul(fna, z[k].v[e]), r[k].v[e]);
+          z[k].v[e] = tmul(tab[fbyte(f[k], e) & 15].inv, r[k].v[e]);
+        }
+        if (mir[k]) stcol(rmir, unsigned(h.s) * 512u + unsigned(h.c), z[k]);
+        if (KH > 1) {
+          float4* const q0 = xs + ((k * kRes1Warps + warp) * 2 + 0) * 32 + lane;
+          const float4 u = q0[0], w = q0[32];
+          q0[0] = make_float4(tadd(tmul(fa, p[k].v[0]), u.x), tadd(tmul(fa, p[k].v[1]), u.y),
+                              tadd(tmul(fa, p[k].v[2]), u.z), tadd(tmul(fa, p[k].v[3]), u.w));
+          q0[32] = make_float4(tadd(tmul(fa, p[k].v[4]), w.x), tadd(tmul(fa, p[k].v[5]), w.y),
+                               tadd(tmul(fa, p[k].v[6]), w.z), tadd(tmul(fa, p[k].v[7]), w.w));
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) x[0].v[e] = tadd(tmul(fa, p[k].v[e]), x[0].v[e]);
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          drr.add(r[k].v[e], r[k].v[e]);
+          drz.add(r[k].v[e], z[k].v[e]);
+        }
       }
     }
     {
@@ -1102,9 +1153,20 @@ __global__ void __launch_bounds__(kRes1Warps * 32, 1) k_pcg_resident1(const __gr
   }
   if (!ok && threadIdx.x == 0) q.status = FSIM_ERR_TIMEOUT;
   // x back to global memory, and p for a MIXED solve's next segment
-  if (mine) {
-    stcol(static_cast<float*>(a.x), og, x);
-    if (DM == 1 && it > it0) stcol(static_cast<float*>((it & 1) ? a.p0 : a.p1), og, p);
+#pragma unroll
+  for (int k = 0; k < KH; ++k) {
+    if (has(k)) {
+      const HalfLeaf h = half(k);
+      const unsigned og = unsigned(h.s) * 512u + unsigned(h.c);
+      if (KH > 1) {
+        const float4 u = xs[((k * kRes1Warps + warp) * 2 + 0) * 32 + lane],
+                     w = xs[((k * kRes1Warps + warp) * 2 + 1) * 32 + lane];
+        x[0].v[0] = u.x; x[0].v[1] = u.y; x[0].v[2] = u.z; x[0].v[3] = u.w;
+        x[0].v[4] = w.x; x[0].v[5] = w.y; x[0].v[6] = w.z; x[0].v[7] = w.w;
+      }
+      stcol(static_cast<float*>(a.x), og, x[0]);
+      if (DM == 1 && it > it0) stcol(static_cast<float*>((it & 1) ? a.p0 : a.p1), og, p[k]);
+    }
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) res_finish(q, sc, it);
 }
@@ -1422,9 +1484,13 @@ int run_resident(fsim_sim* s, PcgArgs& a) {
     name = DM == 0 ? "pcg_resident" : "pcg_resident_mixed";
     const int per = (s->n_pleaf + s->num_sms - 1) / s->num_sms;
     if (per <= kRes1Leaves) {
-      fn = reinterpret_cast<void*>(k_pcg_resident1<DM>);
+      fn = reinterpret_cast<void*>(k_pcg_resident1<DM, 1>);
       smem = kRes1Leaf * per;
       threads = 64 * per;
+    } else if (per <= 2 * kRes1Leaves && per >= (DM == 0 ? 0 : 11)) {
+      fn = reinterpret_cast<void*>(k_pcg_resident1<DM, 2>);
+      smem = kRes1Leaf * per + size_t(2 * kRes1Warps) * 256 * sizeof(float);
+      threads = 32 * kRes1Warps;
     }
   }
   int occ = 0;

@@ -1,6 +1,7 @@
-"""The resident loop's two kernels for fp32 vectors, around the size where one
-takes over from the other: up to eight leaves per SM a warp holds one half
-leaf in registers, above that up to four in tensor and shared memory.  Fixed
+"""The resident loop's kernels for fp32 vectors, around the sizes where one
+takes over from another: up to eight leaves per SM a warp holds one half leaf
+in registers, up to sixteen two (MIXED from eleven on), above that up to four
+in tensor and shared memory.  Fixed
 iteration counts against the spmv / update pair, whose element-wise operations
 are the same; only the order of the dot products' sums differs."""
 import numpy as np
@@ -13,8 +14,9 @@ from test_gpu_pcg_cluster import _first_leaves, _system
 pytestmark = pytest.mark.gpu
 
 
-# leaves per SM on 152 SMs: 2, 8 (one CTA short of a leaf, then all full), 9, 14, 15
-@pytest.mark.parametrize("n", [300, 1215, 1216, 1217, 2128, 2200])
+# leaves per SM on 152 SMs: 2, 8 (one CTA short of a leaf, then all full), 9, 10,
+# 11, 14, 15, 16, 17
+@pytest.mark.parametrize("n", [300, 1215, 1216, 1217, 1520, 1521, 2128, 2200, 2432, 2433])
 @pytest.mark.parametrize("prec", [fsim.PREC_FP32, fsim.PREC_MIXED])
 def test_tracks_the_pair(monkeypatch, n, prec):
     dims = (125, 120, 88)
