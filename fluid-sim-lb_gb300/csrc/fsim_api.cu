@@ -944,7 +944,8 @@ int step_moved(fsim_sim* s, float dt, const fsim_pcg_params* prm, fsim_step_stat
   fsim_pcg_stats ps;
   std::memset(&ps, 0, sizeof(ps));
   // the rest of the step does not need the solve's report: it is read with
-  // the CFL maximum
+  // the CFL maximum (where the solve gave up, the kernels in between return
+  // without a write)
   if ((rc = pcg_solve(s, prm, &ps, nullptr, true))) return rc;
   s->pres_valid = true;
   if ((rc = launch_pressure_update(s, true))) return rc;
@@ -952,7 +953,10 @@ int step_moved(fsim_sim* s, float dt, const fsim_pcg_params* prm, fsim_step_stat
   if ((rc = launch_g2p(s))) return rc;
   float vmax = 0.f;
   if ((rc = read_vmax(s, &vmax))) return rc;
-  if ((rc = pcg_collect(s, prm, &ps))) return rc;
+  if ((rc = pcg_collect(s, prm, &ps))) {
+    s->pres_valid = s->extrapolated = false;
+    return rc;
+  }
   if (st) {
     std::memset(st, 0, sizeof(*st));
     int64_t cnt = 0;

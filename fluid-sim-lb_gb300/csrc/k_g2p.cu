@@ -32,6 +32,7 @@ struct G2PArgs {
   LeafMap lm;
   float flip;
   int split;  // CTAs per leaf
+  const unsigned* gave_up;  // not 0 when the solve in flight timed out, or null
 };
 
 __device__ __forceinline__ int side(int t) { return t < 0 ? -1 : (t > 7 ? 1 : 0); }
@@ -51,7 +52,10 @@ __global__ void __launch_bounds__(256) k_g2p(const __grid_constant__ G2PArgs a) 
   int lx, ly, lz;
   leaf_coords(a.lm, uint32_t(a.leaf_id[s]), lx, ly, lz);
   const int org[3] = {lx * 8, ly * 8, lz * 8};
+  // without a solution the particles keep their velocities
+  const unsigned gave_up = a.gave_up ? *a.gave_up : 0u;
   __syncthreads();
+  if (gave_up) return;
   const int* n = a.lm.n;
   const uint2 lr = a.leaf_range[s];
   // values and on-bits of a node's three components at once, then the selects
@@ -140,6 +144,7 @@ int launch_g2p(fsim_sim* s) {
   a.vold_on = s->vold_on;
   a.lm = s->lm;
   a.flip = s->cfg.flip_factor;
+  a.gave_up = s->pcg_pending ? &s->d_sc->bar_err : nullptr;
   // few leaves: several CTAs per leaf, each with its share of the particles
   // (and a copy of the halo), up to about six CTAs per SM in all: a CTA's
   // passes over its 2,000 to 4,000 particles are the kernel's time there

@@ -52,6 +52,7 @@ struct GridArgs {
   uint32_t* p2g_touch;            // [particle leaf][32] touched bits of the 1000 nodes
   uint32_t* p2g_low;              // [0]: count; then slot * 1536 + D * 512 + voxel of the
                                   // low-weight faces pass 2 leaves to k_p2g_low
+  const unsigned* gave_up;        // fused pressure update: not 0 when the solve in flight timed out
 };
 
 __device__ __forceinline__ void origin_of(const GridArgs& a, int s, int o[3]) {
@@ -759,7 +760,11 @@ __global__ void __launch_bounds__(256) k_pressure_update(const __grid_constant__
   if (threadIdx.x < 27) nb[threadIdx.x] = a.nbr[int64_t(s) * 27 + threadIdx.x];
   int org[3];
   origin_of(a, s, org);
+  // a pressure that is not a solution leaves the faces as they were (the flag
+  // is loaded along with the neighbour table)
+  const unsigned gave_up = FUSED && a.gave_up ? *a.gave_up : 0u;
   __syncthreads();
+  if (gave_up) return;
   const int* n = a.lm.n;
   float vmax = 0.f;
   for (int v = threadIdx.x; v < 512; v += 256) {
@@ -1000,6 +1005,7 @@ GridArgs make_args(fsim_sim* s) {
   a.cnt = s->d_cnt;
   a.p2g_nodes = s->p2g_nodes;
   a.p2g_touch = s->p2g_touch;
+  a.gave_up = s->pcg_pending ? &s->d_sc->bar_err : nullptr;
   return a;
 }
 

@@ -297,7 +297,9 @@ typedef struct fsim_step_stats {
  * run as fused device kernels.  stats may be NULL.  A step that fails after
  * the rebinning leaves the particles' PIC velocities (gvel) undefined: the
  * rebinning moves them only for the per-stage calls, since the step's G2P
- * rewrites them. */
+ * rewrites them.  A step whose pressure solve gives up (FSIM_ERR_TIMEOUT)
+ * leaves the particles moved, with the velocities they had, and no pressure;
+ * time does not advance. */
 int fsim_step(fsim_t* sim, float dt, const fsim_pcg_params* params,
               fsim_step_stats* stats);
 /* One step on a host-resident particle state: the same results as
