@@ -328,9 +328,7 @@ struct fsim_sim {
   // chip): -1 by system size, 0 never, 1 wherever it fits, ahead of the
   // cluster loop (FSIM_PCG_RES)
   int pcg_res = -1;
-  // small FP32 and MIXED solves by one thread-block cluster (where pcg_res is
-  // by size); false once a cluster launch has been refused
-  bool pcg_cluster = true;
+  uint32_t pcg_refused = 0;  // on-chip loop kernels whose launch was refused (k_pcg.cu)
 
   // water sources and the time they see
   std::vector<fsim_source> sources;

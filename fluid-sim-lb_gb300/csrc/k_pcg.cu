@@ -2230,6 +2230,23 @@ int end_one_launch(fsim_sim* s, const PcgArgs& a, LoopTimer& lt) {
   return FSIM_OK;
 }
 
+// What a loop returns when its launch was refused, with nothing run: the solve
+// then takes the next loop.  Any other value is the solve's status code, an
+// error after the launch among them.
+constexpr int kLoopRefused = -1;
+
+// The kernels of the on-chip loops; by precision (a bit each of
+// fsim_sim::pcg_refused, kLoop* + 4 precision), a refused one is left out for
+// the rest of its handle's life, and only that one: their launches need
+// different resources.
+enum { kLoopCluster = 0, kLoopRes1 = 1, kLoopRes2 = 2, kLoopRes = 3 };
+bool loop_refused(const fsim_sim* s, int loop, int precision) {
+  return (s->pcg_refused >> (4 * precision + loop)) & 1u;
+}
+void refuse_loop(fsim_sim* s, int loop, int precision) {
+  s->pcg_refused |= 1u << (4 * precision + loop);
+}
+
 #include "pcg_cluster.cuh"
 
 // The cluster loop takes FP32 and MIXED solves of at most a leaf per warp of
@@ -2239,8 +2256,8 @@ int end_one_launch(fsim_sim* s, const PcgArgs& a, LoopTimer& lt) {
 // where the resident loop takes 4.2 (MIXED 8.3 against 5.6).  FP64 is
 // bound by the FP64 pipe, which 16 SMs hold too little of.
 bool use_cluster(const fsim_sim* s, int precision) {
-  return precision != FSIM_PREC_FP64 && s->pcg_res < 0 && s->pcg_cluster && s->n_pleaf > 0 &&
-         s->n_pleaf <= kClLeaves && !(precision == FSIM_PREC_FP32 && s->pcg_cg1 == 1);
+  return precision != FSIM_PREC_FP64 && s->pcg_res < 0 && s->n_pleaf > 0 &&
+         s->n_pleaf <= kClLeaves && !loop_refused(s, kLoopCluster, precision) && !(precision == FSIM_PREC_FP32 && s->pcg_cg1 == 1);
 }
 
 #include "pcg_resident.cuh"
@@ -2255,7 +2272,8 @@ bool use_resident(const fsim_sim* s, int precision) {
   const int64_t most = precision == FSIM_PREC_FP64 ? kR64Leaves : kResLeaves;
   if (precision == FSIM_PREC_FP32 && s->pcg_cg1 == 1 && s->pcg_res < 0 && s->n_pleaf < 2 * s->num_sms)
     return false;
-  return s->pcg_res != 0 && s->n_pleaf > 0 && s->n_pleaf <= most * s->num_sms;
+  return s->pcg_res != 0 && s->n_pleaf > 0 && s->n_pleaf <= most * s->num_sms &&
+         !loop_refused(s, res_kernel(s, precision), precision);
 }
 
 // One inner solve: setup, then the iterations.  The iterations run as a CUDA
@@ -2275,14 +2293,14 @@ int run_inner(fsim_sim* s, PcgArgs& a, int grid, const char* nm_setup, const cha
   if constexpr (DM < 2) {
     if (use_cluster(s, prec)) {
       const int rc = run_cluster<DM>(s, a);
-      if (rc != FSIM_ERR_CUDA) return rc;
-      s->pcg_cluster = false;  // refused: another loop, for the rest of this handle's life
+      if (rc != kLoopRefused) return rc;
+      refuse_loop(s, kLoopCluster, prec);
     }
   }
   if (use_resident(s, prec)) {
     const int rc = run_resident<DM>(s, a);
-    if (rc != FSIM_ERR_CUDA) return rc;
-    s->pcg_res = 0;  // a refused cooperative launch: the pair
+    if (rc != kLoopRefused) return rc;
+    refuse_loop(s, res_kernel(s, prec), prec);  // the pair
   }
   const int wpb = kHotThreads / 32;
   int occ_a = 1, occ_b = 1;

@@ -638,8 +638,7 @@ __global__ void __launch_bounds__(kClWarps * 32, 1)
   }
 }
 
-// A solve's iterations (one MIXED segment) by the cluster.  FSIM_ERR_CUDA when
-// the launch is refused (the caller then runs the pair).
+// A solve's iterations (one MIXED segment) by the cluster, or kLoopRefused.
 template <int DM>
 int run_cluster(fsim_sim* s, PcgArgs& a) {
   const int per = (a.n_pleaf + kClCtas - 1) / kClCtas;
@@ -669,7 +668,7 @@ int run_cluster(fsim_sim* s, PcgArgs& a) {
   }
   if (e != cudaSuccess) {
     cudaGetLastError();
-    return FSIM_ERR_CUDA;
+    return kLoopRefused;
   }
   s->launches++;
   return end_one_launch(s, a, lt);

@@ -1465,9 +1465,18 @@ __global__ void __launch_bounds__(kR64Threads, 1) k_pcg_resident64(const __grid_
   if (blockIdx.x == 0 && threadIdx.x == 0) res_finish(q, sc, it);
 }
 
+// The loop's kernel for a system that fits: one or two half leaves per warp
+// (MIXED with two from 11 leaves per SM on), or the general one, FP64's too.
+int res_kernel(const fsim_sim* s, int precision) {
+  const int per = (s->n_pleaf + s->num_sms - 1) / s->num_sms;
+  if (precision == FSIM_PREC_FP64) return kLoopRes;
+  if (per <= kRes1Leaves) return kLoopRes1;
+  if (per <= 2 * kRes1Leaves && per >= (precision == FSIM_PREC_FP32 ? 0 : 11)) return kLoopRes2;
+  return kLoopRes;
+}
+
 // The iterations of a solve (of one MIXED segment) by the resident loop: one
-// cooperative launch of one CTA per SM.  FSIM_ERR_CUDA when the launch is
-// refused (the caller then runs the pair).
+// cooperative launch of one CTA per SM, or kLoopRefused.
 template <int DM>
 int run_resident(fsim_sim* s, PcgArgs& a) {
   void* fn;
@@ -1483,11 +1492,12 @@ int run_resident(fsim_sim* s, PcgArgs& a) {
     fn = reinterpret_cast<void*>(k_pcg_resident<DM>);
     name = DM == 0 ? "pcg_resident" : "pcg_resident_mixed";
     const int per = (s->n_pleaf + s->num_sms - 1) / s->num_sms;
-    if (per <= kRes1Leaves) {
+    const int form = res_kernel(s, DM == 0 ? FSIM_PREC_FP32 : FSIM_PREC_MIXED);
+    if (form == kLoopRes1) {
       fn = reinterpret_cast<void*>(k_pcg_resident1<DM, 1>);
       smem = kRes1Leaf * per;
       threads = 64 * per;
-    } else if (per <= 2 * kRes1Leaves && per >= (DM == 0 ? 0 : 11)) {
+    } else if (form == kLoopRes2) {
       fn = reinterpret_cast<void*>(k_pcg_resident1<DM, 2>);
       smem = kRes1Leaf * per + size_t(2 * kRes1Warps) * 256 * sizeof(float);
       threads = 32 * kRes1Warps;
@@ -1499,7 +1509,7 @@ int run_resident(fsim_sim* s, PcgArgs& a) {
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, threads, smem) != cudaSuccess ||
       occ < 1) {
     cudaGetLastError();
-    return FSIM_ERR_CUDA;
+    return kLoopRefused;
   }
   a.cond = 0;
   FSIM_CK(s, cudaMemsetAsync(res_words(a), 0, 2 * kResSetWords * sizeof(unsigned long long),
@@ -1513,7 +1523,7 @@ int run_resident(fsim_sim* s, PcgArgs& a) {
                                                       s->stream);
     if (e != cudaSuccess) {
       cudaGetLastError();
-      return FSIM_ERR_CUDA;
+      return kLoopRefused;
     }
   }
   s->launches++;
