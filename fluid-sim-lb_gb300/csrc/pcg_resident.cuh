@@ -1480,12 +1480,12 @@ int res_kernel(const fsim_sim* s, int precision) {
 template <int DM>
 int run_resident(fsim_sim* s, PcgArgs& a) {
   void* fn;
-  size_t smem = kResSmem;
+  size_t smem = kResSmem, most = kResSmem;  // this launch's shared memory, and the kernel's most
   int threads = kResThreads;
   const char* name;
   if constexpr (DM == 2) {
     fn = reinterpret_cast<void*>(k_pcg_resident64);
-    smem = kR64Smem;
+    smem = most = kR64Smem;
     threads = kR64Threads;
     name = "pcg_resident_f64";
   } else {
@@ -1496,15 +1496,20 @@ int run_resident(fsim_sim* s, PcgArgs& a) {
     if (form == kLoopRes1) {
       fn = reinterpret_cast<void*>(k_pcg_resident1<DM, 1>);
       smem = kRes1Leaf * per;
+      most = kRes1Leaf * kRes1Leaves;
       threads = 64 * per;
     } else if (form == kLoopRes2) {
       fn = reinterpret_cast<void*>(k_pcg_resident1<DM, 2>);
-      smem = kRes1Leaf * per + size_t(2 * kRes1Warps) * 256 * sizeof(float);
+      constexpr size_t kX = size_t(2 * kRes1Warps) * 256 * sizeof(float);
+      smem = kRes1Leaf * per + kX;
+      most = kRes1Leaf * 2 * kRes1Leaves + kX;
       threads = 32 * kRes1Warps;
     }
   }
+  // The attribute belongs to the kernel, not to the handle: every handle sets
+  // the same, or another thread's smaller system would have this launch refused.
   int occ = 0;
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) !=
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(most)) !=
           cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, threads, smem) != cudaSuccess ||
       occ < 1) {
