@@ -219,11 +219,17 @@ __global__ void k_fill_u32(unsigned* __restrict__ p, int64_t n, unsigned v) {
 }
 
 // Rings of cells that can hold a particle within reach of a voxel, or 0 when
-// they do not fit in the leaf neighbourhood.
+// they do not fit in the leaf neighbourhood.  A particle of ring r is at least
+// r away, so r rings do once fl(r - radius) is not below half_width; that may
+// take one more than the ceiling of the rounded sum (0.7395036 + 0.2604965
+// rounds to 1, and 1 - 0.7395036 to less than 0.2604965).
 int gather_rings(const fsim_t* s, float radius, float half_width) {
   if (s->composite_sort || !s->ranges_match) return 0;
   const float reach = std::ceil(radius + half_width);
-  return reach <= float(kLsRings) ? int(reach) : 0;
+  if (!(reach <= float(kLsRings))) return 0;
+  const int rings = float(reach - radius) < half_width ? int(reach) + 1 : int(reach);
+  // bands whose squared reach underflows take the splat
+  return rings <= kLsRings && (radius + half_width) * (radius + half_width) > 0x1p-100f ? rings : 0;
 }
 
 int level_set(fsim_t* s, float radius, float half_width, int mean_iterations, float* f[2],
