@@ -410,11 +410,45 @@ __global__ void __launch_bounds__(256)
 
 // k_sort_leaf: a CTA orders a leaf's bin by (cell, old key, row): a counting
 // sort by cell into shared memory, then each entry's rank among its cell's
-// (about 8, most of them one broadcast for the warp).  keys and perm get the
-// leaf's sorted keys and rows.
+// (about 8, most of them one broadcast for the warp).  A cell of more than
+// kCrowded entries, whose ranks would take the square of that, is sorted in
+// place instead, by a warp, or past kWideCell by the CTA.  One leaf of about
+// 12,000 rows in cells of 24 / 40 / 64 / 128 / 512 / 1,024 / 6,144 (us, rows
+// with old keys): ranks 104 / 73 / 387 / 722 / 2,274 / 3,449 / 4,574, sorted 135 / 94 /
+// 72 / 65 / 71 / 85 / 133; the library's sort of the same rows takes 58 to 101.
+// keys and perm get the leaf's sorted keys and rows.
 constexpr int kLeafSortThreads = 1024;
+constexpr int kCrowded = 48, kWideCell = 1024;
 template <bool OLD>
 using SortEntry = typename std::conditional<OLD, unsigned long long, uint32_t>::type;
+
+// Bitonic sort of e[0 .. m) by threads t of n, sync() between passes.  Every
+// comparison puts the smaller entry first, so places past m (up to the power
+// of two, where larger entries would be) need not exist.
+template <typename E, typename S>
+__device__ __forceinline__ void bitonic_sort(E* e, int m, int t0, int n, S&& sync) {
+  int lg = 0;
+  while ((1 << lg) < m) ++lg;
+  auto order = [&](int i, int j) {
+    if (j >= m) return;
+    const E a = e[i], b = e[j];
+    if (b < a) {
+      e[i] = b;
+      e[j] = a;
+    }
+  };
+  for (int k = 1; k <= lg; ++k) {
+    for (int q = k; q > 0; --q) {
+      const int h = 1 << (q - 1);  // half a block; the first pass of k compares mirrored places
+      for (int t = t0; t < (1 << lg) / 2; t += n) {
+        const int off = t & (h - 1), base = (t - off) * 2;
+        order(base + off, q == k ? base + 2 * h - 1 - off : base + off + h);
+      }
+      sync();
+    }
+  }
+}
+
 template <bool OLD>
 __global__ void __launch_bounds__(kLeafSortThreads)
     k_sort_leaf(const int32_t* __restrict__ leaf_of, const int64_t* __restrict__ cnt,
@@ -427,6 +461,7 @@ __global__ void __launch_bounds__(kLeafSortThreads)
   E* ent = reinterpret_cast<E*>(sort_smem);  // kLeafSort entries
   __shared__ int at[512];                    // a cell's count, then its next place
   __shared__ int wsum[16];
+  __shared__ int crowded, crowd[kLeafSort / kCrowded];  // the crowded cells, in any order
   if (cnt[1] & kLeafOverflow) return;  // the host sorts another way
   const int np = int(cnt[1]), tid = threadIdx.x, lane = tid & 31;
   for (int s = blockIdx.x; s < np; s += gridDim.x) {
@@ -434,6 +469,7 @@ __global__ void __launch_bounds__(kLeafSortThreads)
     const int m = int(lcnt[d]);
     const uint32_t b = next[d] - uint32_t(m);  // k_bin_rows left it at the bin's end
     if (tid < 512) at[tid] = 0;
+    if (tid == 0) crowded = 0;
     __syncthreads();
     for (int j = tid; j < m; j += kLeafSortThreads) atomicAdd(&at[cell[b + j]], 1);
     __syncthreads();
@@ -455,6 +491,7 @@ __global__ void __launch_bounds__(kLeafSortThreads)
       for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
       first += before - c;
       at[tid] = first;
+      if (c > kCrowded) crowd[atomicAdd(&crowded, 1)] = tid;
     }
     __syncthreads();
     for (int j = tid; j < m; j += kLeafSortThreads) {
@@ -466,8 +503,23 @@ __global__ void __launch_bounds__(kLeafSortThreads)
       keys[b + p] = (d << 9) | uint32_t(v);
     }
     __syncthreads();
+    for (int q = 0; q < crowded; ++q) {
+      const int v = crowd[q], beg = v ? at[v - 1] : 0, n = at[v] - beg;
+      if (n > kWideCell) {
+        bitonic_sort(ent + beg, n, tid, kLeafSortThreads, [] { __syncthreads(); });
+        for (int j = tid; j < n; j += kLeafSortThreads) perm[b + beg + j] = uint32_t(ent[beg + j]);
+      }
+    }
+    for (int q = tid >> 5; q < crowded; q += kLeafSortThreads / 32) {
+      const int v = crowd[q], beg = v ? at[v - 1] : 0, n = at[v] - beg;
+      if (n <= kWideCell) {
+        bitonic_sort(ent + beg, n, lane, 32, [] { __syncwarp(); });
+        for (int j = lane; j < n; j += 32) perm[b + beg + j] = uint32_t(ent[beg + j]);
+      }
+    }
     for (int j = tid; j < m; j += kLeafSortThreads) {
       const int v = cell[b + j], end = at[v], beg = v ? at[v - 1] : 0;
+      if (end - beg > kCrowded) continue;
       E e = row[b + j];
       if constexpr (OLD) e |= static_cast<unsigned long long>(old[b + j]) << 32;
       int rank = 0;
