@@ -27,7 +27,9 @@
 // with every warp polling, measured slower: 3.99 against 3.2 us per
 // iteration at 64^3.)  Element-wise arithmetic is the pair's; only the order
 // of the dot products differs.  Scalars stay off the narrow FP64 pipe: fp32
-// for FP32 (as the reference), double-float pairs for MIXED.
+// for FP32 (as the reference); for MIXED the totals are double-float pairs, as
+// the pair's, and alpha and beta the roundings of their fp64 quotients
+// (pcg_scalar.cuh).
 // Measured us per iteration, against the pair (sphere drop; particle leaves):
 //   leaves        24          84          156         189
 //   FP32     2.13 / 6.57  2.62 / 6.42  3.13 / 6.51  3.36 / 6.48
@@ -216,24 +218,7 @@ __device__ __forceinline__ bool cl_sum(P (&v)[NV], P* wp, P* tot, const ClFrame&
   return bad;
 }
 
-// Scalar steps in the partials' type.  FP32: a / b as the pair (fp32).  MIXED:
-// the quotient of two double-float numbers, rounded to fp32: q1 = a.hi / b.hi
-// and a correction from the exact remainder (its error is about 2^-45 of the
-// quotient before the rounding; the pair rounds a double quotient).
-__device__ __forceinline__ float cl_div(float a, float b) { return __fdiv_rn(a, b); }
-__device__ __forceinline__ float cl_div(float2 a, float2 b) {
-  const float q = __fdiv_rn(a.x, b.x);
-  const float e = __fadd_rn(__fmaf_rn(-q, b.x, a.x), __fmaf_rn(-q, b.y, a.y));
-  const float d = __fdiv_rn(e, b.x);
-  const float s = __fadd_rn(q, d);
-  return s == s ? s : q;  // inf and NaN quotients stay what the leading term says
-}
-__device__ __forceinline__ void cl_split(double v, double& o) { o = v; }
-__device__ __forceinline__ void cl_split(double v, float& o) { o = float(v); }
-__device__ __forceinline__ void cl_split(double v, float2& o) {
-  o.x = float(v);
-  o.y = float(v - double(o.x));
-}
+#include "pcg_scalar.cuh"
 
 // T(diag) of a flags byte: the small integer as the low mantissa bits of 2^23,
 // less 2^23 (exact)
@@ -256,8 +241,10 @@ __device__ __forceinline__ ClStop<P> cl_stop_of(const PcgScalars* sc) {
   q.strict = sc->mode == FSIM_PCG_ABSOLUTE;
   if constexpr (std::is_same<P, float>::value)
     q.thr = q.strict ? float(sc->thr) : __double2float_rd(sc->thr);
+  else if constexpr (std::is_same<P, float2>::value)
+    cl_threshold(sc->thr, q.thr);
   else
-    cl_split(sc->thr, q.thr);
+    q.thr = sc->thr;
   return q;
 }
 __device__ __forceinline__ bool cl_stop(const ClStop<double>& q, double rr) {
@@ -267,7 +254,7 @@ __device__ __forceinline__ bool cl_stop(const ClStop<float>& q, float rr) {
   return !q.fixed && (q.strict ? rr < q.thr : rr <= q.thr);
 }
 __device__ __forceinline__ bool cl_stop(const ClStop<float2>& q, float2 rr) {
-  return !q.fixed && (rr.x < q.thr.x || (rr.x == q.thr.x && rr.y <= q.thr.y));
+  return !q.fixed && cl_at_most(rr, q.thr);
 }
 
 // Shared memory of a CTA with W warps, a leaf each: p of its leaves and a zero
@@ -482,7 +469,7 @@ __global__ void __launch_bounds__(kClWarps * 32, 1)
   cl_sync();  // every CTA's z and zeroed words are in place
   load_halo();
   // PCGDriver::Solve's loop test, then at the end of each iteration
-  bool go = !sc->done && it < max_it && !cl_stop(stop, rr);
+  bool go = !sc->done && it < max_it && !converged(sc, sc->rr);
   while (go) {
     // S: p = z + beta p, on the own and the halo columns
 #pragma unroll
@@ -559,7 +546,7 @@ __global__ void __launch_bounds__(kClWarps * 32, 1)
       if ((bad = cl_sum<P, 1, false>(v, wp, tot, c, dst_a, src_a, ++tag))) break;
       pap = v[0];
     }
-    alpha = cl_div(rz, pap);
+    alpha = cl_div(rz, pap, it == it0, sc->rz, true);
     if (!(alpha <= 1e5f)) {  // CHECK_LE(alpha, LARGE_FLOAT)
       status = FSIM_ERR_BREAKDOWN;
       break;
@@ -596,7 +583,7 @@ __global__ void __launch_bounds__(kClWarps * 32, 1)
       rz_old = rz;
       rz = v[1];
     }
-    beta = cl_div(rz, rz_old);
+    beta = cl_div(rz, rz_old, it == it0, sc->rz, false);
     ++it;
     if (!(beta <= 1e5f)) status = FSIM_ERR_BREAKDOWN;  // CHECK_LE(beta, LARGE_FLOAT)
     go = status == FSIM_OK && it < max_it && !cl_stop(stop, rr);

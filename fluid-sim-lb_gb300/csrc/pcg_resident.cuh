@@ -440,6 +440,7 @@ __device__ __forceinline__ bool res_first(const PcgArgs& a, ResShared<P, W>& sh,
 template <typename P>
 struct ResScalars {
   P rr, rz, rz_old, pAp;
+  double rz0;         // the first r.z, from the set-up in fp64
   float alpha, beta;  // FP64 keeps its own
   double alpha64, beta64;
   int status, max_iter;
@@ -449,6 +450,7 @@ template <typename P>
 __device__ __forceinline__ void res_scalars(ResScalars<P>& q, const PcgScalars* sc) {
   cl_split(sc->rr, q.rr);
   cl_split(sc->rz, q.rz);
+  q.rz0 = sc->rz;
   cl_split(sc->rz_old, q.rz_old);
   q.pAp = pzero<P>();
   q.alpha = 0.f;
@@ -761,7 +763,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(const __grid_co
   if (threadIdx.x == 0) {
     res_scalars(q, sc);
     res_start(sh.bar, sc);
-    s_done = sc->done || it >= q.max_iter || cl_stop(q.stop, q.rr);  // PCGDriver::Solve's loop test
+    s_done = sc->done || it >= q.max_iter || converged(sc, sc->rr);  // PCGDriver::Solve's loop test
   }
   P* const rows = part_rows<DM>(a);
   __syncthreads();
@@ -815,7 +817,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(const __grid_co
       const P like[1] = {it == it0 ? q.rz : q.pAp};
       ok = res_sync<P, 1, false>(a, v, like, sh, rows, 0, [&](const P (&tot)[1]) {
         q.pAp = tot[0];
-        q.alpha = cl_div(q.rz, q.pAp);
+        q.alpha = cl_div(q.rz, q.pAp, it == it0, q.rz0, true);
         if (!(q.alpha <= 1e5f)) {  // CHECK_LE(alpha, LARGE_FLOAT)
           q.status = FSIM_ERR_BREAKDOWN;
           s_done = 1;
@@ -875,7 +877,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(const __grid_co
         q.rr = tot[0];
         q.rz_old = q.rz;
         q.rz = tot[1];
-        q.beta = cl_div(q.rz, q.rz_old);
+        q.beta = cl_div(q.rz, q.rz_old, it == it0, q.rz0, false);
         if (!(q.beta <= 1e5f)) {  // CHECK_LE(beta, LARGE_FLOAT)
           q.status = FSIM_ERR_BREAKDOWN;
           s_done = 1;
@@ -1033,7 +1035,7 @@ __global__ void __launch_bounds__(kRes1Warps * 32, 1) k_pcg_resident1(const __gr
   if (threadIdx.x == 0) {
     res_scalars(q, sc);
     res_start(sh.bar, sc);
-    s_done = sc->done || it >= q.max_iter || cl_stop(q.stop, q.rr);  // PCGDriver::Solve's loop test
+    s_done = sc->done || it >= q.max_iter || converged(sc, sc->rr);  // PCGDriver::Solve's loop test
   }
   P* const rows = part_rows<DM>(a);
   __syncthreads();
@@ -1094,7 +1096,7 @@ __global__ void __launch_bounds__(kRes1Warps * 32, 1) k_pcg_resident1(const __gr
       const P like[1] = {it == it0 ? q.rz : q.pAp};
       ok = res_sync<P, 1, false>(a, v, like, sh, rows, 0, [&](const P (&tot)[1]) {
         q.pAp = tot[0];
-        q.alpha = cl_div(q.rz, q.pAp);
+        q.alpha = cl_div(q.rz, q.pAp, it == it0, q.rz0, true);
         if (!(q.alpha <= 1e5f)) {  // CHECK_LE(alpha, LARGE_FLOAT)
           q.status = FSIM_ERR_BREAKDOWN;
           s_done = 1;
@@ -1139,7 +1141,7 @@ __global__ void __launch_bounds__(kRes1Warps * 32, 1) k_pcg_resident1(const __gr
         q.rr = tot[0];
         q.rz_old = q.rz;
         q.rz = tot[1];
-        q.beta = cl_div(q.rz, q.rz_old);
+        q.beta = cl_div(q.rz, q.rz_old, it == it0, q.rz0, false);
         if (!(q.beta <= 1e5f)) {  // CHECK_LE(beta, LARGE_FLOAT)
           q.status = FSIM_ERR_BREAKDOWN;
           s_done = 1;
@@ -1335,7 +1337,7 @@ __global__ void __launch_bounds__(kR64Threads, 1) k_pcg_resident64(const __grid_
   if (threadIdx.x == 0) {
     res_scalars(q, sc);
     res_start(sh.bar, sc);
-    s_done = sc->done || it >= q.max_iter || cl_stop(q.stop, q.rr);  // PCGDriver::Solve's loop test
+    s_done = sc->done || it >= q.max_iter || converged(sc, sc->rr);  // PCGDriver::Solve's loop test
   }
   const int it0 = it;
   __syncthreads();
