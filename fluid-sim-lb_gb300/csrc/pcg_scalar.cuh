@@ -4,8 +4,9 @@
 //
 // FP32: fp32, as the reference.  MIXED: the values of the spmv / update pair,
 // which divides its double-float totals in fp64 and rounds the quotient to the
-// vectors' fp32, without that division: the FP64 pipe takes some 0.7 us for
-// one, twice per iteration of 3.4 us (24 leaves).
+// vectors' fp32, without that division on the narrow FP64 pipe.  us per
+// iteration with it and without: 24 leaves 4.53 / 3.45, 156 7.28 / 4.82 (every
+// warp of the cluster divides), 1,148 7.43 / 6.49, 8,320 20.67 / 19.65.
 
 // RN32(a / b) as fp64 gives it, for double-float totals and the set-up's fp64
 // r.z (the conversions, fp64 too, stay out of the callers)
