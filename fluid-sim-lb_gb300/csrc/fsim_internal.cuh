@@ -281,7 +281,8 @@ struct fsim_sim {
   double* Ap64 = nullptr;
   double* b64 = nullptr;
   fsim::PcgScalars* d_sc = nullptr;
-  double* d_part = nullptr;  // block partials (3 * max_blocks)
+  double* d_part = nullptr;  // block partials and, in the last row, the resident
+                             // loop's barrier words (4 * max_blocks)
   float* d_partf = nullptr;  // fp32 / double-float partials of the hot PCG kernels (16 * max_blocks)
   int max_blocks = 0;
 
@@ -314,7 +315,7 @@ struct fsim_sim {
   // bounded wait has given up (FSIM_PCG_TMA_WITHHOLD=1)
   int tma_spmv = 0;
   int tma_withhold = 0;
-  // FSIM_PCG_RES_WITHHOLD=1 (tests): in the first solve CTA 0 of the resident
+  // FSIM_PCG_RES_WITHHOLD=1 (tests): in the first solve CTA 0 of the on-chip
   // loop skips its first barrier arrival, so that every CTA's bounded wait
   // gives up
   int res_withhold = 0;

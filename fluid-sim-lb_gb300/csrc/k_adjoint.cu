@@ -174,14 +174,10 @@ __device__ __forceinline__ void mac_stencil(int D, const int c[3], const double 
 __device__ __forceinline__ int side_of(const TopoView& t, int64_t i) {
   return t.side ? int(t.side[i]) : -1;
 }
-// trilinear weight of corner (di,dj,dk) and its gradient in the position
-__device__ __forceinline__ double tri_w(const double f[3], int di, int dj, int dk, double g[3]) {
+// trilinear weight of corner (di,dj,dk)
+__device__ __forceinline__ double tri_w(const double f[3], int di, int dj, int dk) {
   const double wx = di ? f[0] : 1.0 - f[0], wy = dj ? f[1] : 1.0 - f[1],
                wz = dk ? f[2] : 1.0 - f[2];
-  const double sx = di ? 1.0 : -1.0, sy = dj ? 1.0 : -1.0, sz = dk ? 1.0 : -1.0;
-  g[0] = sx * wy * wz;
-  g[1] = wx * sy * wz;
-  g[2] = wx * wy * sz;
   return wx * wy * wz;
 }
 
@@ -440,13 +436,12 @@ __global__ void k_rp_pupdate(const TopoView t, const double* __restrict__ u,
 }
 
 // interpolation of one component at the particle (ghost-extrapolated field,
-// inactive faces read as 0), with the gradient in the position
+// inactive faces read as 0)
 template <typename V>
 __device__ __forceinline__ double interp(const TopoView& t, const V* __restrict__ f,
                                          const uint32_t* __restrict__ on, int D, const int st[3],
-                                         const double fr[3], double grad[3]) {
+                                         const double fr[3]) {
   double r = 0.0;
-  grad[0] = grad[1] = grad[2] = 0.0;
   for (int q = 0; q < 8; ++q) {
     const int di = q >> 2, dj = (q >> 1) & 1, dk = q & 1;
     const int g[3] = {st[0] + di, st[1] + dj, st[2] + dk};
@@ -457,9 +452,7 @@ __device__ __forceinline__ double interp(const TopoView& t, const V* __restrict_
     const int v = vox_of(src[0], src[1], src[2]);
     if (!bit_at(on, s, v)) continue;
     const double val = double(f[int64_t(s) * 1536 + D * 512 + v]);
-    double gw[3];
-    r += tri_w(fr, di, dj, dk, gw) * val;
-    grad[0] += gw[0] * val; grad[1] += gw[1] * val; grad[2] += gw[2] * val;
+    r += tri_w(fr, di, dj, dk) * val;
   }
   return r;
 }
@@ -476,10 +469,10 @@ __global__ void k_rp_g2p(const TopoView t, int64_t n, const uint32_t* __restrict
 #pragma unroll
   for (int D = 0; D < 3; ++D) {
     int s3[3];
-    double fr[3], gd[3];
+    double fr[3];
     mac_stencil(D, c, p, s3, fr, side_of(t, i));
-    const double vi = interp(t, unew, t.vel_on, D, s3, fr, gd);
-    const double di = interp(t, dv, t.touched, D, s3, fr, gd);
+    const double vi = interp(t, unew, t.vel_on, D, s3, fr);
+    const double di = interp(t, dv, t.touched, D, s3, fr);
     st[D * n + i] = p[D];
     st[(3 + D) * n + i] = vi + flip * ((di + vp[D * n + i]) - vi);
     st[(6 + D) * n + i] = vi;

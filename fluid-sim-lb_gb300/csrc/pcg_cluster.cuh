@@ -43,9 +43,11 @@
 // barrier, so no CTA's shared memory goes while another may still reach it.
 constexpr int kClCtas = 16;                       // CTAs of the cluster (one per SM)
 constexpr int kClWarps = 12;                      // warps per CTA, at most (168 registers)
-// leaves per warp (written as loops over them: without, the compiler's schedule
+// leaves per warp: one, since p, x and the inverse diagonal are kept for one
+// (written as loops over them all the same: without, the compiler's schedule
 // takes 2.38 us per iteration at 24 leaves instead of 2.13)
 constexpr int kClPerWarp = 1;
+static_assert(kClPerWarp == 1, "Pc, X and inv hold one leaf's columns");
 constexpr int kClLeaves = kClCtas * kClWarps * kClPerWarp;  // 192 particle leaves
 constexpr unsigned kClPolls = 1u << 22;
 
@@ -484,7 +486,7 @@ __global__ void __launch_bounds__(kClWarps * 32, 1)
 #pragma unroll
           for (int z = 0; z < 8; ++z) p.v[z] = tadd(Z[k][q].v[z], tmul(beta, p.v[z]));
           ps_st4(mem, mine, p);
- Pc[q] = p;
+          Pc[q] = p;
         }
         if (rem[k] & 1u) halo_col(x0 == 0 ? xm_i[k] : xp_i[k], hx[k], beta);
         if (rem[k] & 2u) {
@@ -567,8 +569,7 @@ __global__ void __launch_bounds__(kClWarps * 32, 1)
           for (int z = 0; z < 8; ++z) {
             R[k][q].v[z] = tadd(tmul(nalpha, Z[k][q].v[z]), R[k][q].v[z]);
             drr.add(R[k][q].v[z], R[k][q].v[z]);
-            Z[k][q].v[z] = tmul(inv[q][z],
-                                R[k][q].v[z]);
+            Z[k][q].v[z] = tmul(inv[q][z], R[k][q].v[z]);
             drz.add(R[k][q].v[z], Z[k][q].v[z]);
           }
           if (read[k]) ps_st4(zs, mine, Z[k][q]);
@@ -638,6 +639,7 @@ int run_cluster(fsim_sim* s, PcgArgs& a) {
   a.cond = 0;
   LoopTimer lt(s);
   if (e == cudaSuccess) {
+    // (profiles find a solve's iterations by their first kernel's name, pcg_spmv*)
     fsim::ProfScope ps(s, DM == 0 ? "pcg_spmv_update_cluster" : "pcg_spmv_update_cluster_mixed");
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kClCtas);

@@ -181,6 +181,12 @@ __device__ __forceinline__ bool res_slow(const PcgArgs& a, P (&v)[NV], ResShared
 // call are visible to every CTA after it.  False when the wait gave up.  With
 // PcgArgs::res_withhold (tests) CTA 0 does not arrive at the first barrier and
 // the limit is 256 polls.
+// The p.Ap barrier (PUBLISH false) is relaxed in memory: what keeps another
+// CTA's store of z in U behind this CTA's loads of it in S is that every value
+// loaded goes into A p and so into the partial that arrives, and that the
+// store needs alpha, which needs all partials.  A load of z or p that is not
+// used before the arrival (a prefetch across it) would need the release and
+// acquire of the other barrier.
 template <typename P, int NV, bool PUBLISH, int W, typename F>
 __device__ __forceinline__ bool res_sync(const PcgArgs& a, P (&v)[NV], const P (&like)[NV],
                                          ResShared<P, W>& sh, P* slow_rows, int ph, F&& fin) {
@@ -374,8 +380,7 @@ __device__ __forceinline__ void res_finish(const ResScalars<P>& q, PcgScalars* s
 
 // Where a neighbour of the CTA's cells lives.
 struct ResFrame {
-  const float* ps;       // shared p of the CTA's leaves
-  const uint8_t* fsm;    // shared flags
+  const float* ps;  // shared p of the CTA's leaves
   int L0, nl, n_pleaf;
 };
 __device__ __forceinline__ bool res_local(const ResFrame& fr, int slot) {
@@ -385,8 +390,8 @@ __device__ __forceinline__ bool res_local(const ResFrame& fr, int slot) {
 // p (current iteration) of cell (x, y, z) of leaf `slot`: from shared memory
 // for the CTA's leaves, else formed from the mirrors of z and the previous p.
 __device__ __forceinline__ float res_pcell(const ResFrame& fr, const PcgArgs& a,
-                                           const float* pm_old, const DiagInv<float>* tab,
-                                           float beta, int slot, int x, int y, int z) {
+                                           const float* pm_old, float beta, int slot, int x, int y,
+                                           int z) {
   if (res_local(fr, slot)) return fr.ps[(ps_col4(slot - fr.L0, x, y) + (z >> 2) * 64) * 4 + (z & 3)];
   const unsigned o = slot_or_null(slot, fr.n_pleaf) * 512u + unsigned(x * 64 + y * 8 + z);
   // the mirror holds z = M r (the owner's product): pnew_of's operations
@@ -400,8 +405,8 @@ __device__ __forceinline__ float res_pcell(const ResFrame& fr, const PcgArgs& a,
 // from the mirrors of z and the previous p, with the owner's operations.
 // Faces in the CTA's own leaves are left to shared memory (v stays 0).
 __device__ __forceinline__ void res_faces(const ResFrame& fr, const PcgArgs& a, const float* pm_old,
-                                          const DiagInv<float>* tab, float beta, int xb,
-                                          const int fs[6], int lane, float (&v)[4]) {
+                                          float beta, int xb, const int fs[6], int lane,
+                                          float (&v)[4]) {
   const int t = lane >> 1;
   int slot, off;
   if (t < 8) {
@@ -508,10 +513,10 @@ __device__ __forceinline__ void res_ap(const ResFrame& fr, const PcgArgs& a, con
                                        int y, int lane, const int fs[6], const Col<float>& P,
                                        uint2 f, Col<float>& ap) {
   float fv[4];
-  res_faces(fr, a, pm_old, tab, beta, xb, fs, lane, fv);
+  res_faces(fr, a, pm_old, beta, xb, fs, lane, fv);
   res_stencil<false>(fr, tab, s, xb, lx, y, fs, P, f, fv,
-              [&] { return res_pcell(fr, a, pm_old, tab, beta, fs[4], xb + lx, y, 7); },
-              [&] { return res_pcell(fr, a, pm_old, tab, beta, fs[5], xb + lx, y, 0); }, ap);
+              [&] { return res_pcell(fr, a, pm_old, beta, fs[4], xb + lx, y, 7); },
+              [&] { return res_pcell(fr, a, pm_old, beta, fs[5], xb + lx, y, 0); }, ap);
 }
 // The Jacobi inverse by flags & 15 (the table's values).  U of k_pcg_resident
 // reads it from constant memory, off the shared-memory path: most warps ask
@@ -585,7 +590,6 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(const __grid_co
   const int per = (a.n_pleaf + G - 1) / G;  // the host checks per <= kResLeaves
   ResFrame fr;
   fr.ps = ps;
-  fr.fsm = fsm;
   fr.L0 = int(blockIdx.x) * per;
   fr.nl = max(0, min(per, a.n_pleaf - fr.L0));
   fr.n_pleaf = a.n_pleaf;
@@ -856,7 +860,6 @@ __global__ void __launch_bounds__(kRes1Warps * 32, 1) k_pcg_resident1(const __gr
   float4* const xs = reinterpret_cast<float4*>(res_smem + kRes1Leaf * per);  // x, KH > 1
   ResFrame fr;
   fr.ps = ps;
-  fr.fsm = nullptr;
   fr.L0 = int(blockIdx.x) * per;
   fr.nl = max(0, min(per, a.n_pleaf - fr.L0));
   fr.n_pleaf = a.n_pleaf;
