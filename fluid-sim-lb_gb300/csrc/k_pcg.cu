@@ -2251,8 +2251,8 @@ void refuse_loop(fsim_sim* s, int loop, int precision) {
 
 // The cluster loop takes FP32 and MIXED solves of at most a leaf per warp of
 // its 16 CTAs, 192, unless another loop is asked for by its switch: at 189
-// leaves 3.36 us per iteration against the resident loop's 4.2 (MIXED 4.92 /
-// 5.6).  With two leaves per warp it took 5.0 to 5.1 at 227 to 238 leaves,
+// leaves 3.36 us per iteration against the resident loop's 4.2 (MIXED 4.94 /
+// 5.55).  With two leaves per warp it took 5.0 to 5.1 at 227 to 238 leaves,
 // where the resident loop takes 4.2 (MIXED 8.3 against 5.6).  FP64 is
 // bound by the FP64 pipe, which 16 SMs hold too little of.
 bool use_cluster(const fsim_sim* s, int precision) {

@@ -33,10 +33,12 @@
 // Measured us per iteration, against the pair (sphere drop; particle leaves):
 //   leaves        24          84          156         189
 //   FP32     2.13 / 6.57  2.62 / 6.42  3.13 / 6.51  3.36 / 6.48
-//   MIXED    3.42 / 10.1  4.06 / 9.32  4.74 / 9.17  4.92 / 9.51
-// (the resident loop: 4.1 to 4.3 for FP32, 5.5 to 5.6 for MIXED).  At 24
+//   MIXED    3.46 / 10.1  4.08 / 9.32  4.78 / 9.17  4.94 / 9.51
+// (the resident loop: 3.7 to 4.2 for FP32, 5.1 to 5.6 for MIXED).  At 24
 // leaves it is latency (two one-way pushes, four CTA barriers, six warp
-// reductions); from about 100 on also the bandwidth of shared memory.
+// reductions); from about 100 on also the bandwidth of shared memory (156
+// leaves: its SMs issue in 28% of their cycles, MIXED 37%, and wait for CTA
+// barriers first, then for shared memory).
 //
 // The polls are bounded (kClPolls): a CTA whose wait gives up leaves the loop,
 // the other CTAs' waits run out in turn, and all meet at a last cluster

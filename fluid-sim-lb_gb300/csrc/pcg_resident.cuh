@@ -32,8 +32,8 @@
 // Measured us per iteration (particle leaves; 152 SMs), against the pair (the
 // first three columns by k_pcg_resident1, below):
 //   leaves        24          488        1,148       3,204       8,320
-//   FP32     4.12 / 6.56  4.33 / 8.42  4.73 / 12.5  8.96 / 18.6  14.9 / 31.9
-//   MIXED    5.59 / 10.0  5.78 / 10.7  6.42 / 13.5  11.8 / 19.7  19.7 / 34.6
+//   FP32     3.69 / 6.56  4.31 / 8.42  4.74 / 12.5  8.91 / 18.6  14.9 / 31.9
+//   MIXED    5.06 / 10.0  5.80 / 10.7  6.50 / 13.5  11.8 / 19.7  19.7 / 34.6
 // (before the fixed-point barrier FP32 took 5.90, 6.57, 6.96, 9.80 and 15.9).
 constexpr int kResWarps = 28;
 constexpr int kResThreads = kResWarps * 32;
@@ -832,11 +832,12 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_resident(const __grid_co
 // reader, formed from the owner's z like the owner's own p, so z is all that
 // CTAs exchange.  The operations and their order are k_pcg_resident's, so the
 // bits are too.  Bound by the iteration's chain of latencies (two grid
-// barriers, one round trip to L2 for the faces, the CTA barriers).  us per
-// iteration against k_pcg_resident, FP32 and MIXED (leaves per SM):
-//   KH = 1   488 (4): 4.33 / 5.61, 5.78 / 7.60   1,148 (8): 4.73 / 6.07, 6.42 / 8.17
+// barriers, one round trip to L2 for the faces, the CTA barriers: at 1,148
+// leaves an SM issues in 18% of its cycles, MIXED 25%).  us per iteration
+// against k_pcg_resident, FP32 and MIXED (leaves per SM):
+//   KH = 1   488 (4): 4.31 / 5.61, 5.80 / 7.60   1,148 (8): 4.74 / 6.07, 6.50 / 8.17
 //   KH = 2   1,278 (9): 5.99 / 6.23, 8.62 / 8.42   1,456 (10): 6.01 / 6.40, 8.63 / 8.54
-//            1,584 (11): 6.09 / 6.55, 8.73 / 8.89   1,920 (13): 6.23 / 6.92, 8.97 / 9.37
+//            1,584 (11): 6.10 / 6.55, 8.80 / 8.89   1,920 (13): 6.24 / 6.92, 9.04 / 9.37
 // (with p mirrored as well, KH = 1 took 4.88 and 6.40, 5.60 and 7.32).  MIXED
 // spills a little with KH = 2, so it takes it from 11 leaves per SM on.  More
 // than 16 warps leave too few registers (28 warps of 72, KH = 1, 1,278 leaves:
