@@ -947,16 +947,14 @@ int step_moved(fsim_sim* s, float dt, const fsim_pcg_params* prm, fsim_step_stat
   // the CFL maximum (where the solve gave up, the kernels in between return
   // without a write)
   if ((rc = pcg_solve(s, prm, &ps, nullptr, true))) return rc;
-  s->pres_valid = true;
-  if ((rc = launch_pressure_update(s, true))) return rc;
-  s->extrapolated = true;
-  if ((rc = launch_g2p(s))) return rc;
   float vmax = 0.f;
-  if ((rc = read_vmax(s, &vmax))) return rc;
-  if ((rc = pcg_collect(s, prm, &ps))) {
-    s->pres_valid = s->extrapolated = false;
-    return rc;
-  }
+  rc = launch_pressure_update(s, true);
+  if (!rc) rc = launch_g2p(s);
+  if (!rc) rc = read_vmax(s, &vmax);
+  if (!rc) rc = pcg_collect(s, prm, &ps);
+  s->pcg_pending = false;
+  if (rc) return rc;
+  s->pres_valid = s->extrapolated = true;
   if (st) {
     std::memset(st, 0, sizeof(*st));
     int64_t cnt = 0;

@@ -2257,7 +2257,8 @@ void refuse_loop(fsim_sim* s, int loop, int precision) {
 // bound by the FP64 pipe, which 16 SMs hold too little of.
 bool use_cluster(const fsim_sim* s, int precision) {
   return precision != FSIM_PREC_FP64 && s->pcg_res < 0 && s->n_pleaf > 0 &&
-         s->n_pleaf <= kClLeaves && !loop_refused(s, kLoopCluster, precision) && !(precision == FSIM_PREC_FP32 && s->pcg_cg1 == 1);
+         s->n_pleaf <= kClLeaves && !loop_refused(s, kLoopCluster, precision) &&
+         !(precision == FSIM_PREC_FP32 && s->pcg_cg1 == 1);
 }
 
 #include "pcg_resident.cuh"
